@@ -261,6 +261,15 @@ void dfree(T *&p) {
     p = nullptr;
 }
 
+// where the shared-root beam geometry holds (Consts::beamFastLo)
+template <class LP>
+void set_beam_range(Consts<LP> &c) {
+    const double ew4 = (double)(LP)(c.E * c.W4);
+    c.beamFastLo = (ew4 >= std::ldexp(1.0, -40) && ew4 <= std::ldexp(1.0, 60))
+                       ? (LP)std::ldexp(1.0, -40)
+                       : std::numeric_limits<LP>::infinity();
+}
+
 // Derived constants of the sample main (HiDEM/MeshBlock/MainMeshBlock.cpp:69-156) in lp
 // precision, and the search distances of HiDEMLib::setup (HiDEMLib.h:757-761).
 template <class LP>
@@ -281,6 +290,7 @@ void derive(const hidem_params &P, Consts<LP> &c, double &searchDistance, double
     c.W2 = beamWidth * beamWidth;
     c.W4 = beamWidth * beamWidth * beamWidth * beamWidth;
     c.G = (LP)((double)E / 2.0);
+    set_beam_range(c);
     c.bendBreak = (LP)P.bendBreak;
     c.maxLoad = (LP)P.maxLoad;
     c.linkInvDt = c.invDt;
@@ -749,6 +759,8 @@ StepArgs<LP> step_args(hidem_ctx *ctx) {
     a.step = ctx->step;
     a.bendBreak = consts<LP>(ctx).bendBreak;
     a.maxLoad = consts<LP>(ctx).maxLoad;
+    a.wholeLoad = (LP)(1.0 + (double)a.maxLoad - 1e-5 * (1.0 + std::fabs((double)a.maxLoad)));
+    a.wholeBend = (LP)((double)a.bendBreak + 1e-5 * std::fabs((double)a.bendBreak));
     a.diffMax = ctx->diffMax;
     a.events = ctx->events;
     a.eventCount = ctx->eventCount;
@@ -805,8 +817,8 @@ constexpr int kTuneRounds = 3;
 static_assert(2 * kNumCandidates * kTuneRounds <= (int)(sizeof(hidem_ctx::tuneEv) / sizeof(cudaEvent_t)),
               "one event pair per tuning step");
 
-// the force kernel of a step kernel choice (TWO_PASS: the register-capped one, unfused)
-int force_kernel(int k) { return k == HIDEM_STEP_KERNEL_TWO_PASS ? HIDEM_STEP_KERNEL_THREAD_CAPPED : k; }
+// the fused kernel standing in for a step kernel choice (TWO_PASS: the register-capped one)
+int fused_kernel(int k) { return k == HIDEM_STEP_KERNEL_TWO_PASS ? HIDEM_STEP_KERNEL_THREAD_CAPPED : k; }
 
 int step_kernel_now(hidem_ctx *ctx, cudaEvent_t *e0, cudaEvent_t *e1) {
     *e0 = *e1 = nullptr;
@@ -853,61 +865,81 @@ void step_kernel_resolve(hidem_ctx *ctx) {
     ctx->tunedKernel = kTuneCandidates[best];
 }
 
-// n whole timesteps, one fused kernel each (MainMeshBlock.cpp:274-323).
+// the gather layout of the records lives in the record buffer that does not hold the state
+template <class LP>
+int4 *gather_buf(hidem_ctx *ctx) {
+    return reinterpret_cast<int4 *>(ctx->rec[1 - ctx->cur]);
+}
+
+// n whole timesteps (MainMeshBlock.cpp:274-323), each one fused kernel or two passes. The
+// two-pass steps keep the state in the gather layout between them; the records are written
+// again by the call's last step, and before a rebuild or a fused step reads them.
 template <class LP>
 hidem_status run_steps(hidem_ctx *ctx, int nsteps) {
     bool pending = false;      // link update of step-1 not applied yet
     long long pendingStep = 0;
     bool diffReady = false;
+    bool gathered = false;     // the gather layout holds the state
+    bool recStale = false;     // the records do not
+    auto records_now = [&]() {
+        if (!recStale) return;
+        launch_from_gather<LP>(gather_buf<LP>(ctx), (int)ctx->n, recp<LP>(ctx, ctx->cur), ctx->stream);
+        ctx->launches += 1;
+        recStale = false;
+    };
     for (int s = 0; s < nsteps; ++s) {
         const long long t = ctx->step;
         cudaEvent_t e0 = nullptr, e1 = nullptr, t0 = nullptr, t1 = nullptr;
         const int kern = step_kernel_now(ctx, &t0, &t1);
-        if (kern == HIDEM_STEP_KERNEL_TWO_PASS && pending) {
-            // the previous (fused) step's link update, where the reference runs it
-            TRY(link_update_now<LP>(ctx, pendingStep));
-            pending = false;
+        // gridService reads the maxima of the diffs at the start of step t
+        double currDist = 0;
+        if (gs_wants_diff(ctx)) {
+            if (!diffReady) {
+                records_now();
+                TRY(reduce_diff_now(ctx));
+            }
+            TRY(read_diff_max(ctx, &currDist));
         }
-        if (ctx->P.gridRegenInterval == -1 && t % 10 == 0) {
-            // gridService reads the maxima of the diffs at the start of step t
-            TRY(grid_service(ctx, diffReady));
-        } else {
-            TRY(grid_service(ctx, false));
+        if (gs_decide(ctx, currDist)) {
+            records_now();
+            gathered = false;
+            TRY(do_rebuild(ctx));
         }
-        diffReady = false;
-        if (kern == HIDEM_STEP_KERNEL_TWO_PASS) {
-            // force pass, integrate pass (in place), break pass (MainMeshBlock.cpp:295-320)
-            if (ctx->profile) TRY(profile_pair(ctx, &e0, &e1));
-            if (e0) CK(cudaEventRecord(e0, ctx->stream));
-            if (t0) CK(cudaEventRecord(t0, ctx->stream));
-            launch_step<LP>(consts<LP>(ctx), step_args<LP>(ctx), false, (int)ctx->maxNeigh,
-                            (int)ctx->maxLinksPP, HIDEM_STEP_KERNEL_THREAD_CAPPED, ctx->stream);
-            launch_integrate<LP>(consts<LP>(ctx), recp<LP>(ctx, ctx->cur), ctx->type[ctx->ord],
-                                 static_cast<const LP *>(ctx->force), (int)ctx->n, ctx->stream);
-            ctx->launches += 2;
-            if (break_active<LP>(ctx, t)) TRY(link_update_now<LP>(ctx, t));
-            if (t1) CK(cudaEventRecord(t1, ctx->stream));
-            if (e1) CK(cudaEventRecord(e1, ctx->stream));
-            ctx->step = t + 1;
-            continue;
+        const bool reduce = ctx->P.gridRegenInterval == -1 && (t + 1) % 10 == 0;
+        diffReady = reduce;
+        if (reduce) CK(cudaMemsetAsync(ctx->diffMax, 0, 3 * sizeof(unsigned long long), ctx->stream));
+        const bool twoPass = kern == HIDEM_STEP_KERNEL_TWO_PASS;
+        if (twoPass && !gathered) {
+            launch_to_gather<LP>(recp<LP>(ctx, ctx->cur), (int)ctx->n, gather_buf<LP>(ctx), ctx->stream);
+            ctx->launches += 1;
+            gathered = true;
+        }
+        if (!twoPass) {
+            records_now();
+            gathered = false;
         }
         StepArgs<LP> a = step_args<LP>(ctx);
+        a.gather = gather_buf<LP>(ctx);
         a.breakPending = pending ? 1 : 0;
         a.breakStep = pendingStep;
-        a.reduceDiff = (ctx->P.gridRegenInterval == -1 && (t + 1) % 10 == 0) ? 1 : 0;
-        if (a.reduceDiff) {
-            CK(cudaMemsetAsync(ctx->diffMax, 0, 3 * sizeof(unsigned long long), ctx->stream));
-            diffReady = true;
-        }
+        a.reduceDiff = reduce ? 1 : 0;
         if (ctx->profile) TRY(profile_pair(ctx, &e0, &e1));
         if (e0) CK(cudaEventRecord(e0, ctx->stream));
         if (t0) CK(cudaEventRecord(t0, ctx->stream));
-        launch_step<LP>(consts<LP>(ctx), a, true, (int)ctx->maxNeigh, (int)ctx->maxLinksPP, kern,
-                        ctx->stream);
+        if (twoPass) {
+            const bool last = s == nsteps - 1;
+            launch_force<LP>(consts<LP>(ctx), a, ctx->smCount, ctx->stream);
+            launch_integrate_gather<LP>(consts<LP>(ctx), a.gather, last ? recp<LP>(ctx, ctx->cur) : nullptr, a.type,
+                                        a.force, a.n, reduce, ctx->diffMax, ctx->stream);
+            recStale = !last;
+            ctx->launches += 2;
+        } else {
+            launch_step<LP>(consts<LP>(ctx), a, (int)ctx->maxNeigh, (int)ctx->maxLinksPP, kern, ctx->stream);
+            ctx->launches += 1;
+            ctx->cur = 1 - ctx->cur;  // the slot order (type / orig / cellOf) is unchanged
+        }
         if (t1) CK(cudaEventRecord(t1, ctx->stream));
         if (e1) CK(cudaEventRecord(e1, ctx->stream));
-        ctx->launches += 1;
-        ctx->cur = 1 - ctx->cur;  // the slot order (type / orig / cellOf) is unchanged
         pending = break_active<LP>(ctx, t);
         pendingStep = t;
         ctx->step = t + 1;  // finalizeTs
@@ -1198,6 +1230,12 @@ hidem_status batch_upload(hidem_batch *b, const std::vector<char> &pending, int 
         launch_block_table(dfb + g.fbOffset, g.count, b->tbl + g.tblOffset, b->stream);
         launch_block_table(dfb + 2 * nc + g.fbOffset, g.count, b->tbl + g.ltblOffset, b->stream);
         b->ctxs[0]->launches += 2;
+        // the records in the gather layout for the run's two-pass steps
+        if (kernel == HIDEM_STEP_KERNEL_TWO_PASS && g.blocks > 0) {
+            launch_gather_batch<LP>(static_cast<const BatchEntry<LP> *>(b->entries) + g.first, dfb + g.fbOffset,
+                                    b->tbl + g.tblOffset, (int)g.blocks, b->stream);
+            b->ctxs[0]->launches += 1;
+        }
     }
     BCK(cudaGetLastError());
     b->uploadPending = true;
@@ -1206,7 +1244,7 @@ hidem_status batch_upload(hidem_batch *b, const std::vector<char> &pending, int 
 }
 
 template <class LP>
-void batch_enqueue_step(hidem_batch *b, int kernel, int run) {
+void batch_enqueue_step(hidem_batch *b, int kernel, int run, bool last) {
     const int nc = (int)b->ctxs.size();
     const BatchEntry<LP> *ent = static_cast<const BatchEntry<LP> *>(b->entries);
     const int *fb = reinterpret_cast<const int *>(ent + nc);
@@ -1217,7 +1255,7 @@ void batch_enqueue_step(hidem_batch *b, int kernel, int run) {
         std::memcpy(&c, g.consts.data(), sizeof c);
         if (kernel == HIDEM_STEP_KERNEL_TWO_PASS)
             launch_two_pass_batch<LP>(c, ent + g.first, fb + g.fbOffset, b->tbl + g.tblOffset,
-                                      fb + 2 * nc + g.fbOffset, b->tbl + g.ltblOffset, run,
+                                      fb + 2 * nc + g.fbOffset, b->tbl + g.ltblOffset, run, last,
                                       (int)g.blocks, (int)g.linkBlocks, b->stream);
         else
             launch_step_batch<LP>(c, ent + g.first, fb + g.fbOffset, b->tbl + g.tblOffset, run,
@@ -1235,7 +1273,7 @@ hidem_status batch_launch_run(hidem_batch *b, int run, int kernel) {
         b->shape = sh;
     }
     if (!(b->flags & HIDEM_BATCH_GRAPHS)) {
-        for (int j = 0; j < run; ++j) batch_enqueue_step<LP>(b, kernel, j);
+        for (int j = 0; j < run; ++j) batch_enqueue_step<LP>(b, kernel, j, j == run - 1);
         BCK(cudaGetLastError());
         return HIDEM_OK;
     }
@@ -1243,7 +1281,7 @@ hidem_status batch_launch_run(hidem_batch *b, int run, int kernel) {
     if (it == b->graphs.end()) {
         cudaGraph_t g = nullptr;
         BCK(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
-        for (int j = 0; j < run; ++j) batch_enqueue_step<LP>(b, kernel, j);
+        for (int j = 0; j < run; ++j) batch_enqueue_step<LP>(b, kernel, j, j == run - 1);
         const cudaError_t le = cudaGetLastError();
         const cudaError_t ce = cudaStreamEndCapture(b->stream, &g);
         if (le != cudaSuccess || ce != cudaSuccess) {
@@ -1414,8 +1452,8 @@ hidem_status batch_run(hidem_batch *b, int nsteps) {
                     a.reduceDiff = (c->P.gridRegenInterval == -1 && (t + 1) % 10 == 0) ? 1 : 0;
                     if (a.reduceDiff)
                         BCK(cudaMemsetAsync(c->diffMax, 0, 3 * sizeof(unsigned long long), b->stream));
-                    launch_step<LP>(consts<LP>(c), a, true, (int)c->maxNeigh, (int)c->maxLinksPP,
-                                    force_kernel(step_kernel_settled(c)), b->stream);
+                    launch_step<LP>(consts<LP>(c), a, (int)c->maxNeigh, (int)c->maxLinksPP,
+                                    fused_kernel(step_kernel_settled(c)), b->stream);
                     c->launches += 1;
                     b->launches += 1;
                 }
@@ -1665,7 +1703,8 @@ hidem_status hidem_set_particles(hidem_ctx *ctx, const hidem_particle_soa *p, in
     const size_t lp = ctx->lp;
     const size_t recBytes = ctx->mixed ? sizeof(PRec<float>) : sizeof(PRec<double>);
     for (int b = 0; b < 2; ++b) {
-        TRY(dalloc_bytes(ctx, &ctx->rec[b], recBytes * (size_t)n));
+        // whole blocks of 32: either buffer may hold the gather layout
+        TRY(dalloc_bytes(ctx, &ctx->rec[b], recBytes * (size_t)(nblocks32(n) * 32)));
         TRY(dalloc(ctx, &ctx->type[b], n));
         TRY(dalloc(ctx, &ctx->orig[b], n));
         TRY(dalloc(ctx, &ctx->cellOf[b], n));
@@ -1899,37 +1938,34 @@ hidem_status hidem_regenerate(hidem_ctx *ctx) {
 
 hidem_status halo_forces(hidem_ctx *ctx, void *buf, bool pack);
 
-// the split force pass; with sendBuf, the halo send records come out of the same kernel
-// where the force pass is the thread-per-particle one, else from the pack kernel after it
+// the split force pass; with sendBuf, the halo send records come out of the same kernel. The
+// records are laid out for it on every call: a caller may have written them through a device
+// view since the last one.
+extern "C++" {
+template <class LP>
+static hidem_status compute_forces_t(hidem_ctx *ctx, void *sendBuf) {
+    const bool packed = sendBuf && ctx->nHaloSend > 0 && ctx->haloSendPos;
+    launch_to_gather<LP>(recp<LP>(ctx, ctx->cur), (int)ctx->n, gather_buf<LP>(ctx), ctx->stream);
+    StepArgs<LP> a = step_args<LP>(ctx);
+    a.gather = gather_buf<LP>(ctx);
+    if (packed) {
+        a.sendPos = ctx->haloSendPos;
+        a.sendBuf = static_cast<LP *>(sendBuf);
+    }
+    launch_force<LP>(consts<LP>(ctx), a, ctx->smCount, ctx->stream);
+    ctx->launches += 2;
+    CK(cudaGetLastError());
+    if (sendBuf && !packed) TRY(halo_forces(ctx, sendBuf, true));
+    return HIDEM_OK;
+}
+}  // extern "C++"
+
 static hidem_status compute_forces_into(hidem_ctx *ctx, void *sendBuf) {
     if (!ctx) return HIDEM_ERR_ARG;
     if (!ctx->haveParticles || !ctx->haveLinks) return fail(ctx, HIDEM_ERR_STATE, "particles and links must be set");
     CK(cudaSetDevice(ctx->device));
     if (!ctx->built) TRY(do_rebuild(ctx));
-    const int kern = force_kernel(step_kernel_settled(ctx));
-    const bool fusedPack = sendBuf && ctx->nHaloSend > 0 && ctx->haloSendPos &&
-                           (kern == HIDEM_STEP_KERNEL_THREAD || kern == HIDEM_STEP_KERNEL_THREAD_CAPPED);
-    if (ctx->mixed) {
-        StepArgs<float> a = step_args<float>(ctx);
-        if (fusedPack) {
-            a.sendPos = ctx->haloSendPos;
-            a.sendBuf = static_cast<float *>(sendBuf);
-        }
-        launch_step<float>(ctx->cf, a, false, (int)ctx->maxNeigh, (int)ctx->maxLinksPP, kern,
-                           ctx->stream);
-    } else {
-        StepArgs<double> a = step_args<double>(ctx);
-        if (fusedPack) {
-            a.sendPos = ctx->haloSendPos;
-            a.sendBuf = static_cast<double *>(sendBuf);
-        }
-        launch_step<double>(ctx->cd, a, false, (int)ctx->maxNeigh, (int)ctx->maxLinksPP, kern,
-                            ctx->stream);
-    }
-    ctx->launches += 1;
-    CK(cudaGetLastError());
-    if (sendBuf && !fusedPack) TRY(halo_forces(ctx, sendBuf, true));
-    return HIDEM_OK;
+    return ctx->mixed ? compute_forces_t<float>(ctx, sendBuf) : compute_forces_t<double>(ctx, sendBuf);
 }
 
 hidem_status hidem_compute_forces(hidem_ctx *ctx) {
@@ -2451,6 +2487,7 @@ hidem_status hidem_set_functor_params(hidem_ctx *ctx, const hidem_functor_params
         c.W2 = (LP)f->link_W2;
         c.W4 = (LP)f->link_W4;
         c.G = (LP)f->link_G;
+        set_beam_range(c);
         c.bendBreak = (LP)f->break_bendBreak;
         c.maxLoad = (LP)f->break_maxLoad;
     };

@@ -52,6 +52,20 @@ struct alignas(16) PRec<double> {
 static_assert(sizeof(PRec<float>) == 64, "mixed particle record must be 64 bytes");
 static_assert(sizeof(PRec<double>) == 128, "fp64 particle record must be 128 bytes");
 
+// The gather layout of the records: the copy the force pass reads its partners from (and its
+// own particle), in 16-byte chunks, chunk-major in blocks of 32 slots: chunk k of slot s is
+// int4 number (s / 32) * 32 * kGatherChunks + 32 k + s % 32.
+// What bounds the force pass is the L1's data path: one wavefront per 128-byte line a warp
+// touches. In the array of records a 16-byte load of 32 partners touches 16-32 lines (two
+// records to a line); partners of neighbouring slots being neighbouring slots, a chunk of 32
+// of them lies in fewer lines here: on the 0.8M slab (mixed) 183 wavefronts per contact and
+// link end from the records, 116 from this layout (32-byte chunks: as many). Figures per step at
+// force_particle (kernels.cu).
+// Chunks: mixed (x, y), (z, xDiff, uDiff), (yDiff, vDiff, zDiff, wDiff), (radius, thetas); FP64
+// (x, y), (z, d0), (d1, d2), (d3, d4), (d5, radius), (th0, th1), (th2, -).
+template <class LP>
+constexpr int kGatherChunks = sizeof(LP) == 4 ? 4 : 7;
+
 // A regular 2-D map in the reference's Map2d form (PLiB/Geometry/Map2d.h:23-60): lp
 // values, x fastest; the grid metrics in float as the Map2d constructor computes them.
 struct Map2dView {
@@ -86,6 +100,9 @@ struct Consts {
     // HiDEMDefLinkForceFunc (its own invDt / damping / dampingRotation: a caller's main
     // may construct the two functors with different values)
     LP linkInvDt, linkDamping, linkDampingRotation, E, W2, W4, G;
+    // least xy part of a squared link length for which the shared-root evaluation of the
+    // beam's geometry holds (physics.cuh): 2^-40, infinite when E W4 is outside [2^-40, 2^60]
+    LP beamFastLo;
     // HiDEMDefLinkBreakFunc
     LP bendBreak, maxLoad;
     // integrate (mainInvDt: the sample main's invDt, used by the velocity limit)
@@ -124,6 +141,7 @@ template <class LP>
 struct StepArgs {
     const PRec<LP> *in;
     PRec<LP> *out;
+    int4 *gather;             // the records in the gather layout (two-pass steps, split forces)
     const uint8_t *type;
     const uint32_t *counts;   // (#contacts) | (#link ends << 16) per slot
     const long long *nOff;    // contact-list block offsets
@@ -148,6 +166,8 @@ struct StepArgs {
     int *errorFlag;
     int maxContacts, maxEnds; // widest rows of this layout
     LP bendBreak, maxLoad;    // HiDEMDefLinkBreakFunc thresholds (per context in a batch)
+    // stays_whole's bounds: 1 + maxLoad - 1e-5 (1 + |maxLoad|), bendBreak + 1e-5 |bendBreak|
+    LP wholeLoad, wholeBend;
     // halo send records written by the force pass itself (split path; null: none): the
     // slot's position in the send list or -1, and the packed buffer of 6 lp per position
     const int32_t *sendPos;

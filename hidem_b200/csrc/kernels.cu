@@ -6,9 +6,10 @@
 //   contacts     k_nbr_count, k_nbr_fill           (NeighAccel::generateNeighbours, NeighAccel.h:25-137)
 //   link ends    k_side_count, k_side_fill         (LinkAccelSide::generateLinks/sortSideData,
 //                                                   LinkAccelSide.h:92-143,160-417)
-//   timestep     k_step<FUSED>                     (CombinedAccel::iterateCombined + applyForce +
-//                                                   linkUpdate, CombinedAccel.h:122-235)
-//                k_integrate, k_link_break, k_max_diff
+//   timestep     k_force, k_integrate_gather       (CombinedAccel::iterateCombined + applyForce +
+//                k_step, k_step_async,              linkUpdate, CombinedAccel.h:122-235)
+//                k_step_items, k_integrate,
+//                k_link_break, k_max_diff
 #include <algorithm>
 #include <atomic>
 #include <cstdio>
@@ -529,59 +530,335 @@ __device__ __forceinline__ PRec<LP> load_rec_head(const PRec<LP> *p) {
     for (int k = 0; k < CHUNKS; ++k) dst[k] = __ldg(src + k);
     return r;
 }
-// Hint the L2 to fetch a line that a later iteration will load (no register, no wait).
-__device__ __forceinline__ void prefetch_l2(const void *p) {
-    asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
-}
-
 // chunks holding x, y, z, d[6], r
 template <class LP>
 constexpr int kContactChunks = (int)((3 * sizeof(double) + 7 * sizeof(LP) + 15) / 16);
 
-// One particle per thread. FUSED: previous step's link update (if pending), contacts,
-// link ends, integrate, write the record to the other buffer. Split (FUSED=false):
-// contacts and link ends only, forces to a.force (HiDEMLib::computePartForce).
+// Start the L2 fetch of everything this warp will stream: its block's contact indices and its
+// link ends' partner words, CT0..CT5, states (and initial lengths), each one contiguous run of
+// the warp-blocked layout. One bulk prefetch per array, one lane each (nothing to wait for),
+// instead of a prefetch per array and item. Runs are multiples of 32 entries from 32-entry
+// offsets: 16-byte aligned for the byte arrays too.
+__device__ __forceinline__ void bulk_prefetch_l2(const void *p, unsigned bytes) {
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
+}
+template <class LP>
+__device__ __forceinline__ void prefetch_block(const StepArgs<LP> &a, int w, bool lengths) {
+    const int lane = threadIdx.x & 31;
+    const long long s0 = __ldg(a.sOff + w), n0 = __ldg(a.nOff + w);
+    const unsigned ends = (unsigned)(__ldg(a.sOff + w + 1) - s0), contacts = (unsigned)(__ldg(a.nOff + w + 1) - n0);
+    const void *p = nullptr;
+    unsigned bytes = 0;
+#pragma unroll
+    for (int q = 0; q < 6; ++q)
+        if (lane == q) p = a.ct[q] + s0, bytes = ends * (unsigned)sizeof(LP);
+    if (lane == 6) p = a.sPartner + s0, bytes = ends * 4u;
+    if (lane == 7) p = a.sState + s0, bytes = ends;
+    if (lane == 8) p = a.nbr + n0, bytes = contacts * 4u;
+    if (lane == 9 && lengths) p = a.sL0 + s0, bytes = ends * (unsigned)sizeof(LP);
+    if (bytes) bulk_prefetch_l2(p, bytes);
+}
+
+// Whether a whole link between two particles a squared distance D apart (as the break functor
+// forms it) stays whole for certain: its load is below maxLoad by more than 1e-5 (1 + |maxLoad|
+// + |bendBreak| bend), far above the functor's and this test's rounding (a few 2^-23 of the same
+// sum), so the functor's root and division are left to the links near the threshold. A test
+// that is not certain (NaN, a non-positive bound) is false.
+template <class LP>
+__device__ __forceinline__ bool stays_whole(const StepArgs<LP> &a, LP D, const LP *thA, const LP *thB, LP L0) {
+    const LP ax = labs_(thA[0] - thB[0]), ay = labs_(thA[1] - thB[1]), az = labs_(thA[2] - thB[2]);
+    const LP myz = (ay < az) ? az : ay;
+    const LP bend = (ax < myz) ? myz : ax;
+    const LP t = L0 * (a.wholeLoad - a.wholeBend * bend);
+    return t > LP(0) && D < t * t;
+}
+
+// The link state of one end after the previous step's link update (a.breakPending), both ends
+// of a link deciding alike from the same records; end A appends the break event.
+template <class LP, class P>
+__device__ __forceinline__ uint8_t pending_break(const StepArgs<LP> &a, unsigned si, uint32_t pw, const P &me,
+                                                 const P &other, uint8_t st, LP L0, LP x, LP y, LP z) {
+    if (st == 0 || stays_whole<LP>(a, x * x + y * y + z * z, me.th, other.th, L0)) return st;
+    const uint8_t nst = (pw & kSideIsB) ? break_link<LP>(a.bendBreak, a.maxLoad, other, me, st, L0)
+                                        : break_link<LP>(a.bendBreak, a.maxLoad, me, other, st, L0);
+    if (nst != st) {
+        a.sState[si] = nst;
+        a.linkState[__ldg(a.sLink + si)] = nst;  // both sides write the same value
+        if (nst == 0 && !(pw & kSideIsB)) {
+            unsigned long long slot = atomicAdd(a.eventCount, 1ull);
+            if ((long long)slot < a.eventCap) a.events[slot] = make_int2(__ldg(a.sLink + si), (int)a.breakStep);
+        }
+    }
+    return nst;
+}
+
+// ---- the gather layout (internal.h) ----
+
+__device__ __forceinline__ void pack16(int4 *p, double a, double b) {
+    *reinterpret_cast<double2 *>(p) = make_double2(a, b);
+}
+template <class LP>
+__device__ __forceinline__ long long gather_index(int slot) {
+    return (long long)(slot >> 5) * (32 * kGatherChunks<LP>) + (slot & 31);
+}
+__device__ __forceinline__ void store_gather(int4 *base, int slot, const PRec<float> &r) {
+    int4 *p = base + gather_index<float>(slot);
+    pack16(p, r.x, r.y);
+    p[32] = make_int4(__double2loint(r.z), __double2hiint(r.z), __float_as_int(r.d[0]), __float_as_int(r.d[3]));
+    *reinterpret_cast<float4 *>(p + 64) = make_float4(r.d[1], r.d[4], r.d[2], r.d[5]);
+    *reinterpret_cast<float4 *>(p + 96) = make_float4(r.r, r.th[0], r.th[1], r.th[2]);
+}
+__device__ __forceinline__ void store_gather(int4 *base, int slot, const PRec<double> &r) {
+    int4 *p = base + gather_index<double>(slot);
+    pack16(p, r.x, r.y);
+    pack16(p + 32, r.z, r.d[0]);
+    pack16(p + 64, r.d[1], r.d[2]);
+    pack16(p + 96, r.d[3], r.d[4]);
+    pack16(p + 128, r.d[5], r.r);
+    pack16(p + 160, r.th[0], r.th[1]);
+    pack16(p + 192, r.th[2], 0.0);
+}
+// A particle as the functors read it: position and increments, radius, rotations.
+template <class LP>
+struct Body {
+    double x, y, z;
+    Six<LP> d;
+    LP r, th[3];
+};
+// (WITH_R: the radius too; WITH_TH: the rotations too; fields not asked for stay unset)
+template <bool WITH_R, bool WITH_TH>
+__device__ __forceinline__ void load_body(Body<float> &o, const int4 *base, int slot) {
+    const int4 *p = base + gather_index<float>(slot);
+    const double2 c0 = __ldg(reinterpret_cast<const double2 *>(p));
+    const ulonglong2 c1 = __ldg(reinterpret_cast<const ulonglong2 *>(p + 32));
+    const ulonglong2 c2 = __ldg(reinterpret_cast<const ulonglong2 *>(p + 64));
+    o.x = c0.x;
+    o.y = c0.y;
+    o.z = __longlong_as_double((long long)c1.x);
+    o.d.p[0].v = c1.y;
+    o.d.p[1].v = c2.x;
+    o.d.p[2].v = c2.y;
+    if (WITH_TH) {
+        const float4 c3 = __ldg(reinterpret_cast<const float4 *>(p + 96));
+        o.r = c3.x;
+        o.th[0] = c3.y;
+        o.th[1] = c3.z;
+        o.th[2] = c3.w;
+    } else if (WITH_R) {
+        o.r = __ldg(reinterpret_cast<const float *>(p + 96));
+    }
+}
+template <bool WITH_R, bool WITH_TH>
+__device__ __forceinline__ void load_body(Body<double> &o, const int4 *base, int slot) {
+    const double2 *p = reinterpret_cast<const double2 *>(base + gather_index<double>(slot));
+    const double2 c0 = __ldg(p), c1 = __ldg(p + 32), c2 = __ldg(p + 64), c3 = __ldg(p + 96);
+    o.x = c0.x;
+    o.y = c0.y;
+    o.z = c1.x;
+    o.d.f[0] = c1.y;
+    o.d.f[1] = c2.x;
+    o.d.f[2] = c2.y;
+    o.d.f[3] = c3.x;
+    o.d.f[4] = c3.y;
+    if (WITH_R) {
+        const double2 c4 = __ldg(p + 128);
+        o.d.f[5] = c4.x;
+        o.r = c4.y;
+    } else {
+        o.d.f[5] = __ldg(reinterpret_cast<const double *>(p + 128));
+    }
+    if (WITH_TH) {
+        const double2 c5 = __ldg(p + 160);
+        o.th[0] = c5.x;
+        o.th[1] = c5.y;
+        o.th[2] = __ldg(reinterpret_cast<const double *>(p + 192));
+    }
+}
+template <class LP>
+__device__ __forceinline__ PRec<LP> gather_rec(const int4 *base, int slot) {
+    Body<LP> b;
+    load_body<true, true>(b, base, slot);
+    PRec<LP> r;
+    r.x = b.x;
+    r.y = b.y;
+    r.z = b.z;
+    b.d.get(r.d);
+    r.r = b.r;
+#pragma unroll
+    for (int q = 0; q < 3; ++q) r.th[q] = b.th[q];
+    if constexpr (sizeof(PRec<LP>) == 128) r.pad[0] = r.pad[1] = r.pad[2] = 0.0;
+    return r;
+}
+
+// The force pass: one particle per thread, contacts, then link ends, forces to a.force
+// (HiDEMLib::computePartForce), partners read from the gather layout. BRK: the previous step's
+// link update is applied on the way (each end decides its link from the records it has
+// loaded for the beam anyway; a break pass of its own gathers both records of every link
+// again: 0.33 of 2.03 ms per step on the 5.7M slab).
+//
+// What bounds it: the latency of one gather per item, against what the warps in flight can
+// hide. AHEAD keeps the next item's partner and CT in registers while this one is evaluated
+// (96-166 registers); without it, a warp waits for each gather but there are 28 warps an SM
+// instead of 20 (mixed, 72 registers) and no copies between the two register sets (120M
+// against 141M instructions on the 0.8M slab). Measured per step, 5.7M slab, mixed: from the
+// records with AHEAD 2.03 ms (L1 data path 86 % busy), gather layout with AHEAD 1.71 ms, without
+// 1.44 ms at 7 CTAs an SM (6: 1.50, 8: 1.51); FP64: 4.05 ms from the records, 2.67 ms with AHEAD
+// (3 CTAs), 2.95 ms without (4 CTAs). Where every block is resident at once anyway (a small
+// particle set) AHEAD is the faster one in both: 32,000 particles 25.1 against 27.4 us a step.
+template <class LP, bool BRK, bool AHEAD>
+__device__ __forceinline__ void force_particle(const Consts<LP> &c, const StepArgs<LP> &a, const int i) {
+    const Rounding<LP> R = Rounding<LP>::make();
+    if ((i & ~31) < a.n) prefetch_block<LP>(a, i >> 5, BRK);
+    if (i >= a.n) return;
+    Body<LP> me;
+    load_body<true, BRK>(me, a.gather, i);
+    const uint32_t cnt = __ldg(a.counts + i);
+    const int nn = (int)(cnt & 0xffffu), ns = (int)(cnt >> 16);
+    Six<LP> F = Six<LP>::zero();
+    const int32_t *nb = a.nbr + __ldg(a.nOff + (i >> 5)) + (i & 31);
+    // link-end slots fit 31 bits (checked at the rebuild)
+    unsigned si = (unsigned)__ldg(a.sOff + (i >> 5)) + (i & 31);
+
+    auto contact = [&](const Body<LP> &o) {
+        contact_pair<LP>(c, R, (LP)(me.x - o.x), (LP)(me.y - o.y), (LP)(me.z - o.z), me.d, me.r, o.d, o.r, F);
+    };
+    // what a link end is evaluated from, and its evaluation: the break decision, the beam, CT
+    struct End {
+        Body<LP> o;
+        LP CT[6], L0;
+        uint8_t st;
+    };
+    auto load_end = [&](End &e, uint32_t pw, unsigned at) {
+        load_body<false, BRK>(e.o, a.gather, (int)(pw & kSlotMask));
+        e.st = a.sState[at];
+#pragma unroll
+        for (int q = 0; q < 6; ++q) e.CT[q] = a.ct[q][at];
+        if (BRK) e.L0 = __ldg(a.sL0 + at);
+    };
+    auto end = [&](End &e, uint32_t pw, unsigned at) {
+        const LP x = (LP)(me.x - e.o.x), y = (LP)(me.y - e.o.y), z = (LP)(me.z - e.o.z);
+        if (BRK) e.st = pending_break<LP>(a, at, pw, me, e.o, e.st, e.L0, x, y, z);
+        beam_side<LP>(c, R, e.st != 0, x, y, z, me.d, e.o.d, e.CT, F);
+#pragma unroll
+        for (int q = 0; q < 6; ++q) a.ct[q][at] = e.CT[q];
+    };
+
+    if constexpr (!AHEAD) {
+        // the index of the next item is in flight while this one waits for its partner
+        int j = nn > 0 ? __ldg(nb) : 0;
+        uint32_t pw = ns > 0 ? __ldg(a.sPartner + si) : 0u;
+        for (int k = 0; k < nn; ++k) {
+            Body<LP> o;
+            load_body<true, false>(o, a.gather, j);
+            if (k + 1 < nn) j = __ldg(nb + (k + 1) * kWarp);
+            contact(o);
+        }
+        for (int k = 0; k < ns; ++k, si += kWarp) {
+            End e;
+            load_end(e, pw, si);
+            const uint32_t pwc = pw;
+            if (k + 1 < ns) pw = __ldg(a.sPartner + si + kWarp);
+            end(e, pwc, si);
+        }
+    } else {
+        // item k + 1 and the index of item k + 2 are in flight while item k is evaluated, the
+        // first link end behind the last contact
+        Body<LP> o;
+        int jn = 0;
+        if (nn > 0) load_body<true, false>(o, a.gather, __ldg(nb));
+        if (nn > 1) jn = __ldg(nb + kWarp);
+        uint32_t pwn = ns > 0 ? __ldg(a.sPartner + si) : 0u, pwnn = 0;
+        End en;
+        auto first_end = [&]() {
+            if (ns > 0) {
+                load_end(en, pwn, si);
+                if (ns > 1) pwnn = __ldg(a.sPartner + si + kWarp);
+            }
+        };
+        if (nn == 0) first_end();
+        for (int k = 0; k < nn; ++k) {
+            const Body<LP> cur = o;
+            if (k + 1 < nn) {
+                load_body<true, false>(o, a.gather, jn);
+                if (k + 2 < nn) jn = __ldg(nb + (k + 2) * kWarp);
+            } else {
+                first_end();
+            }
+            contact(cur);
+        }
+        for (int k = 0; k < ns; ++k, si += kWarp) {
+            End e = en;
+            const uint32_t pw = pwn;
+            if (k + 1 < ns) {
+                pwn = pwnn;
+                load_end(en, pwn, si + kWarp);
+                if (k + 2 < ns) pwnn = __ldg(a.sPartner + si + 2 * kWarp);
+            }
+            end(e, pw, si);
+        }
+    }
+
+    LP f[6];
+    F.get(f);
+#pragma unroll
+    for (int q = 0; q < 6; ++q) a.force[(long long)q * a.n + i] = f[q];
+    // a particle another rank integrates: its record of the halo send buffer too
+    if (a.sendPos) {
+        const int sp = __ldg(a.sendPos + i);
+        if (sp >= 0) {
+#pragma unroll
+            for (int q = 0; q < 6; ++q) a.sendBuf[6ll * sp + q] = f[q];
+        }
+    }
+}
+
+// One particle per thread: the previous step's link update (if pending), contacts, link
+// ends, integrate, the record written to the other buffer.
 // Both item loops are software-pipelined: while item k is evaluated, the partner record
 // (and for link ends the CT state, link state and initial length) of item k + 1 and the
 // index of item k + 2 are already in flight, and the first link end's loads go out behind
 // the last contact, so each thread keeps its dependent loads outstanding behind its
 // arithmetic. The functors still run in the reference's order per particle.
-template <class LP, bool FUSED>
+template <class LP>
 __device__ __forceinline__ void step_thread_particle(const Consts<LP> &c, const StepArgs<LP> &a,
                                                      const int i) {
     const bool live = i < a.n;
     LP dmax[3] = {LP(0), LP(0), LP(0)};
+    const Rounding<LP> R = Rounding<LP>::make();
+    const bool brk = a.breakPending;
+    if ((i & ~31) < a.n) prefetch_block<LP>(a, i >> 5, brk);
     if (live) {
         PRec<LP> me = load_rec(a.in + i);
         const uint32_t cnt = __ldg(a.counts + i);
-        const uint8_t ty = FUSED ? __ldg(a.type + i) : uint8_t(0);
+        const uint8_t ty = __ldg(a.type + i);
         const int nn = (int)(cnt & 0xffffu), ns = (int)(cnt >> 16);
-        LP F[6] = {0, 0, 0, 0, 0, 0};
+        const Six<LP> mine = Six<LP>::of(me.d);
+        Six<LP> F = Six<LP>::zero();
         constexpr int HC = kContactChunks<LP>;
 
         const int32_t *nb = a.nbr + __ldg(a.nOff + (i >> 5)) + (i & 31);
-        const long long sbase = __ldg(a.sOff + (i >> 5)) + (i & 31);
+        // link-end slots fit 31 bits (checked at the rebuild)
+        unsigned si = (unsigned)__ldg(a.sOff + (i >> 5)) + (i & 31);
         PRec<LP> o;
         int jn = 0;
         if (nn > 0) o = load_rec_head<LP, HC>(a.in + __ldg(nb));
         if (nn > 1) jn = __ldg(nb + kWarp);
         // first link end's partner word while the contacts run
-        uint32_t pwn = (ns > 0) ? __ldg(a.sPartner + sbase) : 0u;
+        uint32_t pwn = (ns > 0) ? __ldg(a.sPartner + si) : 0u;
         PRec<LP> o2;
         uint8_t stn = 0;
         LP ctn[6] = {0, 0, 0, 0, 0, 0};
         LP l0n = LP(0);
         uint32_t pwnn = 0;
-        const bool brk = FUSED && a.breakPending;
         // the first link end's partner record, state and CT go out behind the last contact
         auto first_side = [&]() {
             if (ns > 0) {
                 o2 = load_rec(a.in + (pwn & kSlotMask));
-                stn = a.sState[sbase];
+                stn = a.sState[si];
 #pragma unroll
-                for (int q = 0; q < 6; ++q) ctn[q] = a.ct[q][sbase];
-                if (brk) l0n = __ldg(a.sL0 + sbase);
-                if (ns > 1) pwnn = __ldg(a.sPartner + sbase + kWarp);
+                for (int q = 0; q < 6; ++q) ctn[q] = a.ct[q][si];
+                if (brk) l0n = __ldg(a.sL0 + si);
+                if (ns > 1) pwnn = __ldg(a.sPartner + si + kWarp);
             }
         };
         if (nn == 0) first_side();
@@ -589,19 +866,15 @@ __device__ __forceinline__ void step_thread_particle(const Consts<LP> &c, const 
             const PRec<LP> cur = o;
             if (k + 1 < nn) {
                 o = load_rec_head<LP, HC>(a.in + jn);
-                if (k + 2 < nn) {
-                    jn = __ldg(nb + (k + 2) * kWarp);
-                    if (k + 3 < nn) prefetch_l2(nb + (k + 3) * kWarp);
-                }
+                if (k + 2 < nn) jn = __ldg(nb + (k + 2) * kWarp);
             } else {
                 first_side();
             }
-            contact_pair<LP>(c, LP(1), (LP)(me.x - cur.x), (LP)(me.y - cur.y), (LP)(me.z - cur.z),
-                             me.d, me.r, cur.d, cur.r, F);
+            contact_pair<LP>(c, R, (LP)(me.x - cur.x), (LP)(me.y - cur.y), (LP)(me.z - cur.z), mine, me.r,
+                             Six<LP>::of(cur.d), cur.r, F);
         }
 
-        for (int k = 0; k < ns; ++k) {
-            const long long si = sbase + (long long)k * kWarp;
+        for (int k = 0; k < ns; ++k, si += kWarp) {
             const PRec<LP> cur = o2;
             const uint32_t pw = pwn;
             uint8_t st = stn;
@@ -616,56 +889,24 @@ __device__ __forceinline__ void step_thread_particle(const Consts<LP> &c, const 
 #pragma unroll
                 for (int q = 0; q < 6; ++q) ctn[q] = a.ct[q][si + kWarp];
                 if (brk) l0n = __ldg(a.sL0 + si + kWarp);
-                if (k + 2 < ns) {
-                    pwnn = __ldg(a.sPartner + si + 2 * kWarp);
-                    // the CT and state lines of item k + 2 start their way to L2
-#pragma unroll
-                    for (int q = 0; q < 6; ++q) prefetch_l2(a.ct[q] + si + 2 * kWarp);
-                    prefetch_l2(a.sState + si + 2 * kWarp);
-                }
+                if (k + 2 < ns) pwnn = __ldg(a.sPartner + si + 2 * kWarp);
             }
-            if (brk && st != 0) {
-                const uint8_t nst =
-                    (pw & kSideIsB) ? break_link<LP>(a.bendBreak, a.maxLoad, cur, me, st, L0)
-                                    : break_link<LP>(a.bendBreak, a.maxLoad, me, cur, st, L0);
-                if (nst != st) {
-                    a.sState[si] = nst;
-                    a.linkState[__ldg(a.sLink + si)] = nst;  // both sides write the same value
-                    if (nst == 0 && !(pw & kSideIsB)) {
-                        unsigned long long slot = atomicAdd(a.eventCount, 1ull);
-                        if ((long long)slot < a.eventCap)
-                            a.events[slot] = make_int2(__ldg(a.sLink + si), (int)a.breakStep);
-                    }
-                    st = nst;
-                }
-            }
-            const LP mask = (st == 0) ? LP(0) : LP(1);
-            beam_side<LP>(c, mask, (LP)(me.x - cur.x), (LP)(me.y - cur.y), (LP)(me.z - cur.z),
-                          me.d, cur.d, CT, F);
+            const LP x = (LP)(me.x - cur.x), y = (LP)(me.y - cur.y), z = (LP)(me.z - cur.z);
+            if (brk) st = pending_break<LP>(a, si, pw, me, cur, st, L0, x, y, z);
+            beam_side<LP>(c, R, st != 0, x, y, z, mine, Six<LP>::of(cur.d), CT, F);
 #pragma unroll
             for (int q = 0; q < 6; ++q) a.ct[q][si] = CT[q];
         }
 
-        if (FUSED) {
-            integrate_particle<LP>(c, me, ty, F);
-            store_rec(a.out + i, me);
-            dmax[0] = me.d[0] > LP(0) ? me.d[0] : LP(0);
-            dmax[1] = me.d[1] > LP(0) ? me.d[1] : LP(0);
-            dmax[2] = me.d[2] > LP(0) ? me.d[2] : LP(0);
-        } else {
-#pragma unroll
-            for (int q = 0; q < 6; ++q) a.force[(long long)q * a.n + i] = F[q];
-            // a particle another rank integrates: its record of the halo send buffer too
-            if (a.sendPos) {
-                const int sp = __ldg(a.sendPos + i);
-                if (sp >= 0) {
-#pragma unroll
-                    for (int q = 0; q < 6; ++q) a.sendBuf[6ll * sp + q] = F[q];
-                }
-            }
-        }
+        LP f[6];
+        F.get(f);
+        integrate_particle<LP>(c, me, ty, f);
+        store_rec(a.out + i, me);
+        dmax[0] = me.d[0] > LP(0) ? me.d[0] : LP(0);
+        dmax[1] = me.d[1] > LP(0) ? me.d[1] : LP(0);
+        dmax[2] = me.d[2] > LP(0) ? me.d[2] : LP(0);
     }
-    if (FUSED && a.reduceDiff) {
+    if (a.reduceDiff) {
 #pragma unroll
         for (int q = 0; q < 3; ++q) {
             LP v = dmax[q];
@@ -688,14 +929,37 @@ constexpr int kThreadBlocks = sizeof(LP) == 4 ? 4 : 1;
 // and the asynchronous-copy variant (its partner data lives in shared memory)
 template <class LP>
 constexpr int kAsyncBlocks = sizeof(LP) == 4 ? 5 : 3;
-// the register-capped force pass without the integrate tail (two-pass steps)
+// the force pass of a large particle set (register caps without spills; force_particle)
 template <class LP>
-constexpr int kCapBlocksForces = sizeof(LP) == 4 ? 5 : 3;
+constexpr bool kForceAhead = sizeof(LP) == 8;
+template <class LP>
+constexpr int kForceBlocks = sizeof(LP) == 4 ? 7 : 3;
+// and of one whose blocks are all resident at once even so: up to kFewBlocks CTAs per SM
+template <class LP>
+constexpr int kFewBlocks = sizeof(LP) == 4 ? 4 : 2;
 
-template <class LP, bool FUSED, int MINB>
+template <class LP, int MINB>
 __global__ void __launch_bounds__(kStepThreads, MINB)
     k_step(const Consts<LP> c, const StepArgs<LP> a) {
-    step_thread_particle<LP, FUSED>(c, a, blockIdx.x * blockDim.x + threadIdx.x);
+    step_thread_particle<LP>(c, a, blockIdx.x * blockDim.x + threadIdx.x);
+}
+
+template <class LP, bool BRK, bool AHEAD, int MINB>
+__global__ void __launch_bounds__(kStepThreads, MINB)
+    k_force(const Consts<LP> c, const StepArgs<LP> a) {
+    force_particle<LP, BRK, AHEAD>(c, a, blockIdx.x * blockDim.x + threadIdx.x);
+}
+
+// records -> gather layout, and back
+template <class LP>
+__global__ void __launch_bounds__(256) k_to_gather(const PRec<LP> *__restrict__ rec, int n, int4 *__restrict__ g) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) store_gather(g, i, load_rec(rec + i));
+}
+template <class LP>
+__global__ void __launch_bounds__(256) k_from_gather(const int4 *__restrict__ g, int n, PRec<LP> *__restrict__ rec) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) store_rec(rec + i, gather_rec<LP>(g, i));
 }
 
 // ---- shared-memory staging with bulk copies (cp.async.bulk + mbarrier) ----
@@ -732,7 +996,7 @@ constexpr size_t async_smem_bytes() {
     return (size_t)2 * kStepThreads * (sizeof(PRec<LP>) + 6 * sizeof(LP));
 }
 
-template <class LP, bool FUSED>
+template <class LP>
 __device__ __forceinline__ void step_thread_async(const Consts<LP> &c, const StepArgs<LP> &a,
                                                   const int i, unsigned char *smem) {
     constexpr int NC = kRecChunks<LP>;
@@ -751,14 +1015,16 @@ __device__ __forceinline__ void step_thread_async(const Consts<LP> &c, const Ste
         return r;
     };
 
+    const Rounding<LP> R = Rounding<LP>::make();
     const bool live = i < a.n;
     LP dmax[3] = {LP(0), LP(0), LP(0)};
     if (live) {
         PRec<LP> me = load_rec(a.in + i);
         const uint32_t cnt = __ldg(a.counts + i);
-        const uint8_t ty = FUSED ? __ldg(a.type + i) : uint8_t(0);
+        const uint8_t ty = __ldg(a.type + i);
         const int nn = (int)(cnt & 0xffffu), ns = (int)(cnt >> 16);
-        LP F[6] = {0, 0, 0, 0, 0, 0};
+        const Six<LP> mine = Six<LP>::of(me.d);
+        Six<LP> F = Six<LP>::zero();
         const int32_t *nb = a.nbr + __ldg(a.nOff + (i >> 5)) + (i & 31);
         const long long sbase = __ldg(a.sOff + (i >> 5)) + (i & 31);
 
@@ -782,14 +1048,14 @@ __device__ __forceinline__ void step_thread_async(const Consts<LP> &c, const Ste
                 if (k + 3 < nn) j2 = __ldg(nb + (k + 3) * kWarp);
             }
             cp_async_commit();
-            contact_pair<LP>(c, LP(1), (LP)(me.x - cur.x), (LP)(me.y - cur.y), (LP)(me.z - cur.z),
-                             me.d, me.r, cur.d, cur.r, F);
+            contact_pair<LP>(c, R, (LP)(me.x - cur.x), (LP)(me.y - cur.y), (LP)(me.z - cur.z), mine, me.r,
+                             Six<LP>::of(cur.d), cur.r, F);
         }
         cp_async_wait0();
 
         // link ends: record and CT of item k in slot k & 1; state and initial length one
         // item ahead in registers
-        const bool brk = FUSED && a.breakPending;
+        const bool brk = a.breakPending;
         auto issue_side = [&](int s, long long si, uint32_t pw) {
             const int4 *src = reinterpret_cast<const int4 *>(a.in + (pw & kSlotMask));
 #pragma unroll
@@ -834,41 +1100,23 @@ __device__ __forceinline__ void step_thread_async(const Consts<LP> &c, const Ste
                 if (k + 3 < ns) pw2 = __ldg(a.sPartner + si + 3 * kWarp);
             }
             cp_async_commit();
-            if (brk && st != 0) {
-                const uint8_t nst =
-                    (pw & kSideIsB) ? break_link<LP>(a.bendBreak, a.maxLoad, cur, me, st, L0)
-                                    : break_link<LP>(a.bendBreak, a.maxLoad, me, cur, st, L0);
-                if (nst != st) {
-                    a.sState[si] = nst;
-                    a.linkState[__ldg(a.sLink + si)] = nst;  // both sides write the same value
-                    if (nst == 0 && !(pw & kSideIsB)) {
-                        unsigned long long slot = atomicAdd(a.eventCount, 1ull);
-                        if ((long long)slot < a.eventCap)
-                            a.events[slot] = make_int2(__ldg(a.sLink + si), (int)a.breakStep);
-                    }
-                    st = nst;
-                }
-            }
-            const LP mask = (st == 0) ? LP(0) : LP(1);
-            beam_side<LP>(c, mask, (LP)(me.x - cur.x), (LP)(me.y - cur.y), (LP)(me.z - cur.z),
-                          me.d, cur.d, CT, F);
+            const LP x = (LP)(me.x - cur.x), y = (LP)(me.y - cur.y), z = (LP)(me.z - cur.z);
+            if (brk) st = pending_break<LP>(a, (unsigned)si, pw, me, cur, st, L0, x, y, z);
+            beam_side<LP>(c, R, st != 0, x, y, z, mine, Six<LP>::of(cur.d), CT, F);
 #pragma unroll
             for (int q = 0; q < 6; ++q) a.ct[q][si] = CT[q];
         }
         cp_async_wait0();
 
-        if (FUSED) {
-            integrate_particle<LP>(c, me, ty, F);
-            store_rec(a.out + i, me);
-            dmax[0] = me.d[0] > LP(0) ? me.d[0] : LP(0);
-            dmax[1] = me.d[1] > LP(0) ? me.d[1] : LP(0);
-            dmax[2] = me.d[2] > LP(0) ? me.d[2] : LP(0);
-        } else {
-#pragma unroll
-            for (int q = 0; q < 6; ++q) a.force[(long long)q * a.n + i] = F[q];
-        }
+        LP f[6];
+        F.get(f);
+        integrate_particle<LP>(c, me, ty, f);
+        store_rec(a.out + i, me);
+        dmax[0] = me.d[0] > LP(0) ? me.d[0] : LP(0);
+        dmax[1] = me.d[1] > LP(0) ? me.d[1] : LP(0);
+        dmax[2] = me.d[2] > LP(0) ? me.d[2] : LP(0);
     }
-    if (FUSED && a.reduceDiff) {
+    if (a.reduceDiff) {
 #pragma unroll
         for (int q = 0; q < 3; ++q) {
             LP v = dmax[q];
@@ -881,11 +1129,11 @@ __device__ __forceinline__ void step_thread_async(const Consts<LP> &c, const Ste
     }
 }
 
-template <class LP, bool FUSED, int MINB>
+template <class LP, int MINB>
 __global__ void __launch_bounds__(kStepThreads, MINB)
     k_step_async(const Consts<LP> c, const StepArgs<LP> a) {
     extern __shared__ __align__(16) unsigned char smem[];
-    step_thread_async<LP, FUSED>(c, a, blockIdx.x * blockDim.x + threadIdx.x, smem);
+    step_thread_async<LP>(c, a, blockIdx.x * blockDim.x + threadIdx.x, smem);
 }
 
 __device__ __forceinline__ void mbar_init(uint64_t *bar, uint32_t count) {
@@ -934,9 +1182,10 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t *bar, uint32_t parity
 // shared memory; one warp adds them in the reference's order (contacts in list order, then
 // per link end the damping term and the CT term) and integrates, so the result is
 // bit-identical to k_step.
-template <class LP, bool FUSED>
+template <class LP>
 __device__ __forceinline__ void step_items_block(const Consts<LP> &c, const StepArgs<LP> &a,
                                                  const int w, unsigned char *smem) {
+    const Rounding<LP> R = Rounding<LP>::make();
     const StageLayout L = stage_layout(sizeof(PRec<LP>), sizeof(LP), a.maxContacts, a.maxEnds);
     uint64_t *bar = reinterpret_cast<uint64_t *>(smem);
     PRec<LP> *own = reinterpret_cast<PRec<LP> *>(smem + L.own);
@@ -958,7 +1207,7 @@ __device__ __forceinline__ void step_items_block(const Consts<LP> &c, const Step
     const long long nOff0 = __ldg(a.nOff + w), sOff0 = __ldg(a.sOff + w);
     const int Wn = (int)((__ldg(a.nOff + w + 1) - nOff0) >> 5);
     const int Ws = (int)((__ldg(a.sOff + w + 1) - sOff0) >> 5);
-    const bool wantL0 = FUSED && a.breakPending;
+    const bool wantL0 = a.breakPending;
     LP *tc = terms;                  // [Wn][6][32]
     LP *ts = terms + Wn * 6 * 32;    // [Ws][12][32]
 
@@ -1020,9 +1269,11 @@ __device__ __forceinline__ void step_items_block(const Consts<LP> &c, const Step
             LP s[6];
 #pragma unroll
             for (int u = 0; u < 6; ++u) s[u] = od[u * 32 + lane];
+            Six<LP> tv = Six<LP>::zero();
+            contact_terms(c, R, (LP)(ox[lane] - o.x), (LP)(ox[32 + lane] - o.y), (LP)(ox[64 + lane] - o.z),
+                          Six<LP>::of(s), od[6 * 32 + lane], Six<LP>::of(o.d), o.r, tv);
             LP tt[6];
-            contact_terms<LP>(c, LP(1), (LP)(ox[lane] - o.x), (LP)(ox[32 + lane] - o.y),
-                              (LP)(ox[64 + lane] - o.z), s, od[6 * 32 + lane], o.d, o.r, tt);
+            tv.get(tt);
 #pragma unroll
             for (int u = 0; u < 6; ++u) tc[(k * 6 + u) * 32 + lane] = tt[u];
         }
@@ -1035,38 +1286,27 @@ __device__ __forceinline__ void step_items_block(const Consts<LP> &c, const Step
             const uint32_t pw = spw[q];
             const PRec<LP> o = load_rec(a.in + (pw & kSlotMask));
             uint8_t st = sst[q];
-            if (FUSED && a.breakPending && st != 0) {
+            const LP x = (LP)(ox[lane] - o.x), y = (LP)(ox[32 + lane] - o.y), z = (LP)(ox[64 + lane] - o.z);
+            if (a.breakPending) {
                 PRec<LP> me;
                 me.x = ox[lane];
                 me.y = ox[32 + lane];
                 me.z = ox[64 + lane];
 #pragma unroll
                 for (int u = 0; u < 3; ++u) me.th[u] = od[(7 + u) * 32 + lane];
-                const LP L0 = sl0[q];
-                const uint8_t nst =
-                    (pw & kSideIsB) ? break_link<LP>(a.bendBreak, a.maxLoad, o, me, st, L0)
-                                    : break_link<LP>(a.bendBreak, a.maxLoad, me, o, st, L0);
-                if (nst != st) {
-                    a.sState[si] = nst;
-                    a.linkState[__ldg(a.sLink + si)] = nst;  // both sides write the same value
-                    if (nst == 0 && !(pw & kSideIsB)) {
-                        unsigned long long slot = atomicAdd(a.eventCount, 1ull);
-                        if ((long long)slot < a.eventCap)
-                            a.events[slot] = make_int2(__ldg(a.sLink + si), (int)a.breakStep);
-                    }
-                    st = nst;
-                }
+                st = pending_break<LP>(a, (unsigned)si, pw, me, o, st, sl0[q], x, y, z);
             }
-            const LP mask = (st == 0) ? LP(0) : LP(1);
             LP CT[6];
 #pragma unroll
             for (int u = 0; u < 6; ++u) CT[u] = sct[u * ctStride + q];
             LP s[6];
 #pragma unroll
             for (int u = 0; u < 6; ++u) s[u] = od[u * 32 + lane];
+            Six<LP> dpv, ctv;
+            beam_terms(c, R, st != 0, x, y, z, Six<LP>::of(s), Six<LP>::of(o.d), CT, dpv, ctv);
             LP dp[6], ctt[6];
-            beam_terms<LP>(c, mask, (LP)(ox[lane] - o.x), (LP)(ox[32 + lane] - o.y),
-                           (LP)(ox[64 + lane] - o.z), s, o.d, CT, dp, ctt);
+            dpv.get(dp);
+            ctv.get(ctt);
 #pragma unroll
             for (int u = 0; u < 6; ++u) a.ct[u][si] = CT[u];
 #pragma unroll
@@ -1092,22 +1332,17 @@ __device__ __forceinline__ void step_items_block(const Consts<LP> &c, const Step
 #pragma unroll
                 for (int u = 0; u < 6; ++u) {
                     F[u] = F[u] + ts[(k * 12 + u) * 32 + t];
-                    F[u] = F[u] + ts[(k * 12 + 6 + u) * 32 + t];
+                    F[u] = F[u] - ts[(k * 12 + 6 + u) * 32 + t];
                 }
             }
-            if (FUSED) {
-                PRec<LP> me = own[t];
-                integrate_particle<LP>(c, me, __ldg(a.type + i), F);
-                store_rec(a.out + i, me);
-                dmax[0] = me.d[0] > LP(0) ? me.d[0] : LP(0);
-                dmax[1] = me.d[1] > LP(0) ? me.d[1] : LP(0);
-                dmax[2] = me.d[2] > LP(0) ? me.d[2] : LP(0);
-            } else {
-#pragma unroll
-                for (int u = 0; u < 6; ++u) a.force[(long long)u * a.n + i] = F[u];
-            }
+            PRec<LP> me = own[t];
+            integrate_particle<LP>(c, me, __ldg(a.type + i), F);
+            store_rec(a.out + i, me);
+            dmax[0] = me.d[0] > LP(0) ? me.d[0] : LP(0);
+            dmax[1] = me.d[1] > LP(0) ? me.d[1] : LP(0);
+            dmax[2] = me.d[2] > LP(0) ? me.d[2] : LP(0);
         }
-        if (FUSED && a.reduceDiff) {
+        if (a.reduceDiff) {
 #pragma unroll
             for (int u = 0; u < 3; ++u) {
                 LP v = dmax[u];
@@ -1121,11 +1356,11 @@ __device__ __forceinline__ void step_items_block(const Consts<LP> &c, const Step
     }
 }
 
-template <class LP, bool FUSED>
+template <class LP>
 __global__ void __launch_bounds__(kItemThreads)
     k_step_items(const Consts<LP> c, const StepArgs<LP> a) {
     extern __shared__ __align__(128) unsigned char smem[];
-    step_items_block<LP, FUSED>(c, a, blockIdx.x, smem);
+    step_items_block<LP>(c, a, blockIdx.x, smem);
 }
 
 // One fused step of many independent contexts in one launch. CTA b belongs to the entry
@@ -1169,9 +1404,9 @@ __global__ void __launch_bounds__(KIND == HIDEM_STEP_KERNEL_ITEMS ? kItemThreads
     if (e.reduceEvery10 && sa.step % 10 == 0 && lb == 0 && threadIdx.x < 3)
         sa.diffMax[threadIdx.x] = 0ull;
     if (KIND == HIDEM_STEP_KERNEL_ITEMS)
-        step_items_block<LP, true>(c, sa, lb, smem);
+        step_items_block<LP>(c, sa, lb, smem);
     else
-        step_thread_particle<LP, true>(c, sa, lb * kStepThreads + threadIdx.x);
+        step_thread_particle<LP>(c, sa, lb * kStepThreads + threadIdx.x);
 }
 
 // ---- the two-pass step over a batch (three launches per step and group) ----
@@ -1188,8 +1423,20 @@ __global__ void k_block_table(const int *__restrict__ offs, int *__restrict__ tb
     for (int i = a + threadIdx.x; i < b; i += blockDim.x) tbl[i] = e;
 }
 
+// The gather layout of every entry's records (in the record buffer the run does not step in),
+// at the start of a run.
 template <class LP>
-__global__ void __launch_bounds__(kStepThreads, kCapBlocksForces<LP>)
+__global__ void __launch_bounds__(kStepThreads)
+    k_gather_batch(const BatchEntry<LP> *__restrict__ entries, const int *__restrict__ firstBlocks,
+                   const int *__restrict__ blockEntry) {
+    const int ei = batch_entry(blockEntry);
+    const BatchEntry<LP> &e = entries[ei];
+    const int i = ((int)blockIdx.x - __ldg(firstBlocks + ei)) * kStepThreads + threadIdx.x;
+    if (i < e.a.n) store_gather(reinterpret_cast<int4 *>(e.rec[e.cur0 ^ 1]), i, load_rec(e.rec[e.cur0] + i));
+}
+
+template <class LP>
+__global__ void __launch_bounds__(kStepThreads, kForceBlocks<LP>)
     k_force_batch(const Consts<LP> c, const BatchEntry<LP> *__restrict__ entries,
                   const int *__restrict__ firstBlocks, const int *__restrict__ blockEntry, int s) {
     // the context's arguments in shared memory, where the per-particle loop reads them as
@@ -1200,42 +1447,35 @@ __global__ void __launch_bounds__(kStepThreads, kCapBlocksForces<LP>)
     const BatchEntry<LP> &e = entries[ei];
     if (threadIdx.x == 0) {
         StepArgs<LP> a = e.a;
-        a.in = e.rec[e.cur0];
-        a.out = e.rec[e.cur0];
+        a.gather = reinterpret_cast<int4 *>(e.rec[e.cur0 ^ 1]);
         a.step = e.step0 + s;
         a.breakPending = 0;
-        a.reduceDiff = 0;
         sa = a;
     }
     __syncthreads();
-    const int lb = (int)blockIdx.x - __ldg(firstBlocks + ei);
-    step_thread_particle<LP, false>(c, sa, lb * kStepThreads + threadIdx.x);
+    force_particle<LP, false, kForceAhead<LP>>(
+        c, sa, ((int)blockIdx.x - __ldg(firstBlocks + ei)) * kStepThreads + threadIdx.x);
 }
 
+// The integrate step on the gather layout, in place; the records too where rec is not null.
+// Streaming: 64 + 24 B read and 64 B (128 B with the records) written per particle (mixed).
 template <class LP>
-__global__ void __launch_bounds__(kStepThreads)
-    k_integrate_batch(const Consts<LP> c, const BatchEntry<LP> *__restrict__ entries,
-                      const int *__restrict__ firstBlocks, const int *__restrict__ blockEntry, int s) {
-    const int ei = batch_entry(blockEntry);
-    const BatchEntry<LP> &e = entries[ei];
-    const long long step = e.step0 + s;
-    const int lb = (int)blockIdx.x - __ldg(firstBlocks + ei);
-    const int i = lb * kStepThreads + threadIdx.x;
-    const int n = e.a.n;
-    PRec<LP> *rec = e.rec[e.cur0];
-    if (e.reduceEvery10 && step % 10 == 0 && lb == 0 && threadIdx.x < 3) e.a.diffMax[threadIdx.x] = 0ull;
+__device__ __forceinline__ void integrate_gather(const Consts<LP> &c, int4 *g, PRec<LP> *rec, const uint8_t *type,
+                                                 const LP *force, int n, int i, bool reduce,
+                                                 unsigned long long *diffMax) {
     LP dmax[3] = {LP(0), LP(0), LP(0)};
     if (i < n) {
-        PRec<LP> me = load_rec(rec + i);
+        PRec<LP> me = gather_rec<LP>(g, i);
         LP F[6];
 #pragma unroll
-        for (int q = 0; q < 6; ++q) F[q] = e.a.force[(long long)q * n + i];
-        integrate_particle<LP>(c, me, e.a.type[i], F);
-        store_rec(rec + i, me);
+        for (int q = 0; q < 6; ++q) F[q] = force[(long long)q * n + i];
+        integrate_particle<LP>(c, me, type[i], F);
+        store_gather(g, i, me);
+        if (rec) store_rec(rec + i, me);
 #pragma unroll
         for (int q = 0; q < 3; ++q) dmax[q] = me.d[q] > LP(0) ? me.d[q] : LP(0);
     }
-    if (e.reduceEvery10 && (step + 1) % 10 == 0) {
+    if (reduce) {
 #pragma unroll
         for (int q = 0; q < 3; ++q) {
             LP m = dmax[q];
@@ -1243,15 +1483,37 @@ __global__ void __launch_bounds__(kStepThreads)
                 LP u = __shfl_xor_sync(0xffffffffu, m, o);
                 m = (u > m) ? u : m;
             }
-            if ((threadIdx.x & 31) == 0 && m > LP(0)) atomicMax(e.a.diffMax + q, max_bits(m));
+            if ((threadIdx.x & 31) == 0 && m > LP(0)) atomicMax(diffMax + q, max_bits(m));
         }
     }
 }
 
+template <class LP>
+__global__ void __launch_bounds__(kStepThreads)
+    k_integrate_gather(const Consts<LP> c, int4 *g, PRec<LP> *rec, const uint8_t *__restrict__ type,
+                       const LP *__restrict__ force, int n, bool reduce, unsigned long long *diffMax) {
+    integrate_gather<LP>(c, g, rec, type, force, n, blockIdx.x * blockDim.x + threadIdx.x, reduce, diffMax);
+}
+
+template <class LP>
+__global__ void __launch_bounds__(kStepThreads)
+    k_integrate_batch(const Consts<LP> c, const BatchEntry<LP> *__restrict__ entries,
+                      const int *__restrict__ firstBlocks, const int *__restrict__ blockEntry, int s, bool last) {
+    const int ei = batch_entry(blockEntry);
+    const BatchEntry<LP> &e = entries[ei];
+    const long long step = e.step0 + s;
+    const int lb = (int)blockIdx.x - __ldg(firstBlocks + ei);
+    if (e.reduceEvery10 && step % 10 == 0 && lb == 0 && threadIdx.x < 3) e.a.diffMax[threadIdx.x] = 0ull;
+    integrate_gather<LP>(c, reinterpret_cast<int4 *>(e.rec[e.cur0 ^ 1]), last ? e.rec[e.cur0] : nullptr, e.a.type,
+                         e.a.force, e.a.n, lb * kStepThreads + threadIdx.x,
+                         e.reduceEvery10 && (step + 1) % 10 == 0, e.a.diffMax);
+}
+
 // The break pass of the batch: one thread per link over a grid of its own (the links of
 // entry e take CTAs [linkFirst[e], linkFirst[e + 1]), linkEntry maps a CTA to its entry),
-// so that each thread's two record gathers are in flight beside every other thread's, as
-// in the single-context pass.
+// so that each thread's two gathers are in flight beside every other thread's, as in the
+// single-context pass. Positions and rotations come from the gather layout; the functor's
+// root and division are left to the links near the threshold (stays_whole).
 template <class LP>
 __global__ void __launch_bounds__(kStepThreads)
     k_break_batch(const Consts<LP> c, const BatchEntry<LP> *__restrict__ entries,
@@ -1264,10 +1526,14 @@ __global__ void __launch_bounds__(kStepThreads)
     if ((LP)((LP)step * c.dt) > c.breakTime && l < e.L) {
         const uint8_t st = e.a.linkState[l];
         if (st != 0) {
-            const PRec<LP> *rec = e.rec[e.cur0];
-            const PRec<LP> pa = load_rec(rec + __ldg(e.slotA + l));
-            const PRec<LP> pb = load_rec(rec + __ldg(e.slotB + l));
-            const uint8_t nst = break_link<LP>(e.a.bendBreak, e.a.maxLoad, pa, pb, st, __ldg(e.L0link + l));
+            const int4 *g = reinterpret_cast<const int4 *>(e.rec[e.cur0 ^ 1]);
+            Body<LP> pa, pb;
+            load_body<true, true>(pa, g, __ldg(e.slotA + l));
+            load_body<true, true>(pb, g, __ldg(e.slotB + l));
+            const LP L0 = __ldg(e.L0link + l);
+            const LP x = (LP)(pa.x - pb.x), y = (LP)(pa.y - pb.y), z = (LP)(pa.z - pb.z);
+            if (stays_whole<LP>(e.a, x * x + y * y + z * z, pa.th, pb.th, L0)) return;
+            const uint8_t nst = break_link<LP>(e.a.bendBreak, e.a.maxLoad, pa, pb, st, L0);
             if (nst != st) {
                 e.a.linkState[l] = nst;
                 e.a.sState[e.sideSlot[2 * l]] = nst;
@@ -1472,8 +1738,8 @@ void launch_side_fill(const int *orig, int n, const int *slotOf, const int *plSt
 }
 
 template <class LP>
-void launch_step(const Consts<LP> &c, const StepArgs<LP> &a0, bool fused, int maxContacts,
-                 int maxEnds, int kernel, cudaStream_t s) {
+void launch_step(const Consts<LP> &c, const StepArgs<LP> &a0, int maxContacts, int maxEnds, int kernel,
+                 cudaStream_t s) {
     StepArgs<LP> a = a0;
     a.maxContacts = maxContacts;
     a.maxEnds = maxEnds;
@@ -1481,43 +1747,58 @@ void launch_step(const Consts<LP> &c, const StepArgs<LP> &a0, bool fused, int ma
     if (kernel == HIDEM_STEP_KERNEL_ITEMS && L.total <= kItemSmemLimit) {
         // the shared-memory limit is a per-device attribute: set it once on each device
         // (setting it twice, as racing threads may, is harmless)
-        static std::atomic<unsigned long long> configured[2];
+        static std::atomic<unsigned long long> configured;
         int dev = 0;
         cudaGetDevice(&dev);
         const unsigned long long bit = 1ull << (dev & 63);
-        if (!(configured[fused ? 1 : 0].load() & bit)) {
-            if (fused)
-                cudaFuncSetAttribute(k_step_items<LP, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kItemSmemLimit);
-            else
-                cudaFuncSetAttribute(k_step_items<LP, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kItemSmemLimit);
-            configured[fused ? 1 : 0].fetch_or(bit);
+        if (!(configured.load() & bit)) {
+            cudaFuncSetAttribute(k_step_items<LP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kItemSmemLimit);
+            configured.fetch_or(bit);
         }
-        const int nb = nblk(a.n, 32);
-        if (fused)
-            k_step_items<LP, true><<<nb, kItemThreads, L.total, s>>>(c, a);
-        else
-            k_step_items<LP, false><<<nb, kItemThreads, L.total, s>>>(c, a);
+        k_step_items<LP><<<nblk(a.n, 32), kItemThreads, L.total, s>>>(c, a);
         return;
     }
     // one thread per particle (also for rows too wide for the item kernel's buffers)
     const int nb = nblk(a.n, kStepThreads);
-    if (kernel == HIDEM_STEP_KERNEL_THREAD_ASYNC) {
-        const size_t sm = async_smem_bytes<LP>();
-        if (fused)
-            k_step_async<LP, true, kAsyncBlocks<LP>><<<nb, kStepThreads, sm, s>>>(c, a);
-        else
-            k_step_async<LP, false, kAsyncBlocks<LP>><<<nb, kStepThreads, sm, s>>>(c, a);
-    } else if (kernel == HIDEM_STEP_KERNEL_THREAD_CAPPED) {
-        if (fused)
-            k_step<LP, true, kCapBlocks<LP>><<<nb, kStepThreads, 0, s>>>(c, a);
-        else
-            k_step<LP, false, kCapBlocksForces<LP>><<<nb, kStepThreads, 0, s>>>(c, a);
-    } else {
-        if (fused)
-            k_step<LP, true, kThreadBlocks<LP>><<<nb, kStepThreads, 0, s>>>(c, a);
-        else
-            k_step<LP, false, kThreadBlocks<LP>><<<nb, kStepThreads, 0, s>>>(c, a);
-    }
+    if (kernel == HIDEM_STEP_KERNEL_THREAD_ASYNC)
+        k_step_async<LP, kAsyncBlocks<LP>><<<nb, kStepThreads, async_smem_bytes<LP>(), s>>>(c, a);
+    else if (kernel == HIDEM_STEP_KERNEL_THREAD_CAPPED)
+        k_step<LP, kCapBlocks<LP>><<<nb, kStepThreads, 0, s>>>(c, a);
+    else
+        k_step<LP, kThreadBlocks<LP>><<<nb, kStepThreads, 0, s>>>(c, a);
+}
+
+template <class LP, bool AHEAD, int MINB>
+static void launch_force_as(const Consts<LP> &c, const StepArgs<LP> &a, cudaStream_t s) {
+    const int nb = nblk(a.n, kStepThreads);
+    if (a.breakPending)
+        k_force<LP, true, AHEAD, MINB><<<nb, kStepThreads, 0, s>>>(c, a);
+    else
+        k_force<LP, false, AHEAD, MINB><<<nb, kStepThreads, 0, s>>>(c, a);
+}
+
+// A particle set that fits the chip in one wave at kFewBlocks CTAs an SM gains nothing from
+// more warps an SM: it takes the variant that keeps the next item in flight.
+template <class LP>
+void launch_force(const Consts<LP> &c, const StepArgs<LP> &a, int smCount, cudaStream_t s) {
+    if (nblk(a.n, kStepThreads) <= kFewBlocks<LP> * smCount)
+        launch_force_as<LP, true, kFewBlocks<LP>>(c, a, s);
+    else
+        launch_force_as<LP, kForceAhead<LP>, kForceBlocks<LP>>(c, a, s);
+}
+
+template <class LP>
+void launch_to_gather(const PRec<LP> *rec, int n, int4 *g, cudaStream_t s) {
+    k_to_gather<LP><<<nblk(n, 256), 256, 0, s>>>(rec, n, g);
+}
+template <class LP>
+void launch_from_gather(const int4 *g, int n, PRec<LP> *rec, cudaStream_t s) {
+    k_from_gather<LP><<<nblk(n, 256), 256, 0, s>>>(g, n, rec);
+}
+template <class LP>
+void launch_integrate_gather(const Consts<LP> &c, int4 *g, PRec<LP> *rec, const uint8_t *type, const LP *force,
+                             int n, bool reduce, unsigned long long *diffMax, cudaStream_t s) {
+    k_integrate_gather<LP><<<nblk(n, kStepThreads), kStepThreads, 0, s>>>(c, g, rec, type, force, n, reduce, diffMax);
 }
 
 template <class LP>
@@ -1557,11 +1838,17 @@ void launch_step_batch(const Consts<LP> &c, const BatchEntry<LP> *entries, const
 }
 
 template <class LP>
+void launch_gather_batch(const BatchEntry<LP> *entries, const int *firstBlocks, const int *blockEntry,
+                         int totalBlocks, cudaStream_t s) {
+    k_gather_batch<LP><<<totalBlocks, kStepThreads, 0, s>>>(entries, firstBlocks, blockEntry);
+}
+
+template <class LP>
 void launch_two_pass_batch(const Consts<LP> &c, const BatchEntry<LP> *entries, const int *firstBlocks,
-                           const int *blockEntry, const int *linkFirst, const int *linkEntry, int run,
+                           const int *blockEntry, const int *linkFirst, const int *linkEntry, int run, bool last,
                            int totalBlocks, int totalLinkBlocks, cudaStream_t s) {
     k_force_batch<LP><<<totalBlocks, kStepThreads, 0, s>>>(c, entries, firstBlocks, blockEntry, run);
-    k_integrate_batch<LP><<<totalBlocks, kStepThreads, 0, s>>>(c, entries, firstBlocks, blockEntry, run);
+    k_integrate_batch<LP><<<totalBlocks, kStepThreads, 0, s>>>(c, entries, firstBlocks, blockEntry, run, last);
     k_break_batch<LP><<<totalLinkBlocks, kStepThreads, 0, s>>>(c, entries, linkFirst, linkEntry, run);
 }
 
@@ -1730,15 +2017,22 @@ void launch_max_diff(const PRec<LP> *rec, int n, unsigned long long *out, int nb
                                        const uint8_t *, const int *, const int *, const LP *,      \
                                        const int *, const SideView<LP> &, const long long *,       \
                                        const SideView<LP> &, int *, cudaStream_t);                 \
-    template void launch_step<LP>(const Consts<LP> &, const StepArgs<LP> &, bool, int, int, int,     \
+    template void launch_step<LP>(const Consts<LP> &, const StepArgs<LP> &, int, int, int,          \
                                   cudaStream_t);                                                   \
+    template void launch_force<LP>(const Consts<LP> &, const StepArgs<LP> &, int, cudaStream_t);           \
+    template void launch_to_gather<LP>(const PRec<LP> *, int, int4 *, cudaStream_t);               \
+    template void launch_from_gather<LP>(const int4 *, int, PRec<LP> *, cudaStream_t);             \
+    template void launch_integrate_gather<LP>(const Consts<LP> &, int4 *, PRec<LP> *, const uint8_t *, \
+                                              const LP *, int, bool, unsigned long long *, cudaStream_t); \
     template bool batch_fits<LP>(int, int);                                                        \
     template void prepare_step_batch<LP>();                                                        \
     template void launch_step_batch<LP>(const Consts<LP> &, const BatchEntry<LP> *, const int *,     \
                                         const int *, int, int, int, int, int, cudaStream_t);       \
+    template void launch_gather_batch<LP>(const BatchEntry<LP> *, const int *, const int *, int,    \
+                                          cudaStream_t);                                           \
     template void launch_two_pass_batch<LP>(const Consts<LP> &, const BatchEntry<LP> *, const int *, \
-                                            const int *, const int *, const int *, int, int, int,  \
-                                            cudaStream_t);                                         \
+                                            const int *, const int *, const int *, int, bool, int,  \
+                                            int, cudaStream_t);                                    \
     template void launch_integrate<LP>(const Consts<LP> &, PRec<LP> *, const uint8_t *,            \
                                        const LP *, int, cudaStream_t);                             \
     template void launch_link_break<LP>(const Consts<LP> &, const PRec<LP> *, const int *,         \

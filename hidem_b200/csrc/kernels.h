@@ -136,13 +136,26 @@ void launch_side_fill(const int *orig, int n, const int *slotOf, const int *plSt
                       const LP *L0link, const int *sideSlotOld, const SideView<LP> &oldS,
                       const long long *sOff, const SideView<LP> &newS, int *sideSlotNew,
                       cudaStream_t s);
-// One timestep's forces (fused: + previous link update, integrate, record swap) for
-// rows of at most maxContacts contacts and maxEnds link ends, by the kernel `kernel`
-// (HIDEM_STEP_KERNEL_*, not AUTO; the item kernel falls back to one thread per particle
-// for rows too wide for its shared-memory buffers).
+// One fused timestep (previous link update, forces, integrate, record swap) for rows of at
+// most maxContacts contacts and maxEnds link ends, by the kernel `kernel`
+// (HIDEM_STEP_KERNEL_*, not AUTO or TWO_PASS; the item kernel falls back to one thread per
+// particle for rows too wide for its shared-memory buffers).
 template <class LP>
-void launch_step(const Consts<LP> &c, const StepArgs<LP> &a, bool fused, int maxContacts,
-                 int maxEnds, int kernel, cudaStream_t s);
+void launch_step(const Consts<LP> &c, const StepArgs<LP> &a, int maxContacts, int maxEnds, int kernel,
+                 cudaStream_t s);
+// The force pass (a.gather holds the records in the gather layout), applying the previous
+// step's link update on the way when a.breakPending; the integrate pass on the gather layout
+// (rec: the records too, or null; reduce: the diff maxima into diffMax); and the two layouts'
+// conversions (a gather buffer holds whole blocks of 32 slots).
+template <class LP>
+void launch_force(const Consts<LP> &c, const StepArgs<LP> &a, int smCount, cudaStream_t s);
+template <class LP>
+void launch_integrate_gather(const Consts<LP> &c, int4 *g, PRec<LP> *rec, const uint8_t *type, const LP *force,
+                             int n, bool reduce, unsigned long long *diffMax, cudaStream_t s);
+template <class LP>
+void launch_to_gather(const PRec<LP> *rec, int n, int4 *g, cudaStream_t s);
+template <class LP>
+void launch_from_gather(const int4 *g, int n, PRec<LP> *rec, cudaStream_t s);
 // One context's share of a batched step launch (the constants other than the break
 // thresholds, which travel in `a`, are the launch's). The per-step fields of `a` (in, out,
 // step, breakPending, breakStep, reduceDiff) are not read: launch s of a run derives them
@@ -181,13 +194,18 @@ void launch_step_batch(const Consts<LP> &c, const BatchEntry<LP> *entries, const
                        const int *blockEntry, int run, int totalBlocks, int maxContacts, int maxEnds,
                        int kernel, cudaStream_t s);
 
-// the two-pass step over a run's entries: force pass, integrate pass (in place, with the
-// diff maxima every 10 steps) over the particles' CTAs (firstBlocks, blockEntry,
-// totalBlocks as for the thread kernels); break pass (when t dt > breakTime) over the links'
-// CTAs (linkFirst, linkEntry, totalLinkBlocks: kStepThreads links per CTA)
+// the gather layout of every entry's records (firstBlocks, blockEntry, totalBlocks as for the
+// thread kernels)
+template <class LP>
+void launch_gather_batch(const BatchEntry<LP> *entries, const int *firstBlocks, const int *blockEntry,
+                         int totalBlocks, cudaStream_t s);
+// the two-pass step over a run's entries, on the gather layout: force pass, integrate pass in
+// place (with the diff maxima every 10 steps; last: the records written too) over the
+// particles' CTAs; break pass (when t dt > breakTime) over the links' CTAs (linkFirst,
+// linkEntry, totalLinkBlocks: kStepThreads links per CTA)
 template <class LP>
 void launch_two_pass_batch(const Consts<LP> &c, const BatchEntry<LP> *entries, const int *firstBlocks,
-                           const int *blockEntry, const int *linkFirst, const int *linkEntry, int run,
+                           const int *blockEntry, const int *linkFirst, const int *linkEntry, int run, bool last,
                            int totalBlocks, int totalLinkBlocks, cudaStream_t s);
 
 template <class LP>

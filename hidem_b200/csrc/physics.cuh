@@ -13,152 +13,445 @@ __device__ __forceinline__ double lsqrt(double v) { return sqrt(v); }
 __device__ __forceinline__ float labs_(float v) { return fabsf(v); }
 __device__ __forceinline__ double labs_(double v) { return fabs(v); }
 
+// ---- six-component values: (x, u), (y, v), (z, w) as pairs in single precision ----
+//
+// The mixed build's functors are bound by instruction issue (the force pass issues about 500
+// instructions per contact and link end with scalar arithmetic), and sm_100's packed
+// instructions do two IEEE single-precision operations per issue slot (same rounding per
+// component; the FP32 pipe's rate is unchanged: 0.48 packed against 0.95 scalar instructions
+// per clock and scheduler measured). A translational component and its rotational partner
+// take the same operations with the same transformation entries, so they form the pairs.
+struct Pair {
+    unsigned long long v;
+};
+__device__ __forceinline__ Pair pair_of(float lo, float hi) {
+    Pair r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ Pair pair_of(float both) { return pair_of(both, both); }
+__device__ __forceinline__ void unpair(Pair p, float &lo, float &hi) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(p.v));
+}
+__device__ __forceinline__ Pair operator*(Pair a, Pair b) {
+    Pair r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ Pair operator+(Pair a, Pair b) {
+    Pair r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ Pair operator-(Pair a, Pair b) {
+    Pair r;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ Pair pair_fma(Pair a, Pair b, Pair c) {
+    Pair r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+    return r;
+}
+// A packed product that feeds a packed sum is a fused multiply-add onto -0 (the same rounding,
+// signed zeros included) whose -0 the compiler cannot see through: ptxas 12.9 contracts a
+// packed product and a packed sum into one fused operation even under -fmad=false and with
+// .rn on both (measured: 45 % of random a b + c d differ). The value comes out of a shuffle,
+// so it also stays in a register pair instead of being loaded again at each use.
+template <class LP>
+struct Rounding;
+template <>
+struct Rounding<float> {
+    Pair minusZero;
+    __device__ __forceinline__ static Rounding make() {
+        Rounding r;
+        r.minusZero.v = __shfl_sync(0xffffffffu, 0x8000000080000000ull, 0);
+        return r;
+    }
+    __device__ __forceinline__ Pair product(Pair a, Pair b) const { return pair_fma(a, b, minusZero); }
+};
+template <>
+struct Rounding<double> {
+    __device__ __forceinline__ static Rounding make() { return Rounding(); }
+};
+
+template <class LP>
+struct Six;
+template <>
+struct Six<float> {
+    Pair p[3];  // components (0, 3), (1, 4), (2, 5)
+    __device__ __forceinline__ static Six zero() {
+        Six r;
+#pragma unroll
+        for (int q = 0; q < 3; ++q) r.p[q].v = 0ull;
+        return r;
+    }
+    __device__ __forceinline__ static Six of(const float *f) {
+        Six r;
+#pragma unroll
+        for (int q = 0; q < 3; ++q) r.p[q] = pair_of(f[q], f[q + 3]);
+        return r;
+    }
+    __device__ __forceinline__ void get(float *f) const {
+#pragma unroll
+        for (int q = 0; q < 3; ++q) unpair(p[q], f[q], f[q + 3]);
+    }
+    __device__ __forceinline__ Six operator+(const Six &o) const {
+        Six r;
+#pragma unroll
+        for (int q = 0; q < 3; ++q) r.p[q] = p[q] + o.p[q];
+        return r;
+    }
+    __device__ __forceinline__ Six operator-(const Six &o) const {
+        Six r;
+#pragma unroll
+        for (int q = 0; q < 3; ++q) r.p[q] = p[q] - o.p[q];
+        return r;
+    }
+    __device__ __forceinline__ Six times(Pair k) const {
+        Six r;
+#pragma unroll
+        for (int q = 0; q < 3; ++q) r.p[q] = p[q] * k;
+        return r;
+    }
+    __device__ __forceinline__ Six times(const Rounding<float> &R, Pair k) const {
+        Six r;
+#pragma unroll
+        for (int q = 0; q < 3; ++q) r.p[q] = R.product(p[q], k);
+        return r;
+    }
+};
+template <>
+struct Six<double> {
+    double f[6];
+    __device__ __forceinline__ static Six zero() {
+        Six r;
+#pragma unroll
+        for (int q = 0; q < 6; ++q) r.f[q] = 0.0;
+        return r;
+    }
+    __device__ __forceinline__ static Six of(const double *v) {
+        Six r;
+#pragma unroll
+        for (int q = 0; q < 6; ++q) r.f[q] = v[q];
+        return r;
+    }
+    __device__ __forceinline__ void get(double *v) const {
+#pragma unroll
+        for (int q = 0; q < 6; ++q) v[q] = f[q];
+    }
+    __device__ __forceinline__ Six operator+(const Six &o) const {
+        Six r;
+#pragma unroll
+        for (int q = 0; q < 6; ++q) r.f[q] = f[q] + o.f[q];
+        return r;
+    }
+    __device__ __forceinline__ Six operator-(const Six &o) const {
+        Six r;
+#pragma unroll
+        for (int q = 0; q < 6; ++q) r.f[q] = f[q] - o.f[q];
+        return r;
+    }
+};
+
+// ---- correctly rounded square root, reciprocal and quotient from one approximate 1/sqrt ----
+//
+// The functors take square roots, their reciprocals and quotients by powers of them. Each is
+// IEEE-rounded in the reference; here they share one approximate reciprocal square root r and
+// are brought to the correctly rounded value by fused multiply-add residuals (P. Markstein,
+// "Computation of elementary functions on the IBM RISC System/6000 processor", IBM J. Res.
+// Dev. 34 (1990) 111-119), valid for arguments in [2^-90, 2^90] (roots) whose intermediate
+// powers stay clear of the denormals; callers take the plain IEEE operations outside.
+//   root:        g = v r, s = g + (v - g^2) (r / 2). Equal to the IEEE root for every
+//                significand and exponent parity (checked exhaustively, tests/test_gpu_rounding.py).
+//   reciprocal:  y1 = y0 + y0 (1 - b y0), y = y1 + y1 (1 - b y1). Equal to the IEEE reciprocal
+//                for every significand but the all-ones one, whose iteration ends in a tie:
+//                squared lengths with such a root (tie_root) take the IEEE operations.
+//   quotient:    q1 = q0 + y (a - b q0), q = q1 + y (a - b q1) with y the rounded 1/b: the
+//                IEEE quotient for every divisor but one of all ones (all_ones).
+__device__ __forceinline__ float rsqrt_start(float v) {
+    float r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
+    return r;
+}
+__device__ __forceinline__ float root_from(float v, float r) {
+    const float g = v * r;
+    return __fmaf_rn(__fmaf_rn(-g, g, v), 0.5f * r, g);
+}
+__device__ __forceinline__ float recip_from(float b, float y0) {
+    const float y1 = __fmaf_rn(y0, __fmaf_rn(-b, y0, 1.0f), y0);
+    return __fmaf_rn(y1, __fmaf_rn(-b, y1, 1.0f), y1);
+}
+// (the quotient's three steps from the rounded reciprocal y of b)
+__device__ __forceinline__ float quotient_from(float a, float b, float y) {
+    const float q0 = a * y;
+    const float q1 = __fmaf_rn(__fmaf_rn(-b, q0, a), y, q0);
+    return __fmaf_rn(__fmaf_rn(-b, q1, a), y, q1);
+}
+// the two largest values below an even power of two: their roots round to all ones
+__device__ __forceinline__ bool tie_root(float v) { return ((__float_as_uint(v) ^ 0x007ffffeu) & 0x00fffffeu) == 0u; }
+__device__ __forceinline__ bool all_ones(float v) { return (~__float_as_uint(v) & 0x007fffffu) == 0u; }
+constexpr float kFastLo = 9.094947017729282e-13f;  // 2^-40
+constexpr float kFastHi = 1.099511627776e12f;      // 2^40
+constexpr float kRootLo = 8.077935669463161e-28f;  // 2^-90
+constexpr float kRootHi = 1.2379400392853803e27f;  // 2^90
+
 // Contact / damping between two particles: HiDEMDefNeighForceFunc::operator()
 // (HiDEMDefaultFunctions.h:21-87). s = self (xDiff..wDiff), sr its radius, o / orr the
-// other. contact_terms returns the six values the functor adds to the forces; adding
-// them to F in component order is exactly the functor's update.
-template <class LP>
-__device__ __forceinline__ void contact_terms(const Consts<LP> &c, LP mask, LP xDist, LP yDist,
-                                              LP zDist, const LP *s, LP sr, const LP *o, LP orr,
-                                              LP *t) {
-    LP xDist2 = xDist * xDist;
-    LP yDist2 = yDist * yDist;
-    LP zDist2 = zDist * zDist;
-    LP particleDistance2 = xDist2 + yDist2 + zDist2;
-    LP radSum = sr + orr;
-    LP activeDist2 = (radSum + c.attractDistance) * (radSum + c.attractDistance);
-    mask = (particleDistance2 >= activeDist2) ? LP(0) : mask;
-    LP particleDistance = lsqrt(particleDistance2);
-    LP invDist = LP(1) / particleDistance;
-    LP xComp = xDist * invDist;
-    LP yComp = yDist * invDist;
-    LP zComp = zDist * invDist;
-    LP Cnst = 0;
-    LP dimDist = radSum - particleDistance;
-    Cnst = (particleDistance < radSum) ? lsqrt(dimDist * dimDist * dimDist) : Cnst;
-    Cnst = (particleDistance >= radSum && particleDistance < radSum + c.attractDistance)
-               ? c.attractScaleForce * dimDist
-               : Cnst;
-    Cnst = Cnst * c.scaleE;
-    t[0] = mask * ((-c.damping) * ((s[0] - o[0]) * c.invDt) + (Cnst * xComp));
-    t[1] = mask * ((-c.damping) * ((s[1] - o[1]) * c.invDt) + (Cnst * yComp));
-    t[2] = mask * ((-c.damping) * ((s[2] - o[2]) * c.invDt) + (Cnst * zComp));
-    t[3] = mask * ((-c.dampingRotation) * ((s[3] - o[3]) * c.invDt));
-    t[4] = mask * ((-c.dampingRotation) * ((s[4] - o[4]) * c.invDt));
-    t[5] = mask * ((-c.dampingRotation) * ((s[5] - o[5]) * c.invDt));
-}
-
+// other. Adds the six values the functor adds to the forces, in component order.
+//
 // A pair beyond the active distance gets mask 0, and every term the functor adds is then
 // 0 times a finite value (the distance is positive there): adding those signed zeros
 // leaves each force component's value unchanged (a zero component at most changes its
 // sign, which no later operation can observe), so such pairs skip the arithmetic. A NaN
-// distance fails the comparison and takes the full path, as in the functor.
-template <class LP>
-__device__ __forceinline__ void contact_pair(const Consts<LP> &c, LP mask, LP xDist, LP yDist,
-                                             LP zDist, const LP *s, LP sr, const LP *o, LP orr,
-                                             LP *F) {
-    {
-        const LP particleDistance2 = xDist * xDist + yDist * yDist + zDist * zDist;
-        const LP radSum = sr + orr;
-        const LP activeDist2 = (radSum + c.attractDistance) * (radSum + c.attractDistance);
-        if (particleDistance2 >= activeDist2) return;
+// distance fails the comparison and takes the full path, as in the functor, whose mask
+// of 1 multiplies nothing here. contact_terms writes the values for an in-range pair (the
+// item kernel's zeros for a skipped one) and returns whether there are any.
+__device__ __forceinline__ bool contact_terms(const Consts<float> &c, const Rounding<float> &R, float xDist, float yDist, float zDist,
+                                              const Six<float> &s, float sr, const Six<float> &o, float orr,
+                                              Six<float> &t) {
+    const float d2 = xDist * xDist + yDist * yDist + zDist * zDist;
+    const float radSum = sr + orr;
+    if (d2 >= (radSum + c.attractDistance) * (radSum + c.attractDistance)) return false;
+    float dist, inv;
+    if (d2 >= kFastLo && d2 < kFastHi && !tie_root(d2)) {
+        const float r = rsqrt_start(d2);
+        dist = root_from(d2, r);
+        inv = recip_from(dist, r);
+    } else {
+        dist = sqrtf(d2);
+        inv = 1.0f / dist;
     }
-    LP t[6];
-    contact_terms<LP>(c, mask, xDist, yDist, zDist, s, sr, o, orr, t);
+    const float dim = radSum - dist;
+    float Cnst = 0.f;
+    if (dist < radSum) {
+        const float d3 = dim * dim * dim;
+        Cnst = (d3 >= kRootLo && d3 < kRootHi) ? root_from(d3, rsqrt_start(d3)) : sqrtf(d3);
+    }
+    if (dist >= radSum && dist < radSum + c.attractDistance) Cnst = c.attractScaleForce * dim;
+    Cnst = Cnst * c.scaleE;
+    t = (s - o).times(pair_of(c.invDt)).times(R, pair_of(-c.damping, -c.dampingRotation));
+    const float comp[3] = {Cnst * (xDist * inv), Cnst * (yDist * inv), Cnst * (zDist * inv)};
 #pragma unroll
-    for (int k = 0; k < 6; ++k) F[k] = F[k] + t[k];
+    for (int q = 0; q < 3; ++q) {
+        float a, b;
+        unpair(t.p[q], a, b);
+        t.p[q] = pair_of(a + comp[q], b);
+    }
+    return true;
+}
+__device__ __forceinline__ bool contact_terms(const Consts<double> &c, const Rounding<double> &, double xDist, double yDist, double zDist,
+                                              const Six<double> &s, double sr, const Six<double> &o, double orr,
+                                              Six<double> &t) {
+    const double d2 = xDist * xDist + yDist * yDist + zDist * zDist;
+    const double radSum = sr + orr;
+    if (d2 >= (radSum + c.attractDistance) * (radSum + c.attractDistance)) return false;
+    const double dist = sqrt(d2);
+    const double inv = 1.0 / dist;
+    const double dim = radSum - dist;
+    double Cnst = 0.0;
+    Cnst = (dist < radSum) ? sqrt(dim * dim * dim) : Cnst;
+    Cnst = (dist >= radSum && dist < radSum + c.attractDistance) ? c.attractScaleForce * dim : Cnst;
+    Cnst = Cnst * c.scaleE;
+    const double comp[3] = {xDist * inv, yDist * inv, zDist * inv};
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+        t.f[q] = (-c.damping) * ((s.f[q] - o.f[q]) * c.invDt) + Cnst * comp[q];
+        t.f[q + 3] = (-c.dampingRotation) * ((s.f[q + 3] - o.f[q + 3]) * c.invDt);
+    }
+    return true;
 }
 
-// Bonded beam on one link end: HiDEMDefLinkForceFunc::operator()
-// (HiDEMDefaultFunctions.h:90-204). CT is this side's history state (in/out). The
-// functor adds two values to each force component, first the damping term (dp), later
-// the CT term (ct); beam_terms returns both, beam_side applies them in that order.
 template <class LP>
-__device__ __forceinline__ void beam_terms(const Consts<LP> &c, LP mask, LP xDist, LP yDist,
-                                           LP zDist, const LP *s, const LP *o, LP *CT, LP *dp,
-                                           LP *ct) {
-    dp[0] = (-c.linkDamping * ((s[0] - o[0]) * c.linkInvDt)) * mask;
-    dp[1] = (-c.linkDamping * ((s[1] - o[1]) * c.linkInvDt)) * mask;
-    dp[2] = (-c.linkDamping * ((s[2] - o[2]) * c.linkInvDt)) * mask;
-    dp[3] = (-c.linkDampingRotation * ((s[3] - o[3]) * c.linkInvDt)) * mask;
-    dp[4] = (-c.linkDampingRotation * ((s[4] - o[4]) * c.linkInvDt)) * mask;
-    dp[5] = (-c.linkDampingRotation * ((s[5] - o[5]) * c.linkInvDt)) * mask;
+__device__ __forceinline__ void contact_pair(const Consts<LP> &c, const Rounding<LP> &R, LP xDist, LP yDist, LP zDist,
+                                             const Six<LP> &s, LP sr, const Six<LP> &o, LP orr, Six<LP> &F) {
+    Six<LP> t;
+    if (contact_terms(c, R, xDist, yDist, zDist, s, sr, o, orr, t)) F = F + t;
+}
 
+// The beam functor's values of one link end's geometry: 1 / length, 1 / length in the xy
+// plane, the two squared lengths, and the stiffnesses E W4 / L^3 and E W4 / (2 L^2).
+template <class LP>
+struct BeamGeometry {
+    LP invLI, invLP, D, xy, K1, K5;
+};
+template <class LP>
+__device__ __forceinline__ BeamGeometry<LP> beam_geometry_ieee(const Consts<LP> &c, LP xDist, LP yDist, LP zDist) {
+    BeamGeometry<LP> g;
     LP xDist2 = xDist * xDist;
     LP yDist2 = yDist * yDist;
     if (xDist == LP(0) && yDist == LP(0)) {
         xDist2 = LP(1e-10);
         yDist2 = LP(1e-10);
     }
-    LP zDist2 = zDist * zDist;
-    LP distSum = xDist2 + yDist2 + zDist2;
-    LP invLI = LP(1) / lsqrt(distSum);
-    LP invLP = LP(1) / lsqrt(xDist2 + yDist2);
-    LP invLILP = invLI * invLP;
-    LP LI = invLI * distSum;
+    g.xy = xDist2 + yDist2;
+    g.D = g.xy + zDist * zDist;
+    g.invLI = LP(1) / lsqrt(g.D);
+    g.invLP = LP(1) / lsqrt(g.xy);
+    const LP LI = g.invLI * g.D;
+    const LP L2 = LI * LI;
+    const LP L3 = LI * LI * LI;
+    g.K1 = c.E * c.W4 / L3;
+    g.K5 = c.E * c.W4 / (LP(2) * L2);
+    return g;
+}
+// Two approximate reciprocal square roots (of the squared length and its xy part) start
+// everything: the two roots, their reciprocals, and, from the powers of 1 / length, the two
+// quotients; c.beamFastLo admits the arguments for which no intermediate value leaves
+// the normal numbers (it is infinite when E W4 itself is out of range).
+__device__ __forceinline__ BeamGeometry<float> beam_geometry(const Consts<float> &c, float xDist, float yDist,
+                                                             float zDist) {
+    const float xy = xDist * xDist + yDist * yDist;
+    const float D = xy + zDist * zDist;
+    if (!(xy >= c.beamFastLo && D < kFastHi) || tie_root(xy) || tie_root(D)) return beam_geometry_ieee<float>(c, xDist, yDist, zDist);
+    BeamGeometry<float> g;
+    g.xy = xy;
+    g.D = D;
+    const float rD = rsqrt_start(D), rxy = rsqrt_start(xy);
+    g.invLI = recip_from(root_from(D, rD), rD);
+    g.invLP = recip_from(root_from(xy, rxy), rxy);
+    const float LI = g.invLI * D;
+    const float L2 = LI * LI, L3 = L2 * LI;
+    const float i2 = g.invLI * g.invLI;
+    g.K1 = quotient_from(c.E * c.W4, L3, recip_from(L3, i2 * g.invLI));
+    g.K5 = quotient_from(c.E * c.W4, 2.0f * L2, recip_from(2.0f * L2, 0.5f * i2));
+    if (all_ones(L3) || all_ones(L2)) {
+        g.K1 = c.E * c.W4 / L3;
+        g.K5 = c.E * c.W4 / (2.0f * L2);
+    }
+    return g;
+}
+__device__ __forceinline__ BeamGeometry<double> beam_geometry(const Consts<double> &c, double xDist, double yDist,
+                                                              double zDist) {
+    return beam_geometry_ieee<double>(c, xDist, yDist, zDist);
+}
 
-    LP T00 = xDist * invLI, T01 = yDist * invLI, T02 = zDist * invLI;
-    LP T10 = -yDist * invLP, T11 = xDist * invLP;
-    LP T20 = -(zDist * xDist) * invLILP;
-    LP T21 = -(zDist * yDist) * invLILP;
-    LP T22 = (xDist2 + yDist2) * invLILP;
+// Bonded beam on one link end: HiDEMDefLinkForceFunc::operator()
+// (HiDEMDefaultFunctions.h:90-204). CT is this side's history state (in/out). The
+// functor adds two values to each force component, first the damping term (dp), later
+// minus the turned CT term (ct here): beam_side applies them in that order. The functor's
+// mask multiplies both: by 1 for a whole link, which changes nothing and is left out, and
+// by 0 for a broken one (whose products are zeros, or NaN where a term is not finite).
+__device__ __forceinline__ void beam_terms(const Consts<float> &c, const Rounding<float> &R, bool whole, float xDist, float yDist, float zDist,
+                                           const Six<float> &s, const Six<float> &o, float *CT, Six<float> &dp,
+                                           Six<float> &ct) {
+    dp = (s - o).times(pair_of(c.linkInvDt)).times(R, pair_of(-c.linkDamping, -c.linkDampingRotation));
+    const BeamGeometry<float> g = beam_geometry(c, xDist, yDist, zDist);
+    const float invLILP = g.invLI * g.invLP;
+    const Pair T00 = pair_of(xDist * g.invLI), T01 = pair_of(yDist * g.invLI), T02 = pair_of(zDist * g.invLI);
+    const Pair T10 = pair_of(-yDist * g.invLP), T11 = pair_of(xDist * g.invLP);
+    const Pair T20 = pair_of(-(zDist * xDist) * invLILP);
+    const Pair T21 = pair_of(-(zDist * yDist) * invLILP);
+    const Pair T22 = pair_of(g.xy * invLILP);
 
-    LP B0 = T00 * s[0] + T01 * s[1] + T02 * s[2];
-    LP B1 = T10 * s[0] + T11 * s[1];
-    LP B2 = T20 * s[0] + T21 * s[1] + T22 * s[2];
-    LP B4 = T10 * s[3] + T11 * s[4];
-    LP B5 = T20 * s[3] + T21 * s[4] + T22 * s[5];
-    LP B6 = T00 * o[0] + T01 * o[1] + T02 * o[2];
-    LP B7 = T10 * o[0] + T11 * o[1];
-    LP B8 = T20 * o[0] + T21 * o[1] + T22 * o[2];
-    LP B10 = T10 * o[3] + T11 * o[4];
-    LP B11 = T20 * o[3] + T21 * o[4] + T22 * o[5];
+    const Pair s03 = R.product(T00, s.p[0]) + R.product(T01, s.p[1]) + R.product(T02, s.p[2]);  // (B0, B3)
+    const Pair s14 = R.product(T10, s.p[0]) + R.product(T11, s.p[1]);                            // (B1, B4)
+    const Pair s25 = R.product(T20, s.p[0]) + R.product(T21, s.p[1]) + R.product(T22, s.p[2]);  // (B2, B5)
+    const Pair o03 = R.product(T00, o.p[0]) + R.product(T01, o.p[1]) + R.product(T02, o.p[2]);  // (B6, B9)
+    const Pair o14 = R.product(T10, o.p[0]) + R.product(T11, o.p[1]);                            // (B7, B10)
+    const Pair o25 = R.product(T20, o.p[0]) + R.product(T21, o.p[1]) + R.product(T22, o.p[2]);  // (B8, B11)
+    float B1, B4, B2, B5, B7, B10, B8, B11;
+    unpair(s14, B1, B4);
+    unpair(s25, B2, B5);
+    unpair(o14, B7, B10);
+    unpair(o25, B8, B11);
 
-    LP L2 = LI * LI;
-    LP L3 = LI * LI * LI;
-    LP LIDiv6 = (LP(1) / LP(6)) * invLI;
-    LP K0 = c.E * c.W2 * invLI;
-    LP K1 = c.E * c.W4 / L3;
-    LP K5 = c.E * c.W4 / (LP(2) * L2);
+    const float K1 = g.K1, K5 = g.K5;
+    const float LIDiv6 = (1.0f / 6.0f) * g.invLI;
+    const float K4 = c.E * c.W4 * LIDiv6;
+    const float K3 = K4 * 2.0f;
+    const Pair K02 = pair_of(c.E * c.W2 * g.invLI, c.G * c.W4 * LIDiv6);
+    const Pair c03 = pair_of(CT[0], CT[3]) + (R.product(K02, s03) - R.product(K02, o03));
+    // CT1 with CT5, CT2 with CT4: their four terms take the same B values
+    const Pair c15 = pair_of(CT[1], CT[5]) +
+                     (pair_of(K1 * B1, K5 * B1) + pair_of(K5 * B5, K3 * B5) - pair_of(K1 * B7, K5 * B7) +
+                      pair_of(K5 * B11, K4 * B11));
+    const Pair c24 = pair_of(CT[2], CT[4]) +
+                     (pair_of(K1 * B2, -K5 * B2) + pair_of(-K5 * B4, K3 * B4) - pair_of(K1 * B8, -K5 * B8) +
+                      pair_of(-K5 * B10, K4 * B10));
+    unpair(c03, CT[0], CT[3]);
+    unpair(c15, CT[1], CT[5]);
+    unpair(c24, CT[2], CT[4]);
+    const Pair c14 = pair_of(CT[1], CT[4]), c25 = pair_of(CT[2], CT[5]);
+    ct.p[0] = R.product(T00, c03) + R.product(T10, c14) + R.product(T20, c25);
+    ct.p[1] = R.product(T01, c03) + R.product(T11, c14) + R.product(T21, c25);
+    ct.p[2] = R.product(T02, c03) + R.product(T22, c25);
+    if (!whole) {
+        dp = dp.times(R, pair_of(0.f));
+        ct = ct.times(R, pair_of(0.f));
+    }
+}
+__device__ __forceinline__ void beam_terms(const Consts<double> &c, const Rounding<double> &, bool whole, double xDist, double yDist,
+                                           double zDist, const Six<double> &s, const Six<double> &o, double *CT,
+                                           Six<double> &dp, Six<double> &ct) {
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+        dp.f[q] = -c.linkDamping * ((s.f[q] - o.f[q]) * c.linkInvDt);
+        dp.f[q + 3] = -c.linkDampingRotation * ((s.f[q + 3] - o.f[q + 3]) * c.linkInvDt);
+    }
+    const BeamGeometry<double> g = beam_geometry(c, xDist, yDist, zDist);
+    const double invLI = g.invLI, invLP = g.invLP, invLILP = invLI * invLP;
+    const double T00 = xDist * invLI, T01 = yDist * invLI, T02 = zDist * invLI;
+    const double T10 = -yDist * invLP, T11 = xDist * invLP;
+    const double T20 = -(zDist * xDist) * invLILP;
+    const double T21 = -(zDist * yDist) * invLILP;
+    const double T22 = g.xy * invLILP;
 
+    const double B0 = T00 * s.f[0] + T01 * s.f[1] + T02 * s.f[2];
+    const double B1 = T10 * s.f[0] + T11 * s.f[1];
+    const double B2 = T20 * s.f[0] + T21 * s.f[1] + T22 * s.f[2];
+    const double B4 = T10 * s.f[3] + T11 * s.f[4];
+    const double B5 = T20 * s.f[3] + T21 * s.f[4] + T22 * s.f[5];
+    const double B6 = T00 * o.f[0] + T01 * o.f[1] + T02 * o.f[2];
+    const double B7 = T10 * o.f[0] + T11 * o.f[1];
+    const double B8 = T20 * o.f[0] + T21 * o.f[1] + T22 * o.f[2];
+    const double B10 = T10 * o.f[3] + T11 * o.f[4];
+    const double B11 = T20 * o.f[3] + T21 * o.f[4] + T22 * o.f[5];
+
+    const double LIDiv6 = (1.0 / 6.0) * invLI;
+    const double K0 = c.E * c.W2 * invLI;
+    const double K1 = g.K1, K5 = g.K5;
     CT[0] = CT[0] + (K0 * B0 + (-K0) * B6);
     CT[1] = CT[1] + (K1 * B1 + K5 * B5 + (-K1) * B7 + K5 * B11);
     CT[2] = CT[2] + (K1 * B2 + (-K5) * B4 + (-K1) * B8 + (-K5) * B10);
+    ct.f[0] = T00 * CT[0] + T10 * CT[1] + T20 * CT[2];
+    ct.f[1] = T01 * CT[0] + T11 * CT[1] + T21 * CT[2];
+    ct.f[2] = T02 * CT[0] + T22 * CT[2];
 
-    ct[0] = (-(T00 * CT[0] + T10 * CT[1] + T20 * CT[2])) * mask;
-    ct[1] = (-(T01 * CT[0] + T11 * CT[1] + T21 * CT[2])) * mask;
-    ct[2] = (-(T02 * CT[0] + T22 * CT[2])) * mask;
-
-    LP K2 = c.G * c.W4 * LIDiv6;
-    LP K3 = c.E * c.W4 * LIDiv6 * LP(2);
-    LP K4 = c.E * c.W4 * LIDiv6;
-    LP B3 = T00 * s[3] + T01 * s[4] + T02 * s[5];
-    LP B9 = T00 * o[3] + T01 * o[4] + T02 * o[5];
-
+    const double K2 = c.G * c.W4 * LIDiv6;
+    const double K3 = c.E * c.W4 * LIDiv6 * 2.0;
+    const double K4 = c.E * c.W4 * LIDiv6;
+    const double B3 = T00 * s.f[3] + T01 * s.f[4] + T02 * s.f[5];
+    const double B9 = T00 * o.f[3] + T01 * o.f[4] + T02 * o.f[5];
     CT[3] = CT[3] + (K2 * B3 + (-K2) * B9);
     CT[4] = CT[4] + ((-K5) * B2 + K3 * B4 + K5 * B8 + K4 * B10);
     CT[5] = CT[5] + (K5 * B1 + K3 * B5 + (-K5) * B7 + K4 * B11);
-
-    ct[3] = (-(T00 * CT[3] + T10 * CT[4] + T20 * CT[5])) * mask;
-    ct[4] = (-(T01 * CT[3] + T11 * CT[4] + T21 * CT[5])) * mask;
-    ct[5] = (-(T02 * CT[3] + T22 * CT[5])) * mask;
+    ct.f[3] = T00 * CT[3] + T10 * CT[4] + T20 * CT[5];
+    ct.f[4] = T01 * CT[3] + T11 * CT[4] + T21 * CT[5];
+    ct.f[5] = T02 * CT[3] + T22 * CT[5];
+    if (!whole) {
+#pragma unroll
+        for (int q = 0; q < 6; ++q) {
+            dp.f[q] = dp.f[q] * 0.0;
+            ct.f[q] = ct.f[q] * 0.0;
+        }
+    }
 }
 
 template <class LP>
-__device__ __forceinline__ void beam_side(const Consts<LP> &c, LP mask, LP xDist, LP yDist,
-                                          LP zDist, const LP *s, const LP *o, LP *CT, LP *F) {
-    LP dp[6], ct[6];
-    beam_terms<LP>(c, mask, xDist, yDist, zDist, s, o, CT, dp, ct);
-#pragma unroll
-    for (int k = 0; k < 6; ++k) F[k] = (F[k] + dp[k]) + ct[k];
+__device__ __forceinline__ void beam_side(const Consts<LP> &c, const Rounding<LP> &R, bool whole, LP xDist, LP yDist, LP zDist,
+                                          const Six<LP> &s, const Six<LP> &o, LP *CT, Six<LP> &F) {
+    Six<LP> dp, ct;
+    beam_terms(c, R, whole, xDist, yDist, zDist, s, o, CT, dp, ct);
+    F = (F + dp) - ct;
 }
 
 // Link break test: HiDEMDefLinkBreakFunc::operator() (HiDEMDefaultFunctions.h:207-242)
 // with end A as particle 1 and end B as particle 2 and the functor's two thresholds.
 // Returns the new state.
-template <class LP>
-__device__ __forceinline__ uint8_t break_link(const LP bendBreak, const LP maxLoad,
-                                              const PRec<LP> &a, const PRec<LP> &b,
+// (P: anything with x, y, z and th[3])
+template <class LP, class P>
+__device__ __forceinline__ uint8_t break_link(const LP bendBreak, const LP maxLoad, const P &a, const P &b,
                                               uint8_t state, LP initialLen) {
     if (state == 0) return 0;
     LP xDist = (LP)(a.x - b.x);

@@ -1,0 +1,81 @@
+"""The two-pass step's force pass: sizes at the edges of its blocks of 32 slots, CTAs of 128
+and the rule between its two variants, its folded link update against the break pass of the
+split calls, and the geometries its shared-root evaluation hands to the plain IEEE operations.
+Bit-exact against the oracle (or the split calls at sizes the oracle is slow at)."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+from hidem_b200 import abi, workloads
+from hidem_b200.hidemlib import HiDEMLib
+from oracle import oracle
+from test_gpu_parity import L_OUT, P_OUT, PRECS, assert_same, gpu_run
+
+pytestmark = pytest.mark.gpu
+
+
+# 4, 32, 36, 128, 132 and 1,500 particles: part of a block, whole blocks, part of a CTA
+@pytest.mark.parametrize("precision", PRECS)
+@pytest.mark.parametrize("cells", [(1, 1, 1), (2, 2, 2), (3, 3, 1), (2, 4, 4), (3, 11, 1), (15, 5, 5)])
+def test_two_pass_sizes(gpu, precision, cells):
+    P, p, l = workloads.ice_block(cells=cells, precision=precision, seed=8, gridRegenInterval=9)
+    ref = oracle.port().run(P, p, l, 24)
+    res = gpu_run(P, p, l, 24, kernel=abi.STEP_KERNEL_TWO_PASS)
+    assert_same(res, ref[0], ref[1], ref[3])
+    assert int((ref[1]["state"] == 0).sum()) > 0 or cells == (1, 1, 1)  # links break on the way
+
+
+# below and above the sizes where the variants change (75,776 particles mixed, 37,888 FP64)
+@pytest.mark.parametrize("precision,cells", [(abi.PREC_MIXED, (29, 29, 22)), (abi.PREC_MIXED, (29, 29, 23)),
+                                             (abi.PREC_FP64, (21, 21, 21)), (abi.PREC_FP64, (22, 21, 21))])
+def test_two_pass_against_split_calls(gpu, precision, cells):
+    P, p, l = workloads.ice_block(cells=cells, precision=precision, seed=9)
+    fused = gpu_run(P, p, l, 14, kernel=abi.STEP_KERNEL_TWO_PASS)
+    items = gpu_run(P, p, l, 14, kernel=abi.STEP_KERNEL_ITEMS)
+    assert_same(fused, items[0], items[1], items[3])
+    split = gpu_run(P, p, l, 14, mode="split")
+    assert_same(fused, split[0], split[1], split[3])
+    assert len(fused[3]) > 0
+
+
+def _pair(precision, sep, **over):
+    """Two bonded particles `sep` apart at a random attitude, spinning and drifting."""
+    lp = abi.lp_dtype(precision)
+    p = abi.empty_particles(2, precision)
+    for k, f in enumerate(("xCord", "yCord", "zCord")):
+        p[f][:] = [0.25, 0.25 + sep[k]]
+    rng = np.random.default_rng(3)
+    for f in P_OUT[3:]:
+        p[f][:] = rng.uniform(-1e-6, 1e-6, 2).astype(lp)
+    p["radius"][:] = 0.5
+    p["globalKeys"][:] = [0, 1]
+    l = abi.empty_links(1, precision)
+    l["globalKeyEndA"][0], l["globalKeyEndB"][0] = 0, 1
+    l["state"][0] = 1
+    l["initialLen"][0] = np.float32(np.sqrt(np.sum(np.square(sep))))
+    return workloads.block_params(precision, breakTime=1e9, **over), p, l
+
+
+# vertical (no xy part), nearly vertical (its square outside the shared-root range), near
+# coincidence, squared lengths whose root rounds to all ones, E W4 outside the admitted range
+@pytest.mark.parametrize("precision", PRECS)
+@pytest.mark.parametrize("sep,over", [((0.0, 0.0, 1.0), {}), ((1e-7, 0.0, 0.97), {}), ((1e-9, -1e-9, 0.9), {}),
+                                      ((3e-7, 2e-7, 1e-7), {}), ((0.9999999, 0.0, 0.0), {}),
+                                      ((0.0, 1.9999999, 0.0), {}), ((0.6, 0.5, 0.4), dict(E=1e-14)),
+                                      ((0.6, 0.5, 0.4), dict(E=1e21))])
+def test_geometries_outside_the_shared_root_range(gpu, precision, sep, over):
+    P, p, l = _pair(precision, sep, **over)
+    ref = oracle.port().run(P, p, l, 1)
+    for kernel in (abi.STEP_KERNEL_TWO_PASS, abi.STEP_KERNEL_ITEMS, abi.STEP_KERNEL_THREAD):
+        lib = HiDEMLib(P)
+        lib.set_step_kernel(kernel)
+        lib.set_particles(p)
+        lib.set_links(l)
+        lib.step(1)
+        out, links = lib.get_particles(), lib.get_links()
+        lib.close()
+        for k in P_OUT:
+            assert np.array_equal(out[k], ref[0][k], equal_nan=True), (k, kernel)
+        for k in L_OUT:
+            assert np.array_equal(links[k], ref[1][k], equal_nan=True), (k, kernel)
