@@ -62,6 +62,17 @@ inline bool on_device(const void *p) {
     }
     return a.type == cudaMemoryTypeDevice;
 }
+// whether a kernel on `device` may write a caller's array of `elem`-byte values: device memory
+// of that GPU, aligned for the values (a copy takes any address)
+inline bool writable_here(int device, const void *p, size_t elem) {
+    if (reinterpret_cast<uintptr_t>(p) % elem) return false;
+    cudaPointerAttributes a{};
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return a.type == cudaMemoryTypeDevice && a.device == device;
+}
 // bytes between a caller's array (host or device memory) and host memory
 inline cudaError_t from_caller(void *hostDst, const void *src, size_t bytes) {
     if (on_device(src)) return cudaMemcpy(hostDst, src, bytes, cudaMemcpyDeviceToHost);
@@ -429,12 +440,19 @@ hidem_status side_alloc(hidem_ctx *ctx, SideSet &s, long long cap) {
     return HIDEM_OK;
 }
 
-void side_free(SideSet &s) {
-    dfree(s.partner);
-    for (int k = 0; k < 6; ++k) dfree(s.ct[k]);
-    dfree(s.state);
-    dfree(s.L0);
-    dfree(s.link);
+// frees on a stream (buffers come from the stream-ordered pool: a plain cudaFree waits for the
+// whole device first)
+template <class T>
+void dfree_on(T *&p, cudaStream_t st) {
+    if (p) cudaFreeAsync((void *)p, st);
+    p = nullptr;
+}
+void side_free(SideSet &s, cudaStream_t st) {
+    dfree_on(s.partner, st);
+    for (int k = 0; k < 6; ++k) dfree_on(s.ct[k], st);
+    dfree_on(s.state, st);
+    dfree_on(s.L0, st);
+    dfree_on(s.link, st);
     s.cap = 0;
 }
 
@@ -1611,7 +1629,7 @@ void hidem_destroy(hidem_ctx *ctx) {
         dfree(ctx->orig[b]);
         dfree(ctx->cellOf[b]);
         dfree(ctx->sideSlot[b]);
-        side_free(ctx->side[b]);
+        side_free(ctx->side[b], ctx->stream);
     }
     dfree(ctx->slotOf);
     dfree(ctx->perm);
@@ -1805,8 +1823,8 @@ hidem_status hidem_set_links(hidem_ctx *ctx, const hidem_link_soa *l, int64_t L)
         unsigned long long h[2];
         CK(cudaMemcpyAsync(h, mins, sizeof h, cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
-        dfree(mins);
-        if (dkeys) dfree(dkeys);
+        dfree_on(mins, st);
+        dfree_on(dkeys, st);
         if (h[0] != ~0ull) bad = (long long)h[0];
         if (h[1] != ~0ull) self = (long long)h[1];
     } else {
@@ -1865,8 +1883,8 @@ hidem_status hidem_set_links(hidem_ctx *ctx, const hidem_link_soa *l, int64_t L)
     TRY(dalloc(ctx, &ctx->plLink, 2 * L));
     TRY(dalloc(ctx, &ctx->plEnd, 2 * L));
     for (int b = 0; b < 2; ++b) TRY(dalloc(ctx, &ctx->sideSlot[b], 2 * L));
-    side_free(ctx->side[0]);
-    side_free(ctx->side[1]);
+    side_free(ctx->side[0], st);
+    side_free(ctx->side[1], st);
     TRY(side_alloc(ctx, ctx->side[0], 2 * L));
     ctx->curSide = 0;
     TRY(dalloc(ctx, &ctx->events, std::max<long long>(L, 1)));
@@ -1910,10 +1928,10 @@ hidem_status hidem_set_links(hidem_ctx *ctx, const hidem_link_soa *l, int64_t L)
         if (l->globalKeys) CK(cudaMemcpyAsync(ctx->dLinkKeys, l->globalKeys, 8 * (size_t)L, cudaMemcpyDefault, st));
         else launch_iota64(ctx->dLinkKeys, L, st);
     }
+    dfree_on(deg, st);
+    dfree_on(cursor, st);
     CK(cudaStreamSynchronize(st));
     CK(cudaGetLastError());
-    dfree(deg);
-    dfree(cursor);
     ctx->L = L;
     ctx->haveLinks = true;
     ctx->built = false;
@@ -2175,43 +2193,119 @@ hidem_status hidem_profile_read(hidem_ctx *ctx, double *step_kernel_ms, int64_t 
     return HIDEM_OK;
 }
 
+extern "C++" {
+// The state in caller order: fields the caller wants in this device's memory are written
+// there by the kernel, the others into the idle record buffer and copied from it.
+template <class LP>
+static hidem_status get_particles_t(hidem_ctx *ctx, hidem_particle_soa *out) {
+    const long long n = ctx->n;
+    cudaStream_t st = ctx->stream;
+    char *stage = static_cast<char *>(ctx->rec[1 - ctx->cur]);
+    struct Copy {
+        void *dst;
+        const void *src;
+        size_t bytes;
+    };
+    std::vector<Copy> copies;
+    size_t used = 0;
+    auto place = [&](void *dst, size_t elem) -> void * {
+        if (!dst || writable_here(ctx->device, dst, elem)) return dst;
+        void *p = stage + used;
+        used += elem * (size_t)n;
+        copies.push_back({dst, p, elem * (size_t)n});
+        return p;
+    };
+    SoaOut<LP> s{};
+    double *xyz[3] = {out->xCord, out->yCord, out->zCord};
+    void *d[6] = {out->xDiff, out->yDiff, out->zDiff, out->uDiff, out->vDiff, out->wDiff};
+    void *th[3] = {out->xTheta, out->yTheta, out->zTheta};
+    for (int k = 0; k < 3; ++k) s.x[k] = static_cast<double *>(place(xyz[k], sizeof(double)));
+    for (int k = 0; k < 6; ++k) s.d[k] = static_cast<LP *>(place(d[k], sizeof(LP)));
+    s.r = static_cast<LP *>(place(out->radius, sizeof(LP)));
+    for (int k = 0; k < 3; ++k) s.th[k] = static_cast<LP *>(place(th[k], sizeof(LP)));
+    if (out->type && !writable_here(ctx->device, out->type, 1)) {
+        // the record buffer is full when every field is staged: the rebuild's permutation scratch
+        s.type = reinterpret_cast<uint8_t *>(ctx->perm);
+        copies.push_back({out->type, s.type, (size_t)n});
+    } else {
+        s.type = out->type;
+    }
+    launch_unpack_records<LP>(recp<LP>(ctx, ctx->cur), ctx->orig[ctx->ord], (int)n, s, ctx->type[ctx->ord], st);
+    ctx->launches += 1;
+    for (const Copy &c : copies) CK(cudaMemcpyAsync(c.dst, c.src, c.bytes, cudaMemcpyDefault, st));
+    return HIDEM_OK;
+}
+
+// Side data and link state in caller order, straight into the caller's device memory or, array
+// after array, through one staging buffer.
+template <class LP>
+static hidem_status get_sides_t(hidem_ctx *ctx, hidem_link_soa *out) {
+    const long long L = ctx->L;
+    cudaStream_t st = ctx->stream;
+    SideSet &s = ctx->side[ctx->curSide];
+    const int *slot = ctx->sideSlot[ctx->curSide];
+    SideGather<LP> direct{}, all{};
+    for (int k = 0; k < 6; ++k) all.ct[k] = static_cast<const LP *>(s.ct[k]);
+    all.state = s.state;
+    direct = all;
+    bool any = false, staged = false;
+    for (int k = 0; k < 6; ++k) {
+        if (!out->CT[k]) continue;
+        if (writable_here(ctx->device, out->CT[k], sizeof(LP))) {
+            direct.out[k] = static_cast<LP *>(out->CT[k]);
+            any = true;
+        } else {
+            staged = true;
+        }
+    }
+    if (out->state) {
+        if (writable_here(ctx->device, out->state, 1)) {
+            direct.stateOut = out->state;
+            any = true;
+        } else {
+            staged = true;
+        }
+    }
+    if (any) {
+        launch_gather_sides<LP>(slot, L, direct, st);
+        ctx->launches += 1;
+    }
+    if (!staged) return HIDEM_OK;
+    void *stage = nullptr;
+    TRY(dalloc_bytes(ctx, &stage, sizeof(LP) * (size_t)(2 * L)));
+    for (int k = 0; k < 7; ++k) {
+        SideGather<LP> g = all;
+        void *dst = nullptr;
+        size_t bytes = 0;
+        if (k < 6 && out->CT[k] && !direct.out[k]) {
+            g.out[k] = static_cast<LP *>(stage);
+            dst = out->CT[k];
+            bytes = sizeof(LP) * (size_t)(2 * L);
+        } else if (k == 6 && out->state && !direct.stateOut) {
+            g.stateOut = static_cast<uint8_t *>(stage);
+            dst = out->state;
+            bytes = (size_t)L;
+        } else {
+            continue;
+        }
+        launch_gather_sides<LP>(slot, L, g, st);
+        ctx->launches += 1;
+        CK(cudaMemcpyAsync(dst, stage, bytes, cudaMemcpyDefault, st));
+    }
+    CK(cudaFreeAsync(stage, st));
+    return HIDEM_OK;
+}
+}  // extern "C++"
+
 hidem_status hidem_get_particles(hidem_ctx *ctx, hidem_particle_soa *out) {
     if (!ctx || !out) return HIDEM_ERR_ARG;
     if (!ctx->haveParticles) return fail(ctx, HIDEM_ERR_STATE, "no particles set");
     CK(cudaSetDevice(ctx->device));
-    const long long n = ctx->n;
-    cudaStream_t st = ctx->stream;
-    // unpack the slot-ordered records into caller order in the idle record buffer
-    void *stage = ctx->rec[1 - ctx->cur];
-    const size_t lp = ctx->lp;
-    if (ctx->mixed) {
-        SoaIn<float> s = soa_layout<float>(stage, n);
-        launch_unpack_records<float>(recp<float>(ctx, ctx->cur), ctx->orig[ctx->ord], (int)n, s, st);
-    } else {
-        SoaIn<double> s = soa_layout<double>(stage, n);
-        launch_unpack_records<double>(recp<double>(ctx, ctx->cur), ctx->orig[ctx->ord], (int)n, s, st);
-    }
-    ctx->launches += 1;
-    const char *b = static_cast<const char *>(stage);
-    double *xyz[3] = {out->xCord, out->yCord, out->zCord};
-    for (int k = 0; k < 3; ++k)
-        if (xyz[k]) CK(cudaMemcpyAsync(xyz[k], b + 8 * (size_t)n * k, 8 * (size_t)n, cudaMemcpyDefault, st));
-    const char *lpb = b + 24 * (size_t)n;
-    void *lpf[10] = {out->xDiff, out->yDiff, out->zDiff, out->uDiff, out->vDiff, out->wDiff,
-                     out->radius, out->xTheta, out->yTheta, out->zTheta};
-    for (int k = 0; k < 10; ++k)
-        if (lpf[k]) CK(cudaMemcpyAsync(lpf[k], lpb + lp * (size_t)n * k, lp * (size_t)n, cudaMemcpyDefault, st));
-    if (out->type) {
-        // the type bytes in caller order, staged in the rebuild's permutation scratch
-        uint8_t *tstage = reinterpret_cast<uint8_t *>(ctx->perm);
-        launch_scatter_u8(ctx->type[ctx->ord], ctx->orig[ctx->ord], (int)n, tstage, st);
-        ctx->launches += 1;
-        CK(cudaMemcpyAsync(out->type, tstage, (size_t)n, cudaMemcpyDefault, st));
-    }
+    TRY(ctx->mixed ? get_particles_t<float>(ctx, out) : get_particles_t<double>(ctx, out));
     // the host-held fields while the copies run
-    if (out->owners) CK(to_caller(out->owners, ctx->owners.data(), 4 * (size_t)n));
-    if (out->globalKeys) CK(to_caller(out->globalKeys, ctx->keys.data(), 8 * (size_t)n));
-    CK(cudaStreamSynchronize(st));
+    if (out->owners) CK(to_caller(out->owners, ctx->owners.data(), 4 * (size_t)ctx->n));
+    if (out->globalKeys) CK(to_caller(out->globalKeys, ctx->keys.data(), 8 * (size_t)ctx->n));
+    CK(cudaStreamSynchronize(ctx->stream));
     return HIDEM_OK;
 }
 
@@ -2222,31 +2316,8 @@ hidem_status hidem_get_links(hidem_ctx *ctx, hidem_link_soa *out) {
     const long long L = ctx->L;
     if (L == 0) return HIDEM_OK;
     cudaStream_t st = ctx->stream;
-    SideSet &s = ctx->side[ctx->curSide];
+    TRY(ctx->mixed ? get_sides_t<float>(ctx, out) : get_sides_t<double>(ctx, out));
     const size_t lp = ctx->lp;
-    void *stage = nullptr;
-    uint8_t *lstate = nullptr;
-    TRY(dalloc_bytes(ctx, &stage, lp * (size_t)(2 * L)));
-    TRY(dalloc(ctx, &lstate, L));
-    const int *slot = ctx->sideSlot[ctx->curSide];
-    // side data and link state back in caller order
-    for (int k = 0; k < 6; ++k) {
-        if (!out->CT[k]) continue;
-        if (ctx->mixed)
-            launch_gather_sides<float>(slot, L, static_cast<const float *>(s.ct[k]), static_cast<float *>(stage), nullptr, nullptr, st);
-        else
-            launch_gather_sides<double>(slot, L, static_cast<const double *>(s.ct[k]), static_cast<double *>(stage), nullptr, nullptr, st);
-        CK(cudaMemcpyAsync(out->CT[k], stage, lp * (size_t)(2 * L), cudaMemcpyDefault, st));
-        ctx->launches += 1;
-    }
-    if (out->state) {
-        if (ctx->mixed)
-            launch_gather_sides<float>(slot, L, nullptr, nullptr, s.state, lstate, st);
-        else
-            launch_gather_sides<double>(slot, L, nullptr, nullptr, s.state, lstate, st);
-        CK(cudaMemcpyAsync(out->state, lstate, (size_t)L, cudaMemcpyDefault, st));
-        ctx->launches += 1;
-    }
     if (out->initialLen) CK(cudaMemcpyAsync(out->initialLen, ctx->L0link, lp * (size_t)L, cudaMemcpyDefault, st));
     if (out->owners) CK(cudaMemcpyAsync(out->owners, ctx->dLinkOwners, 4 * (size_t)L, cudaMemcpyDefault, st));
     if (out->globalKeys) CK(cudaMemcpyAsync(out->globalKeys, ctx->dLinkKeys, 8 * (size_t)L, cudaMemcpyDefault, st));
@@ -2254,8 +2325,6 @@ hidem_status hidem_get_links(hidem_ctx *ctx, hidem_link_soa *out) {
     if (out->globalKeyEndB) CK(cudaMemcpyAsync(out->globalKeyEndB, ctx->dLinkKeyB, 8 * (size_t)L, cudaMemcpyDefault, st));
     if (out->particleLinkNum) CK(cudaMemcpyAsync(out->particleLinkNum, ctx->dLinkNum, 4 * (size_t)L, cudaMemcpyDefault, st));
     CK(cudaStreamSynchronize(st));
-    dfree(stage);
-    dfree(lstate);
     return HIDEM_OK;
 }
 

@@ -1665,16 +1665,6 @@ void launch_send_pos(const int *slotOf, const int *index, long long m, int n, in
     if (m > 0) k_send_pos<<<nblk(m, 256), 256, 0, s>>>(slotOf, index, m, pos);
 }
 
-__global__ void k_scatter_u8(const uint8_t *__restrict__ in, const int *__restrict__ to, int n,
-                             uint8_t *__restrict__ out) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) out[to[i]] = in[i];
-}
-
-void launch_scatter_u8(const uint8_t *in, const int *to, int n, uint8_t *out, cudaStream_t s) {
-    if (n > 0) k_scatter_u8<<<nblk(n, 256), 256, 0, s>>>(in, to, n, out);
-}
-
 void launch_scatter(const int *cellOf, int n, const int *cellStart, int *cursor, int *perm,
                     cudaStream_t s) {
     k_scatter<<<nblk(n, 256), 256, 0, s>>>(cellOf, n, cellStart, cursor, perm);
@@ -2078,21 +2068,25 @@ __global__ void k_pack_records(SoaIn<LP> s, int n, PRec<LP> *__restrict__ rec) {
     store_rec(rec + i, r);
 }
 
+// Slot-ordered records into caller-order arrays (null: not wanted).
 template <class LP>
 __global__ void k_unpack_records(const PRec<LP> *__restrict__ rec, const int *__restrict__ orig,
-                                 int n, SoaIn<LP> s) {
+                                 int n, SoaOut<LP> s, const uint8_t *__restrict__ typeIn) {
     int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
     const PRec<LP> r = load_rec(rec + k);
     const int i = orig[k];
-    const_cast<double *>(s.x)[i] = r.x;
-    const_cast<double *>(s.y)[i] = r.y;
-    const_cast<double *>(s.z)[i] = r.z;
+    if (s.x[0]) s.x[0][i] = r.x;
+    if (s.x[1]) s.x[1][i] = r.y;
+    if (s.x[2]) s.x[2][i] = r.z;
 #pragma unroll
-    for (int q = 0; q < 6; ++q) const_cast<LP *>(s.d[q])[i] = r.d[q];
-    const_cast<LP *>(s.r)[i] = r.r;
+    for (int q = 0; q < 6; ++q)
+        if (s.d[q]) s.d[q][i] = r.d[q];
+    if (s.r) s.r[i] = r.r;
 #pragma unroll
-    for (int q = 0; q < 3; ++q) const_cast<LP *>(s.th[q])[i] = r.th[q];
+    for (int q = 0; q < 3; ++q)
+        if (s.th[q]) s.th[q][i] = r.th[q];
+    if (s.type) s.type[i] = typeIn[k];
 }
 
 template <class LP>
@@ -2179,16 +2173,22 @@ __global__ void k_side_init(const uint8_t *__restrict__ linkState, long long L,
     sideState[s] = linkState[s >> 1];
 }
 
-// side data back in the caller's order: CT[k][2l+e] and the link state
+// Side data back in the caller's order: CT[k][2l+e] and the link state (null: not wanted). One
+// thread per link: both ends' slots in one load, every wanted array gathered through them, so
+// that the slots (272 MB on the 5.7M slab) are read once and not once per array.
 template <class LP>
-__global__ void k_gather_sides(const int *__restrict__ sideSlot, long long L,
-                               const LP *__restrict__ ct, LP *__restrict__ out,
-                               const uint8_t *__restrict__ sState, uint8_t *__restrict__ linkState) {
-    long long s = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= 2 * L) return;
-    const int src = sideSlot[s];
-    if (ct) out[s] = ct[src];
-    if (linkState && (s & 1) == 0) linkState[s >> 1] = sState[src];
+__global__ void __launch_bounds__(256) k_gather_sides(const int2 *__restrict__ sideSlot, long long L,
+                                                      SideGather<LP> g) {
+    const long long l = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (l >= L) return;
+    const int2 src = sideSlot[l];
+#pragma unroll
+    for (int q = 0; q < 6; ++q)
+        if (g.out[q]) {
+            g.out[q][2 * l] = g.ct[q][src.x];
+            g.out[q][2 * l + 1] = g.ct[q][src.y];
+        }
+    if (g.stateOut) g.stateOut[l] = g.state[src.x];
 }
 
 __global__ void k_link_keys_identity(const long long *__restrict__ ka, const long long *__restrict__ kb,
@@ -2320,9 +2320,9 @@ void launch_pack_records(const SoaIn<LP> &s, int n, PRec<LP> *rec, cudaStream_t 
     k_pack_records<LP><<<nblk(n, 256), 256, 0, st>>>(s, n, rec);
 }
 template <class LP>
-void launch_unpack_records(const PRec<LP> *rec, const int *orig, int n, const SoaIn<LP> &s,
-                           cudaStream_t st) {
-    k_unpack_records<LP><<<nblk(n, 256), 256, 0, st>>>(rec, orig, n, s);
+void launch_unpack_records(const PRec<LP> *rec, const int *orig, int n, const SoaOut<LP> &s,
+                           const uint8_t *type, cudaStream_t st) {
+    k_unpack_records<LP><<<nblk(n, 256), 256, 0, st>>>(rec, orig, n, s, type);
 }
 template <class LP>
 void launch_unpack_force(const LP *force, const int *orig, int n, LP *out, cudaStream_t st) {
@@ -2350,20 +2350,18 @@ void launch_side_init(const uint8_t *linkState, long long L, int *sideSlot, uint
     if (L > 0) k_side_init<<<nblk(2 * L, 256), 256, 0, st>>>(linkState, L, sideSlot, sideState);
 }
 template <class LP>
-void launch_gather_sides(const int *sideSlot, long long L, const LP *ct, LP *out,
-                         const uint8_t *sState, uint8_t *linkState, cudaStream_t st) {
-    if (L > 0) k_gather_sides<LP><<<nblk(2 * L, 256), 256, 0, st>>>(sideSlot, L, ct, out, sState, linkState);
+void launch_gather_sides(const int *sideSlot, long long L, const SideGather<LP> &g, cudaStream_t st) {
+    if (L > 0) k_gather_sides<LP><<<nblk(L, 256), 256, 0, st>>>(reinterpret_cast<const int2 *>(sideSlot), L, g);
 }
 
 #define HIDEM_INSTANTIATE_IO(LP)                                                                   \
     template void launch_pack_records<LP>(const SoaIn<LP> &, int, PRec<LP> *, cudaStream_t);       \
-    template void launch_unpack_records<LP>(const PRec<LP> *, const int *, int, const SoaIn<LP> &,  \
-                                            cudaStream_t);                                         \
+    template void launch_unpack_records<LP>(const PRec<LP> *, const int *, int, const SoaOut<LP> &, \
+                                            const uint8_t *, cudaStream_t);                        \
     template void launch_unpack_force<LP>(const LP *, const int *, int, LP *, cudaStream_t);       \
     template void launch_halo_forces<LP>(LP *, const int *, const int *, long long, int, LP *, bool, \
                                          cudaStream_t);                                            \
-    template void launch_gather_sides<LP>(const int *, long long, const LP *, LP *,                \
-                                          const uint8_t *, uint8_t *, cudaStream_t);
+    template void launch_gather_sides<LP>(const int *, long long, const SideGather<LP> &, cudaStream_t);
 HIDEM_INSTANTIATE_IO(float)
 HIDEM_INSTANTIATE_IO(double)
 

@@ -49,11 +49,29 @@ struct SoaIn {
     const LP *th[3];
 };
 
+// and the ones read back (null: not wanted)
+template <class LP>
+struct SoaOut {
+    double *x[3];
+    LP *d[6];
+    LP *r;
+    LP *th[3];
+    uint8_t *type;
+};
+// link-end data read back: CT0..CT5 and the link state of the sides (null out: not wanted)
+template <class LP>
+struct SideGather {
+    const LP *ct[6];
+    const uint8_t *state;
+    LP *out[6];
+    uint8_t *stateOut;
+};
+
 template <class LP>
 void launch_pack_records(const SoaIn<LP> &s, int n, PRec<LP> *rec, cudaStream_t st);
 template <class LP>
-void launch_unpack_records(const PRec<LP> *rec, const int *orig, int n, const SoaIn<LP> &s,
-                           cudaStream_t st);
+void launch_unpack_records(const PRec<LP> *rec, const int *orig, int n, const SoaOut<LP> &s,
+                           const uint8_t *type, cudaStream_t st);
 template <class LP>
 void launch_unpack_force(const LP *force, const int *orig, int n, LP *out, cudaStream_t st);
 // pack: buf[6k + q] = force of particle index[k] (input order), component q;
@@ -85,8 +103,7 @@ void launch_iota32(int *out, int count, cudaStream_t st);
 template <class LP>
 void launch_max_radius(const PRec<LP> *rec, int n, unsigned long long *out, cudaStream_t st);
 template <class LP>
-void launch_gather_sides(const int *sideSlot, long long L, const LP *ct, LP *out,
-                         const uint8_t *sState, uint8_t *linkState, cudaStream_t st);
+void launch_gather_sides(const int *sideSlot, long long L, const SideGather<LP> &g, cudaStream_t st);
 
 template <class LP>
 void launch_bounds(const PRec<LP> *rec, int n, double *partial, int nb, double *out, cudaStream_t s);
@@ -101,8 +118,6 @@ void launch_scatter(const int *cellOf, int n, const int *cellStart, int *cursor,
                     cudaStream_t s);
 // pos[s] = position of slot s in the halo send list `index` (particle indices), else -1
 void launch_send_pos(const int *slotOf, const int *index, long long m, int n, int *pos, cudaStream_t s);
-// out[to[i]] = in[i] for i < n (slot-order bytes into caller order)
-void launch_scatter_u8(const uint8_t *in, const int *to, int n, uint8_t *out, cudaStream_t s);
 // Members of a neighbour-grid cell of at most kSmallCell are sorted by one thread; larger
 // cells (listed in bigList, which holds n / kSmallCell + 1 entries) by one CTA each, up to
 // kBigCellCap members: a larger cell sets errorCode in errorFlag. origOld == nullptr sorts
