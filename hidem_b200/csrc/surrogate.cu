@@ -381,6 +381,8 @@ struct MlpMaps {
 
 struct MlpArgs {
     int layers, k0;                 // hidden layers, first layer's K
+    int perGroup;                   // k_mlp_pp: blocks a CTA has in flight
+    long long liveRows;             // k_mlp_pp: rows of y that exist (the last block's may not all)
     const float *bias[kMlpMaxLayers];
     const float *wo, *bo;           // output layer [3][W], [3]
     float *y;                       // [rows][3]
@@ -682,6 +684,9 @@ __device__ __forceinline__ void pp_epilogue(uint32_t taddr, int c0s, int row, lo
 // output layer runs in the last layer's epilogue: each warp sums its 64 columns in k order
 // per row, and the four partial sums of a row are added in column order. The hidden layers'
 // arithmetic is that of k_mlp_fwd (same MMAs in the same order, same epilogue).
+// Where there are no more blocks than SMs a CTA takes one block alone (g.perGroup == 1): a
+// second one would only wait beside an idle SM (a training batch of 8,192 rows is 64 blocks:
+// 113 us on 32 SMs in ping-pong, 66 us on 64). The arithmetic of a block is the same either way.
 template <int BN>
 __global__ void __launch_bounds__(kPPThreads, 1)
     k_mlp_pp(const __grid_constant__ MlpMaps maps, const MlpArgs g, int rows) {
@@ -711,7 +716,8 @@ __global__ void __launch_bounds__(kPPThreads, 1)
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int L = g.layers;
     const int nk0 = g.k0 / 64, nkw = BN / 64;
-    const int nPairs = (rows / 128 + 1) / 2;
+    const int per = g.perGroup;  // blocks a CTA has in flight: 2 in ping-pong, or 1
+    const int nGroups = (rows / 128 + per - 1) / per;
 
     if (tid == 0) {
         for (int s = 0; s < S; ++s) {
@@ -741,10 +747,10 @@ __global__ void __launch_bounds__(kPPThreads, 1)
         // ---- copies: k counts the loads, n[b] the units of block b
         uint32_t k = 0, n[2] = {0, 0};
         bool ok = true;
-        for (int p = blockIdx.x; ok && p < nPairs; p += gridDim.x) {
+        for (int p = blockIdx.x; ok && p < nGroups; p += gridDim.x) {
             for (int l = 0; ok && l < L; ++l) {
-                for (int b = 0; ok && b < 2; ++b) {
-                    const int m0 = (2 * p + b) * 128;
+                for (int b = 0; ok && b < per; ++b) {
+                    const int m0 = (per * p + b) * 128;
                     unsigned char *ab = act + b * ACT;
                     // the feature tiles overwrite the block's activation tile: wait for the
                     // epilogue of the block's previous unit to release it
@@ -788,9 +794,9 @@ __global__ void __launch_bounds__(kPPThreads, 1)
                                ((uint32_t)(128 >> 4) << 24);
         uint32_t k = 0, n[2] = {0, 0};
         bool ok = true;
-        for (int p = blockIdx.x; ok && p < nPairs; p += gridDim.x) {
+        for (int p = blockIdx.x; ok && p < nGroups; p += gridDim.x) {
             for (int l = 0; ok && l < L; ++l) {
-                for (int b = 0; ok && b < 2; ++b) {
+                for (int b = 0; ok && b < per; ++b) {
                     if (n[b] > 0 && !mb_wait_or_fail(accFree + b, (n[b] - 1) & 1, fail)) {
                         ok = false;
                         break;
@@ -835,16 +841,16 @@ __global__ void __launch_bounds__(kPPThreads, 1)
         const uint32_t tl = (uint32_t)(q * 32) << 16;
         uint32_t n[2] = {0, 0}, no[2] = {0, 0};
         bool ok = true;
-        for (int p = blockIdx.x; ok && p < nPairs; p += gridDim.x) {
+        for (int p = blockIdx.x; ok && p < nGroups; p += gridDim.x) {
             for (int l = 0; ok && l < L; ++l) {
-                for (int b = 0; ok && b < 2; ++b) {
+                for (int b = 0; ok && b < per; ++b) {
                     if (!mb_wait_or_fail(accFull + b, n[b] & 1, fail)) {
                         ok = false;
                         break;
                     }
                     tc_fence_after();
-                    const long long grow = (long long)(2 * p + b) * 128 + row;
-                    const bool live = grow < rows;
+                    const long long grow = (long long)(per * p + b) * 128 + row;
+                    const bool live = grow < g.liveRows;
                     const bool last = l == L - 1;
                     unsigned char *ab = act + b * ACT;
                     const float *bias = g.bias[l];
@@ -930,19 +936,43 @@ int feature_width(int nin, int bands) {
 // one hardware sine / cosine pair per band (the features are rounded to BF16, far coarser
 // than the approximation); for a fixed band the lanes' (sin, cos) pairs are consecutive
 // 4-byte words of the row. Then the padding.
-__global__ void k_features(const float *__restrict__ in, const int *__restrict__ idx, int rows,
-                           int nin, int bands, int K0, bf16 *__restrict__ X) {
+// A training batch draws its rows uniformly (with replacement) from n samples, by a splitmix64
+// hash of (seed, step, row), and leaves them in idx (null: rows as they come). Rows from `live`
+// on are zero rows (a ragged last block).
+__device__ __forceinline__ int sample_row(unsigned long long seed, unsigned long long step, int b, long long n) {
+    unsigned long long z = seed + 0x9E3779B97F4A7C15ull * (step * 0x100000001B3ull + (unsigned long long)b + 1);
+    z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
+    z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
+    z = z ^ (z >> 31);
+    return (int)(z % (unsigned long long)n);
+}
+__global__ void k_features(const float *__restrict__ in, int *__restrict__ idx, unsigned long long seed,
+                           unsigned long long step, long long n, int rows, int live, int nin, int bands, int K0,
+                           bf16 *__restrict__ X) {
     const int b = blockIdx.x * blockDim.y + threadIdx.y;
     if (b >= rows) return;
-    const int src = idx ? idx[b] : b;
+    const int src = idx ? sample_row(seed, step, b, n) : b;
+    if (idx && threadIdx.x == 0) idx[b] = src;
     bf16 *x = X + (long long)b * K0;
     const bool pairs = (nin & 1) == 0;  // (sin, cos) pairs start on 4-byte boundaries
-    for (int i = threadIdx.x; i < nin; i += blockDim.x) {
-        const float v = in[(long long)src * nin + i];
-        x[i] = __float2bfloat16_rn(v);
-        for (int f = 0; f < bands; ++f) {
+    // all of the lane's inputs first, so that their loads overlap
+    float v[kMaxIn / 32];
+#pragma unroll
+    for (int t = 0; t < kMaxIn / 32; ++t) {
+        const int i = threadIdx.x + 32 * t;
+        v[t] = i < nin && b < live ? __ldg(in + (long long)src * nin + i) : 0.f;
+    }
+#pragma unroll
+    for (int t = 0; t < kMaxIn / 32; ++t)
+        if (threadIdx.x + 32 * t < nin) x[threadIdx.x + 32 * t] = __float2bfloat16_rn(v[t]);
+    for (int f = 0; f < bands; ++f) {
+        const float w = (float)(1 << f) * 3.14159265358979f;
+#pragma unroll
+        for (int t = 0; t < kMaxIn / 32; ++t) {
+            const int i = threadIdx.x + 32 * t;
+            if (i >= nin) continue;
             float sv, cv;
-            __sincosf((float)(1 << f) * 3.14159265358979f * v, &sv, &cv);
+            __sincosf(w * v[t], &sv, &cv);
             const int c = nin + 2 * (nin * f + i);
             if (pairs) {
                 *reinterpret_cast<__nv_bfloat162 *>(x + c) = __floats2bfloat162_rn(sv, cv);
@@ -1022,6 +1052,29 @@ __global__ void __launch_bounds__(256) k_sum_splits(const float *__restrict__ pa
         out[e] = t;
     }
 }
+// The same over the output layer's chunk partials [chunk][3][W + 1]: column W of each of the
+// three rows is that output's bias.
+__global__ void __launch_bounds__(256) k_sum_out(const float *__restrict__ part, int chunks, int W,
+                                                 float *__restrict__ gw, float *__restrict__ gb) {
+    __shared__ float red[8][33];
+    const int count = kOut * (W + 1);
+    const int e = blockIdx.x * 32 + threadIdx.x;
+    float acc = 0.f;
+    if (e < count) {
+#pragma unroll 4
+        for (int s = threadIdx.y; s < chunks; s += 8) acc += part[(long long)s * count + e];
+    }
+    red[threadIdx.y][threadIdx.x] = acc;
+    __syncthreads();
+    if (threadIdx.y == 0 && e < count) {
+        float t = 0.f;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) t += red[j][threadIdx.x];
+        const int j = e / (W + 1), k = e % (W + 1);
+        if (k < W) gw[j * W + k] = t;
+        else gb[j] = t;
+    }
+}
 inline dim3 sum_splits_grid(long long count) { return dim3((unsigned)((count + 31) / 32)); }
 
 // Column sums of a BF16 [rows][N] matrix (N even) over row chunks of kChunk: part[chunk][N].
@@ -1082,16 +1135,22 @@ __global__ void k_loss(const float *__restrict__ Y, const float *__restrict__ ta
 }
 
 // Output layer backward into the last hidden layer:
-// dZ[b][k] = (sum_j dY[b][j] Wo[j][k]) * SiLU'(Z[b][k]), stored BF16
-__global__ void k_out_bwd(const float *__restrict__ dY, const float *__restrict__ Wo,
+// dZ[b][k] = (sum_j dY[b][j] Wo[j][k]) * SiLU'(Z[b][k]), stored BF16 (dY formed as k_loss does)
+__global__ void k_out_bwd(const float *__restrict__ Y, const float *__restrict__ targets,
+                          const int *__restrict__ idx, const float *__restrict__ Wo,
                           const float *__restrict__ Z, int rows, int W, bf16 *__restrict__ dZ) {
     // one CTA row per batch row (blockIdx.x), its columns over blockIdx.y
     const int b = blockIdx.x, k = blockIdx.y * blockDim.x + threadIdx.x;
     if (b >= rows || k >= W) return;
     const long long e = (long long)b * W + k;
+    const int src = idx ? idx[b] : b;
+    const float inv = 2.0f / (float)(rows * kOut);
     float g = 0.f;
 #pragma unroll
-    for (int j = 0; j < kOut; ++j) g += dY[(long long)b * kOut + j] * Wo[j * W + k];
+    for (int j = 0; j < kOut; ++j) {
+        const float d = Y[(long long)b * kOut + j] - targets[(long long)src * kOut + j];
+        g += (d * inv) * Wo[j * W + k];
+    }
     dZ[e] = __float2bfloat16_rn(g * silu_grad(Z[e]));
 }
 
@@ -1125,10 +1184,36 @@ __global__ void __launch_bounds__(256) k_out_grad(const float *__restrict__ dY, 
     }
 }
 
-// Adam on a flat FP32 parameter array (t = step count after this update)
+// Where each hidden layer's weights lie in the flat parameters, and their BF16 copies: as is
+// ([W][K_l]) and transposed.
+struct WeightViews {
+    int layers, W;
+    int K[kMlpMaxLayers];
+    long long off[kMlpMaxLayers];
+    bf16 *wb[kMlpMaxLayers], *wbT[kMlpMaxLayers];
+};
+__device__ __forceinline__ void store_bf16_copies(const WeightViews &v, long long e, float w) {
+    for (int l = 0; l < v.layers; ++l) {
+        const long long q = e - v.off[l];
+        if (q >= 0 && q < (long long)v.W * v.K[l]) {
+            const int r = (int)(q / v.K[l]), c = (int)(q % v.K[l]);
+            const bf16 h = __float2bfloat16_rn(w);
+            v.wb[l][q] = h;
+            v.wbT[l][(long long)c * v.W + r] = h;
+        }
+    }
+}
+__global__ void k_weight_bf16(const float *__restrict__ p, const WeightViews v) {
+    const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const int l = v.layers - 1;
+    if (e < v.off[l] + (long long)v.W * v.K[l]) store_bf16_copies(v, e, p[e]);
+}
+
+// Adam on the flat FP32 parameter array (t = step count after this update), with the BF16
+// copies of the weights it changes
 __global__ void k_adam(float *__restrict__ p, const float *__restrict__ g, float *__restrict__ m,
                        float *__restrict__ v, long long n, float lr, float b1, float b2, float eps,
-                       float c1, float c2) {
+                       float c1, float c2, const WeightViews views) {
     const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= n) return;
     const float gr = g[e];
@@ -1136,31 +1221,9 @@ __global__ void k_adam(float *__restrict__ p, const float *__restrict__ g, float
     const float vv = b2 * v[e] + (1.f - b2) * gr * gr;
     m[e] = mm;
     v[e] = vv;
-    p[e] -= lr * (mm / c1) / (sqrtf(vv / c2) + eps);
-}
-
-// BF16 copies of a [R][C] FP32 weight: as is and transposed
-__global__ void k_weight_bf16(const float *__restrict__ w, int R, int C, bf16 *__restrict__ wb,
-                              bf16 *__restrict__ wbT) {
-    const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= (long long)R * C) return;
-    const int r = (int)(e / C), c = (int)(e % C);
-    const bf16 h = __float2bfloat16_rn(w[e]);
-    wb[e] = h;
-    wbT[(long long)c * R + r] = h;
-}
-
-// Batch rows drawn uniformly (with replacement) from n samples: a splitmix64 hash of
-// (seed, step, row)
-__global__ void k_sample(unsigned long long seed, unsigned long long step, int rows, long long n,
-                         int *__restrict__ idx) {
-    const int b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= rows) return;
-    unsigned long long z = seed + 0x9E3779B97F4A7C15ull * (step * 0x100000001B3ull + (unsigned long long)b + 1);
-    z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
-    z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
-    z = z ^ (z >> 31);
-    idx[b] = (int)(z % (unsigned long long)n);
+    const float w = p[e] - lr * (mm / c1) / (sqrtf(vv / c2) + eps);
+    p[e] = w;
+    store_bf16_copies(views, e, w);
 }
 
 }  // namespace
@@ -1185,16 +1248,23 @@ struct hidem_surrogate {
     std::vector<float *> Z;                      // [B][W] pre-activations
     std::vector<bf16 *> H;                       // [B][W] activations
     float *Y = nullptr, *dY = nullptr;           // [B][3]
-    bf16 *dZa = nullptr, *dZb = nullptr;         // [B][W]
-    bf16 *dZT = nullptr, *inT = nullptr;         // [W][B], [max K][B]
-    float *part = nullptr;                       // split / chunk partials
-    long long partCap = 0;
-    float *lossPart = nullptr, *lossHost = nullptr;
+    // per hidden layer: dZ [B][W], dZ^T [W][B], the layer's input transposed [K_l][B], the split
+    // partials of its weight gradient and the chunk partials of its bias gradient
+    std::vector<bf16 *> dZ, dZT, inT;
+    std::vector<float *> part, partB;
+    float *partOut = nullptr;                    // chunk partials of the output layer's gradient
+    std::vector<cudaStream_t> side;              // per hidden layer, then the output layer's
+    std::vector<cudaEvent_t> evDz, evDone;
+    cudaEvent_t evForward = nullptr;
+    WeightViews weights{};
+    char *arena = nullptr;                       // every device buffer but the training set
+    float *lossPart = nullptr, *lossHost = nullptr;  // block losses; pinned, with the error flag behind
+    int *errHost = nullptr;
     int *idx = nullptr;
     float *dataIn = nullptr, *dataT = nullptr;   // training set [n][nin], [n][3]
     long long nData = 0;
     float *scratchIn = nullptr, *scratchT = nullptr;  // caller rows for predict / gradients
-    int PB = 0;                                   // rows per predict chunk
+    int PB = 0;                                   // rows the predict buffers hold
     float *predIn = nullptr, *predY = nullptr;    // predict chunk: inputs [PB][nin], outputs [PB][3]
     bf16 *predX = nullptr;                        // predict chunk features [PB][K0]
     long long steps = 0;
@@ -1271,7 +1341,7 @@ hidem_status sfail(hidem_surrogate *s, hidem_status st, const char *fmt, ...) {
     } while (0)
 
 template <int BN, int EPI>
-hidem_status gemm(hidem_surrogate *s, const bf16 *A, int M, int K, const bf16 *Bm, int splits,
+hidem_status gemm(hidem_surrogate *s, cudaStream_t st, const bf16 *A, int M, int K, const bf16 *Bm, int splits,
                   GemmArgs g) {
     // per-device attribute, set once on each device (a repeated set is harmless)
     static std::atomic<unsigned long long> configured{0};
@@ -1299,31 +1369,22 @@ hidem_status gemm(hidem_surrogate *s, const bf16 *A, int M, int K, const bf16 *B
     g.K = K;
     g.kTiles = K / 64 / splits;
     g.err = s->dErr;
-    k_umma_gemm<BN, EPI><<<dim3(M / 128, splits), kGemmThreads, gemm_smem_bytes<BN>(), s->stream>>>(ta, tb, tz, g);
+    k_umma_gemm<BN, EPI><<<dim3(M / 128, splits), kGemmThreads, gemm_smem_bytes<BN>(), st>>>(ta, tb, tz, g);
     SCK(cudaGetLastError());
     return HIDEM_OK;
 }
 
 template <int EPI>
-hidem_status gemm_n(hidem_surrogate *s, int N, const bf16 *A, int M, int K, const bf16 *Bm,
+hidem_status gemm_n(hidem_surrogate *s, cudaStream_t st, int N, const bf16 *A, int M, int K, const bf16 *Bm,
                     int splits, const GemmArgs &g) {
-    if (N == 256) return gemm<256, EPI>(s, A, M, K, Bm, splits, g);
-    if (N == 128) return gemm<128, EPI>(s, A, M, K, Bm, splits, g);
+    if (N == 256) return gemm<256, EPI>(s, st, A, M, K, Bm, splits, g);
+    if (N == 128) return gemm<128, EPI>(s, st, A, M, K, Bm, splits, g);
     return sfail(s, HIDEM_ERR_ARG, "GEMM width %d (128 or 256)", N);
 }
 
-// the partial buffer is sized at creation for the largest batch; a call that would need
-// more is a bug, reported rather than reallocating under queued work
-hidem_status ensure_part(hidem_surrogate *s, long long count) {
-    if (s->partCap >= count) return HIDEM_OK;
-    return sfail(s, HIDEM_ERR_CAPACITY, "partial buffer too small (%lld < %lld)", s->partCap, count);
-}
-
+// the BF16 copies of every hidden layer's weights, in one launch
 hidem_status refresh_bf16(hidem_surrogate *s) {
-    for (int l = 0; l < s->L; ++l) {
-        const long long n = (long long)s->W * s->Kl[l];
-        k_weight_bf16<<<(unsigned)((n + 255) / 256), 256, 0, s->stream>>>(s->P + s->offW[l], s->W, s->Kl[l], s->Wb[l], s->WbT[l]);
-    }
+    k_weight_bf16<<<(unsigned)((s->np + 255) / 256), 256, 0, s->stream>>>(s->P, s->weights);
     SCK(cudaGetLastError());
     return HIDEM_OK;
 }
@@ -1367,7 +1428,7 @@ hidem_status mlp_forward_t(hidem_surrogate *s, const bf16 *X, int rows, float *Y
 
 // The same pass as the persistent ping-pong kernel (k_mlp_pp, 256-wide networks): one CTA
 // per SM at most, each taking pairs of 128-row blocks.
-hidem_status mlp_forward_pp(hidem_surrogate *s, const bf16 *X, int rows, float *Y, bool keepZ) {
+hidem_status mlp_forward_pp(hidem_surrogate *s, const bf16 *X, int rows, int live, float *Y, bool keepZ) {
     static std::atomic<unsigned long long> configured{0};
     int dev = 0;
     cudaGetDevice(&dev);
@@ -1395,16 +1456,20 @@ hidem_status mlp_forward_pp(hidem_surrogate *s, const bf16 *X, int rows, float *
     a.bo = s->P + s->offBo;
     a.y = Y;
     a.err = s->dErr;
-    const int pairs = (rows / 128 + 1) / 2;
-    const int grid = std::min(pairs, std::max(1, s->smCount));
+    const int sms = std::max(1, s->smCount);
+    a.liveRows = live;
+    a.perGroup = rows / 128 <= sms ? 1 : 2;
+    const int groups = (rows / 128 + a.perGroup - 1) / a.perGroup;
+    const int grid = std::min(groups, sms);
     k_mlp_pp<256><<<grid, kPPThreads, pp_smem_bytes(), s->stream>>>(maps, a, rows);
     SCK(cudaGetLastError());
     return HIDEM_OK;
 }
 
+bool ping_pong(const hidem_surrogate *s) { return s->W == 256 && s->forwardKind != HIDEM_SURROGATE_FORWARD_BLOCK; }
+
 hidem_status mlp_forward(hidem_surrogate *s, const bf16 *X, int rows, float *Y, bool keepZ) {
-    if (s->W == 256 && s->forwardKind != HIDEM_SURROGATE_FORWARD_BLOCK)
-        return mlp_forward_pp(s, X, rows, Y, keepZ);
+    if (ping_pong(s)) return mlp_forward_pp(s, X, rows, rows, Y, keepZ);
     return s->W == 256 ? mlp_forward_t<256>(s, X, rows, Y, keepZ) : mlp_forward_t<128>(s, X, rows, Y, keepZ);
 }
 
@@ -1412,62 +1477,73 @@ hidem_status forward(hidem_surrogate *s, int rows, bool keepZ) {
     return mlp_forward(s, s->X0, rows, s->Y, keepZ);
 }
 
-// loss and all gradients into G for the rows of X0 (targets[idx[b]] or targets[b])
+// a step of work on `to` that must see everything queued on `from` so far
+hidem_status order_after(hidem_surrogate *s, cudaStream_t from, cudaStream_t to, cudaEvent_t e) {
+    SCK(cudaEventRecord(e, from));
+    SCK(cudaStreamWaitEvent(to, e, 0));
+    return HIDEM_OK;
+}
+
+// Loss and all gradients into G for the rows of X0 (targets[idx[b]] or targets[b]).
+// The chain of data gradients (dZ of the last layer down to the first) is the critical path
+// and runs on the surrogate's stream; each layer's weight and bias gradients, and the loss with
+// the output layer's, need only that layer's dZ and run beside it on a stream of their own,
+// in buffers of their own. A settling batch (8,192 rows) is some forty kernels of 3-20 us that
+// fill a fraction of the chip each: one after another they took 0.36 of the step's 0.48 ms.
+// The sums and their order are those of the serial chain.
 hidem_status backward(hidem_surrogate *s, int rows, const float *targets, const int *idx) {
     const int W = s->W, L = s->L;
     const int nb = (rows + 255) / 256;
-    k_loss<<<nb, 256, 0, s->stream>>>(s->Y, targets, idx, rows, s->dY, s->lossPart);
-    // output layer
     const int chunks = (rows + kChunk - 1) / kChunk;
-    STRY(ensure_part(s, (long long)(chunks + 1) * kOut * (W + 1)));
-    k_out_grad<<<dim3((W + 1 + 31) / 32, chunks), dim3(32, 8), 0, s->stream>>>(s->dY, s->H[L - 1], rows, W, s->part);
-    // sum the chunk partials into a [3][W + 1] block, then split weights and biases
-    float *outBlock = s->part + (long long)chunks * kOut * (W + 1);
-    k_sum_splits<<<sum_splits_grid((long long)kOut * (W + 1)), dim3(32, 8), 0, s->stream>>>(s->part, chunks, (long long)kOut * (W + 1), outBlock);
-    for (int j = 0; j < kOut; ++j) {
-        SCK(cudaMemcpyAsync(s->G + s->offWo + (long long)j * W, outBlock + (long long)j * (W + 1),
-                            sizeof(float) * W, cudaMemcpyDeviceToDevice, s->stream));
-        SCK(cudaMemcpyAsync(s->G + s->offBo + j, outBlock + (long long)j * (W + 1) + W, sizeof(float),
-                            cudaMemcpyDeviceToDevice, s->stream));
-    }
-    bf16 *dZ = s->dZa, *dZn = s->dZb;
-    k_out_bwd<<<dim3((unsigned)rows, (unsigned)((W + 255) / 256)), 256, 0, s->stream>>>(s->dY, s->P + s->offWo, s->Z[L - 1], rows, W, dZ);
+    cudaStream_t st = s->stream, so = s->side[L];
+    // loss, output layer: chunk partials summed into a [3][W + 1] block, split into weights and biases
+    STRY(order_after(s, st, so, s->evForward));
+    k_loss<<<nb, 256, 0, so>>>(s->Y, targets, idx, rows, s->dY, s->lossPart);
+    k_out_grad<<<dim3((W + 1 + 31) / 32, chunks), dim3(32, 8), 0, so>>>(s->dY, s->H[L - 1], rows, W, s->partOut);
+    k_sum_out<<<sum_splits_grid((long long)kOut * (W + 1)), dim3(32, 8), 0, so>>>(s->partOut, chunks, W, s->G + s->offWo,
+                                                                               s->G + s->offBo);
+    SCK(cudaEventRecord(s->evDone[L], so));
+    k_out_bwd<<<dim3((unsigned)rows, (unsigned)((W + 255) / 256)), 256, 0, st>>>(s->Y, targets, idx, s->P + s->offWo,
+                                                                               s->Z[L - 1], rows, W, s->dZ[L - 1]);
     SCK(cudaGetLastError());
     // hidden layers, last to first
     for (int l = L - 1; l >= 0; --l) {
         const int K = s->Kl[l];
         const bf16 *in = l == 0 ? s->X0 : s->H[l - 1];
+        bf16 *dZ = s->dZ[l];
+        cudaStream_t sl = s->side[l];
         // dW_l = dZ^T * in: both operands transposed to K-major [.][rows], split over rows
-        k_transpose<<<dim3((W + kTrTile - 1) / kTrTile, (rows + kTrTile - 1) / kTrTile), 256, 0, s->stream>>>(dZ, rows, W, s->dZT);
-        k_transpose<<<dim3((K + kTrTile - 1) / kTrTile, (rows + kTrTile - 1) / kTrTile), 256, 0, s->stream>>>(in, rows, K, s->inT);
+        SCK(cudaStreamWaitEvent(sl, s->evForward, 0));
+        k_transpose<<<dim3((K + kTrTile - 1) / kTrTile, (rows + kTrTile - 1) / kTrTile), 256, 0, sl>>>(in, rows, K, s->inT[l]);
+        STRY(order_after(s, st, sl, s->evDz[l]));
+        k_transpose<<<dim3((W + kTrTile - 1) / kTrTile, (rows + kTrTile - 1) / kTrTile), 256, 0, sl>>>(dZ, rows, W, s->dZT[l]);
+        if (l > 0) {
+            // dZ_{l-1} = (dZ_l * W_l) . SiLU'(Z_{l-1}); B operand W_l^T is [K_l][W]
+            GemmArgs gd{};
+            gd.outH = s->dZ[l - 1];
+            gd.zIn = s->Z[l - 1];
+            gd.ldo = K;
+            STRY(gemm_n<EPI_SILU_GRAD>(s, st, K, dZ, rows, W, s->WbT[l], 1, gd));
+        }
         int splits = s->splits;
         while (splits > 1 && ((rows / 64) % splits)) splits >>= 1;
-        STRY(ensure_part(s, (long long)splits * W * K));
         // columns of dW in tiles of 256 (then 128): rows n0.. of the K-major input
         for (int n0 = 0; n0 < K;) {
             const int bn = K - n0 >= 256 ? 256 : 128;
             GemmArgs g{};
-            g.outF = s->part + n0;
+            g.outF = s->part[l] + n0;
             g.splitStride = (long long)W * K;
             g.ldo = K;
-            STRY(gemm_n<EPI_F32>(s, bn, s->dZT, W, rows, s->inT + (long long)n0 * rows, splits, g));
+            STRY(gemm_n<EPI_F32>(s, sl, bn, s->dZT[l], W, rows, s->inT[l] + (long long)n0 * rows, splits, g));
             n0 += bn;
         }
-        k_sum_splits<<<sum_splits_grid((long long)W * K), dim3(32, 8), 0, s->stream>>>(s->part, splits, (long long)W * K, s->G + s->offW[l]);
+        k_sum_splits<<<sum_splits_grid((long long)W * K), dim3(32, 8), 0, sl>>>(s->part[l], splits, (long long)W * K, s->G + s->offW[l]);
         // db_l = column sums of dZ
-        STRY(ensure_part(s, (long long)chunks * W + W));
-        k_colsum_bf16<<<dim3((W + 63) / 64, chunks), dim3(32, 8), 0, s->stream>>>(dZ, rows, W, s->part);
-        k_sum_splits<<<sum_splits_grid(W), dim3(32, 8), 0, s->stream>>>(s->part, chunks, W, s->G + s->offB[l]);
-        if (l > 0) {
-            // dZ_{l-1} = (dZ_l * W_l) . SiLU'(Z_{l-1}); B operand W_l^T is [K_l][W]
-            GemmArgs gd{};
-            gd.outH = dZn;
-            gd.zIn = s->Z[l - 1];
-            gd.ldo = K;
-            STRY(gemm_n<EPI_SILU_GRAD>(s, K, dZ, rows, W, s->WbT[l], 1, gd));
-            std::swap(dZ, dZn);
-        }
+        k_colsum_bf16<<<dim3((W + 63) / 64, chunks), dim3(32, 8), 0, sl>>>(dZ, rows, W, s->partB[l]);
+        k_sum_splits<<<sum_splits_grid(W), dim3(32, 8), 0, sl>>>(s->partB[l], chunks, W, s->G + s->offB[l]);
+        SCK(cudaEventRecord(s->evDone[l], sl));
     }
+    for (int l = 0; l <= L; ++l) SCK(cudaStreamWaitEvent(st, s->evDone[l], 0));
     SCK(cudaGetLastError());
     return HIDEM_OK;
 }
@@ -1482,10 +1558,11 @@ hidem_status read_loss(hidem_surrogate *s, int rows, double *loss) {
     return HIDEM_OK;
 }
 
+// waits for the stream, with the error flag travelling ahead of the wait into pinned memory
 hidem_status check_err(hidem_surrogate *s) {
-    int flag = 0;
-    SCK(cudaMemcpyAsync(&flag, s->dErr, sizeof(int), cudaMemcpyDeviceToHost, s->stream));
+    SCK(cudaMemcpyAsync(s->errHost, s->dErr, sizeof(int), cudaMemcpyDeviceToHost, s->stream));
     SCK(cudaStreamSynchronize(s->stream));
+    const int flag = *s->errHost;
     if (flag) {
         SCK(cudaMemsetAsync(s->dErr, 0, sizeof(int), s->stream));
         return sfail(s, HIDEM_ERR_DEVICE, "tensor-core GEMM: %s",
@@ -1516,15 +1593,17 @@ void hidem_surrogate_destroy(hidem_surrogate *s) {
     if (!s) return;
     cudaSetDevice(s->device);
     if (s->stream) cudaStreamSynchronize(s->stream);
-    void *bufs[] = {s->P, s->G, s->Mm, s->Vv, s->X0, s->Y, s->dY, s->dZa, s->dZb, s->dZT, s->inT,
-                    s->part, s->lossPart, s->idx, s->dataIn, s->dataT, s->scratchIn, s->scratchT, s->dErr,
-                    s->predIn, s->predY, s->predX};
-    for (void *b : bufs)
+    for (cudaStream_t t : s->side)
+        if (t) {
+            cudaStreamSynchronize(t);
+            cudaStreamDestroy(t);
+        }
+    for (const auto &v : {s->evDz, s->evDone})
+        for (cudaEvent_t e : v)
+            if (e) cudaEventDestroy(e);
+    if (s->evForward) cudaEventDestroy(s->evForward);
+    for (void *b : {(void *)s->arena, (void *)s->dataIn, (void *)s->dataT})
         if (b) cudaFree(b);
-    for (auto *p : s->Wb) if (p) cudaFree(p);
-    for (auto *p : s->WbT) if (p) cudaFree(p);
-    for (auto *p : s->Z) if (p) cudaFree(p);
-    for (auto *p : s->H) if (p) cudaFree(p);
     if (s->lossHost) cudaFreeHost(s->lossHost);
     if (s->stream) cudaStreamDestroy(s->stream);
     delete s;
@@ -1574,8 +1653,6 @@ hidem_status hidem_surrogate_create(const hidem_surrogate_config *c, int device,
     off += kOut;
     s->np = off;
     const int chunks = (B + kChunk - 1) / kChunk;
-    long long partNeed = std::max<long long>((long long)(chunks + 1) * kOut * (W + 1), (long long)chunks * W + W);
-    partNeed = std::max<long long>(partNeed, (long long)s->splits * W * std::max(W, K0));
     auto fail = [&](cudaError_t e) {
         err = std::string("surrogate setup failed: ") + cudaGetErrorString(e);
         hidem_surrogate_destroy(s);
@@ -1583,45 +1660,81 @@ hidem_status hidem_surrogate_create(const hidem_surrogate_config *c, int device,
     };
     cudaError_t e = cudaSetDevice(device);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&s->smCount, cudaDevAttrMultiProcessorCount, device);
-    if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking);
+    // the surrogate's stream before its side streams wherever both have CTAs to place
+    int low = 0, high = 0;
+    if (e == cudaSuccess) e = cudaDeviceGetStreamPriorityRange(&low, &high);
+    if (e == cudaSuccess) e = cudaStreamCreateWithPriority(&s->stream, cudaStreamNonBlocking, high);
+    // one allocation for every buffer: sized by a first round, handed out by a second
+    size_t arenaBytes = 0;
+    char *arena = nullptr;
     auto dm = [&](void **p, size_t bytes) {
-        if (e == cudaSuccess) e = cudaMalloc(p, bytes);
+        if (arena) *p = arena + arenaBytes;
+        arenaBytes += (bytes + 255) / 256 * 256;
     };
-    dm((void **)&s->dErr, sizeof(int));
-    dm((void **)&s->P, sizeof(float) * s->np);
-    dm((void **)&s->G, sizeof(float) * s->np);
-    dm((void **)&s->Mm, sizeof(float) * s->np);
-    dm((void **)&s->Vv, sizeof(float) * s->np);
     s->Wb.assign(L, nullptr);
     s->WbT.assign(L, nullptr);
     s->Z.assign(L, nullptr);
     s->H.assign(L, nullptr);
-    for (int l = 0; l < L; ++l) {
-        dm((void **)&s->Wb[l], sizeof(bf16) * W * s->Kl[l]);
-        dm((void **)&s->WbT[l], sizeof(bf16) * W * s->Kl[l]);
-        dm((void **)&s->Z[l], sizeof(float) * (size_t)B * W);
-        dm((void **)&s->H[l], sizeof(bf16) * (size_t)B * W);
-    }
-    dm((void **)&s->X0, sizeof(bf16) * (size_t)B * K0);
-    dm((void **)&s->Y, sizeof(float) * (size_t)B * kOut);
-    dm((void **)&s->dY, sizeof(float) * (size_t)B * kOut);
-    dm((void **)&s->dZa, sizeof(bf16) * (size_t)B * W);
-    dm((void **)&s->dZb, sizeof(bf16) * (size_t)B * W);
-    dm((void **)&s->dZT, sizeof(bf16) * (size_t)B * W);
-    dm((void **)&s->inT, sizeof(bf16) * (size_t)B * std::max(W, K0));
-    dm((void **)&s->part, sizeof(float) * partNeed);
-    s->partCap = partNeed;
-    dm((void **)&s->lossPart, sizeof(float) * ((B + 255) / 256));
-    dm((void **)&s->idx, sizeof(int) * B);
-    dm((void **)&s->scratchIn, sizeof(float) * (size_t)B * s->nin);
-    dm((void **)&s->scratchT, sizeof(float) * (size_t)B * kOut);
-    // rows per predict chunk: with the persistent forward pass, 1,024 block pairs per chunk
-    // keep the last round of pairs over the SMs a small share of a chunk
+    for (auto *v : {&s->dZ, &s->dZT, &s->inT}) v->assign(L, nullptr);
+    for (auto *v : {&s->part, &s->partB}) v->assign(L, nullptr);
     s->PB = std::max(B, 262144);
-    dm((void **)&s->predIn, sizeof(float) * (size_t)s->PB * s->nin);
-    dm((void **)&s->predY, sizeof(float) * (size_t)s->PB * kOut);
-    dm((void **)&s->predX, sizeof(bf16) * (size_t)s->PB * K0);
-    if (e == cudaSuccess) e = cudaMallocHost((void **)&s->lossHost, sizeof(float) * ((B + 255) / 256));
+    auto buffers = [&]() {
+        dm((void **)&s->dErr, sizeof(int));
+        dm((void **)&s->P, sizeof(float) * s->np);
+        dm((void **)&s->G, sizeof(float) * s->np);
+        dm((void **)&s->Mm, sizeof(float) * s->np);
+        dm((void **)&s->Vv, sizeof(float) * s->np);
+        for (int l = 0; l < L; ++l) {
+            dm((void **)&s->Wb[l], sizeof(bf16) * W * s->Kl[l]);
+            dm((void **)&s->WbT[l], sizeof(bf16) * W * s->Kl[l]);
+            dm((void **)&s->Z[l], sizeof(float) * (size_t)B * W);
+            dm((void **)&s->H[l], sizeof(bf16) * (size_t)B * W);
+            dm((void **)&s->dZ[l], sizeof(bf16) * (size_t)B * W);
+            dm((void **)&s->dZT[l], sizeof(bf16) * (size_t)B * W);
+            dm((void **)&s->inT[l], sizeof(bf16) * (size_t)B * s->Kl[l]);
+            dm((void **)&s->part[l], sizeof(float) * (size_t)s->splits * W * s->Kl[l]);
+            dm((void **)&s->partB[l], sizeof(float) * (size_t)chunks * W);
+        }
+        dm((void **)&s->partOut, sizeof(float) * (size_t)chunks * kOut * (W + 1));
+        dm((void **)&s->X0, sizeof(bf16) * (size_t)B * K0);
+        dm((void **)&s->Y, sizeof(float) * (size_t)B * kOut);
+        dm((void **)&s->dY, sizeof(float) * (size_t)B * kOut);
+        dm((void **)&s->lossPart, sizeof(float) * ((B + 255) / 256));
+        dm((void **)&s->idx, sizeof(int) * B);
+        dm((void **)&s->scratchIn, sizeof(float) * (size_t)B * s->nin);
+        dm((void **)&s->scratchT, sizeof(float) * (size_t)B * kOut);
+        dm((void **)&s->predIn, sizeof(float) * (size_t)s->PB * s->nin);
+        dm((void **)&s->predY, sizeof(float) * (size_t)s->PB * kOut);
+        dm((void **)&s->predX, sizeof(bf16) * (size_t)s->PB * K0);
+    };
+    buffers();
+    if (e == cudaSuccess) e = cudaMalloc((void **)&s->arena, arenaBytes);
+    if (e != cudaSuccess) return fail(e);
+    arena = s->arena;
+    arenaBytes = 0;
+    buffers();
+    auto event = [&](cudaEvent_t *ev) {
+        if (e == cudaSuccess) e = cudaEventCreateWithFlags(ev, cudaEventDisableTiming);
+    };
+    s->side.assign(L + 1, nullptr);
+    s->evDz.assign(L, nullptr);
+    s->evDone.assign(L + 1, nullptr);
+    for (int l = 0; l < L; ++l) event(&s->evDz[l]);
+    for (int l = 0; l <= L; ++l) {
+        if (e == cudaSuccess) e = cudaStreamCreateWithPriority(&s->side[l], cudaStreamNonBlocking, low);
+        event(&s->evDone[l]);
+    }
+    event(&s->evForward);
+    s->weights.layers = L;
+    s->weights.W = W;
+    for (int l = 0; l < L; ++l) {
+        s->weights.K[l] = s->Kl[l];
+        s->weights.off[l] = s->offW[l];
+        s->weights.wb[l] = s->Wb[l];
+        s->weights.wbT[l] = s->WbT[l];
+    }
+    if (e == cudaSuccess) e = cudaMallocHost((void **)&s->lossHost, sizeof(float) * ((B + 255) / 256 + 1));
+    s->errHost = reinterpret_cast<int *>(s->lossHost + (B + 255) / 256);
     if (e == cudaSuccess) e = cudaMemsetAsync(s->dErr, 0, sizeof(int), s->stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(s->Mm, 0, sizeof(float) * s->np, s->stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(s->Vv, 0, sizeof(float) * s->np, s->stream);
@@ -1700,8 +1813,8 @@ hidem_status hidem_surrogate_train(hidem_surrogate *s, int32_t steps, double *lo
     SCK(cudaSetDevice(s->device));
     const int B = s->B;
     for (int it = 0; it < steps; ++it) {
-        k_sample<<<(B + 255) / 256, 256, 0, s->stream>>>(s->cfg.seed, (unsigned long long)s->steps, B, s->nData, s->idx);
-        k_features<<<(B + 7) / 8, dim3(32, 8), 0, s->stream>>>(s->dataIn, s->idx, B, s->nin, s->cfg.fourier_bands, s->K0, s->X0);
+        k_features<<<(B + 7) / 8, dim3(32, 8), 0, s->stream>>>(s->dataIn, s->idx, s->cfg.seed, (unsigned long long)s->steps,
+                                                              s->nData, B, B, s->nin, s->cfg.fourier_bands, s->K0, s->X0);
         STRY(forward(s, B, true));
         STRY(backward(s, B, s->dataT, s->idx));
         s->steps += 1;
@@ -1710,8 +1823,8 @@ hidem_status hidem_surrogate_train(hidem_surrogate *s, int32_t steps, double *lo
         double lr = s->cfg.learning_rate;
         if (s->cfg.cosine_decay) lr *= 0.5 * (1.0 + std::cos(3.14159265358979 * it / (double)steps));
         k_adam<<<(unsigned)((s->np + 255) / 256), 256, 0, s->stream>>>(s->P, s->G, s->Mm, s->Vv, s->np,
-                                                                      (float)lr, b1, b2, 1e-8f, c1, c2);
-        STRY(refresh_bf16(s));
+                                                                      (float)lr, b1, b2, 1e-8f, c1, c2, s->weights);
+        SCK(cudaGetLastError());
     }
     if (steps > 0 && loss) STRY(read_loss(s, B, loss));
     return check_err(s);
@@ -1725,13 +1838,11 @@ hidem_status hidem_surrogate_predict(hidem_surrogate *s, const float *inputs, in
     for (int64_t r0 = 0; r0 < n; r0 += PB) {
         const int rows = (int)std::min<int64_t>(PB, n - r0);
         const int padded = (rows + 127) / 128 * 128;
-        if (padded > rows) SCK(cudaMemsetAsync(s->predIn, 0, sizeof(float) * s->nin * padded, s->stream));
         SCK(cudaMemcpyAsync(s->predIn, inputs + r0 * s->nin, sizeof(float) * s->nin * rows, cudaMemcpyHostToDevice, s->stream));
-        k_features<<<(padded + 7) / 8, dim3(32, 8), 0, s->stream>>>(s->predIn, nullptr, padded, s->nin, s->cfg.fourier_bands, s->K0, s->predX);
+        k_features<<<(padded + 7) / 8, dim3(32, 8), 0, s->stream>>>(s->predIn, nullptr, 0, 0, 0, padded, rows, s->nin, s->cfg.fourier_bands, s->K0, s->predX);
         STRY(mlp_forward(s, s->predX, padded, s->predY, false));
         SCK(cudaMemcpyAsync(out + r0 * kOut, s->predY, sizeof(float) * kOut * rows, cudaMemcpyDeviceToHost, s->stream));
     }
-    SCK(cudaStreamSynchronize(s->stream));
     return check_err(s);
 }
 
@@ -1739,26 +1850,26 @@ hidem_status hidem_surrogate_predict_device(hidem_surrogate *s, const float *inp
     if (!s) return HIDEM_ERR_ARG;
     if (!inputs || !out || n < 0) return sfail(s, HIDEM_ERR_ARG, "bad arguments");
     SCK(cudaSetDevice(s->device));
-    const int PB = s->PB;
-    for (int64_t r0 = 0; r0 < n; r0 += PB) {
-        const int rows = (int)std::min<int64_t>(PB, n - r0);
-        const int padded = (rows + 127) / 128 * 128;
-        const float *in = inputs + r0 * s->nin;
-        if (padded > rows) {
-            // the ragged last chunk: zero rows up to the next multiple of 128
-            SCK(cudaMemsetAsync(s->predIn, 0, sizeof(float) * s->nin * padded, s->stream));
-            SCK(cudaMemcpyAsync(s->predIn, in, sizeof(float) * s->nin * rows, cudaMemcpyDeviceToDevice, s->stream));
-            in = s->predIn;
+    // chunks of whole rounds of block pairs over the SMs, as equal as that allows: a chunk of the
+    // buffer's size and a small rest cost a round of their own each
+    const int64_t round = 256ll * std::max(1, s->smCount);
+    const int64_t chunks = std::max<int64_t>(1, (n + s->PB - 1) / s->PB);
+    const int64_t step = std::min<int64_t>(s->PB, ((n + chunks - 1) / chunks + round - 1) / round * round);
+    for (int64_t r0 = 0; r0 < n; r0 += step) {
+        const int rows = (int)std::min<int64_t>(step, n - r0);
+        const int padded = (rows + 127) / 128 * 128;  // the ragged last block: zero rows
+        k_features<<<(padded + 7) / 8, dim3(32, 8), 0, s->stream>>>(inputs + r0 * s->nin, nullptr, 0, 0, 0, padded, rows,
+                                                                  s->nin, s->cfg.fourier_bands, s->K0, s->predX);
+        if (ping_pong(s)) {
+            STRY(mlp_forward_pp(s, s->predX, padded, rows, out + r0 * kOut, false));
+            continue;
         }
-        k_features<<<(padded + 7) / 8, dim3(32, 8), 0, s->stream>>>(in, nullptr, padded, s->nin, s->cfg.fourier_bands,
-                                                                  s->K0, s->predX);
         float *y = padded > rows ? s->predY : out + r0 * kOut;
         STRY(mlp_forward(s, s->predX, padded, y, false));
         if (padded > rows)
             SCK(cudaMemcpyAsync(out + r0 * kOut, s->predY, sizeof(float) * kOut * rows, cudaMemcpyDeviceToDevice,
                                 s->stream));
     }
-    SCK(cudaStreamSynchronize(s->stream));
     return check_err(s);
 }
 
@@ -1784,12 +1895,11 @@ hidem_status hidem_surrogate_gradients(hidem_surrogate *s, const float *inputs, 
     const int rows = (int)n;
     SCK(cudaMemcpyAsync(s->scratchIn, inputs, sizeof(float) * s->nin * rows, cudaMemcpyHostToDevice, s->stream));
     SCK(cudaMemcpyAsync(s->scratchT, targets, sizeof(float) * kOut * rows, cudaMemcpyHostToDevice, s->stream));
-    k_features<<<(rows + 7) / 8, dim3(32, 8), 0, s->stream>>>(s->scratchIn, nullptr, rows, s->nin, s->cfg.fourier_bands, s->K0, s->X0);
+    k_features<<<(rows + 7) / 8, dim3(32, 8), 0, s->stream>>>(s->scratchIn, nullptr, 0, 0, 0, rows, rows, s->nin, s->cfg.fourier_bands, s->K0, s->X0);
     STRY(forward(s, rows, true));
     STRY(backward(s, rows, s->scratchT, nullptr));
     STRY(read_loss(s, rows, loss));
     SCK(cudaMemcpyAsync(grads, s->G, sizeof(float) * s->np, cudaMemcpyDeviceToHost, s->stream));
-    SCK(cudaStreamSynchronize(s->stream));
     return check_err(s);
 }
 
