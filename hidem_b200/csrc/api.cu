@@ -401,7 +401,6 @@ hidem_status check_device_error(hidem_ctx *ctx) {
         const char *what = flag == 1   ? "particle outside the grid bounds"
                            : flag == 2 ? "more than 65535 contacts for one particle"
                            : flag == 3 ? "more than 65535 link ends for one particle"
-                           : flag == 4 ? "shared-memory staging copies did not complete in time"
                            : flag == 5 ? "more than 4096 particles in one neighbour-grid cell"
                                        : "device check failed";
         return fail(ctx, flag == 5 ? HIDEM_ERR_CAPACITY : HIDEM_ERR_DEVICE, "device check %d: %s", flag, what);
@@ -824,14 +823,16 @@ hidem_status profile_pair(hidem_ctx *ctx, cudaEvent_t *e0, cudaEvent_t *e1) {
     return HIDEM_OK;
 }
 
-// Step-kernel autotuner: the first kTuneRounds * 3 fused steps of a context cycle
-// through the candidate kernels with an event pair around each launch; after the rounds
-// have run, the fastest (summed over all but the first round) is kept.
-constexpr int kTuneCandidates[] = {HIDEM_STEP_KERNEL_ITEMS, HIDEM_STEP_KERNEL_THREAD,
-                                   HIDEM_STEP_KERNEL_THREAD_CAPPED, HIDEM_STEP_KERNEL_THREAD_ASYNC,
-                                   HIDEM_STEP_KERNEL_TWO_PASS};
+// The step kernel of AUTO. A context of more than kTuneMax particles takes the two-pass step:
+// 5.7M particles 1.44 ms a step against 2.17 ms for the best one-kernel step (mixed), 0.8M
+// 0.24 ms against 0.34 ms. Smaller ones time the item kernel against it: the first kTuneRounds * 2 steps of
+// the context alternate with an event pair around each; the faster, summed over all but the
+// first round, is kept (8,892 particles in FP64: 14.5 us a step against 22.0 us; 32,000 mixed:
+// 24.3 against 23.3 us).
+constexpr long long kTuneMax = 65536;
+constexpr int kTuneCandidates[] = {HIDEM_STEP_KERNEL_ITEMS, HIDEM_STEP_KERNEL_TWO_PASS};
 constexpr int kNumCandidates = (int)(sizeof(kTuneCandidates) / sizeof(int));
-constexpr int kTuneRounds = 3;
+constexpr int kTuneRounds = 5;
 static_assert(2 * kNumCandidates * kTuneRounds <= (int)(sizeof(hidem_ctx::tuneEv) / sizeof(cudaEvent_t)),
               "one event pair per tuning step");
 
@@ -842,6 +843,7 @@ int step_kernel_now(hidem_ctx *ctx, cudaEvent_t *e0, cudaEvent_t *e1) {
     *e0 = *e1 = nullptr;
     if (ctx->stepKernel != HIDEM_STEP_KERNEL_AUTO) return ctx->stepKernel;
     if (ctx->tunedKernel != HIDEM_STEP_KERNEL_AUTO) return ctx->tunedKernel;
+    if (ctx->n > kTuneMax) return ctx->tunedKernel = HIDEM_STEP_KERNEL_TWO_PASS;
     if (ctx->tuneStep < kNumCandidates * kTuneRounds) {
         const int k = ctx->tuneStep++;
         for (int q = 0; q < 2; ++q)
@@ -851,14 +853,14 @@ int step_kernel_now(hidem_ctx *ctx, cudaEvent_t *e0, cudaEvent_t *e1) {
         *e1 = ctx->tuneEv[2 * k + 1];
         return kTuneCandidates[k % kNumCandidates];
     }
-    return HIDEM_STEP_KERNEL_THREAD;  // rounds done, choice made at the next sync
+    return HIDEM_STEP_KERNEL_TWO_PASS;  // rounds done, choice made at the next sync
 }
 
 // the kernel of a launch outside the tuning rounds
 int step_kernel_settled(const hidem_ctx *ctx) {
     if (ctx->stepKernel != HIDEM_STEP_KERNEL_AUTO) return ctx->stepKernel;
     if (ctx->tunedKernel != HIDEM_STEP_KERNEL_AUTO) return ctx->tunedKernel;
-    return HIDEM_STEP_KERNEL_THREAD;
+    return HIDEM_STEP_KERNEL_TWO_PASS;
 }
 
 // called after the stream has been synchronised
@@ -872,7 +874,7 @@ void step_kernel_resolve(hidem_ctx *ctx) {
         if (!ctx->tuneEv[2 * k] || !ctx->tuneEv[2 * k + 1] ||
             cudaEventElapsedTime(&ms, ctx->tuneEv[2 * k], ctx->tuneEv[2 * k + 1]) != cudaSuccess) {
             cudaGetLastError();
-            ctx->tunedKernel = HIDEM_STEP_KERNEL_THREAD;
+            ctx->tunedKernel = HIDEM_STEP_KERNEL_TWO_PASS;
             return;
         }
         t[k % kNumCandidates] += ms;
@@ -952,7 +954,8 @@ hidem_status run_steps(hidem_ctx *ctx, int nsteps) {
             recStale = !last;
             ctx->launches += 2;
         } else {
-            launch_step<LP>(consts<LP>(ctx), a, (int)ctx->maxNeigh, (int)ctx->maxLinksPP, kern, ctx->stream);
+            launch_step<LP>(consts<LP>(ctx), a, (int)ctx->maxNeigh, (int)ctx->maxLinksPP, kern, ctx->smCount,
+                            ctx->stream);
             ctx->launches += 1;
             ctx->cur = 1 - ctx->cur;  // the slot order (type / orig / cellOf) is unchanged
         }
@@ -1471,7 +1474,7 @@ hidem_status batch_run(hidem_batch *b, int nsteps) {
                     if (a.reduceDiff)
                         BCK(cudaMemsetAsync(c->diffMax, 0, 3 * sizeof(unsigned long long), b->stream));
                     launch_step<LP>(consts<LP>(c), a, (int)c->maxNeigh, (int)c->maxLinksPP,
-                                    fused_kernel(step_kernel_settled(c)), b->stream);
+                                    fused_kernel(step_kernel_settled(c)), c->smCount, b->stream);
                     c->launches += 1;
                     b->launches += 1;
                 }

@@ -7,27 +7,10 @@ namespace hidem {
 constexpr int kStepThreads = 128;
 constexpr int kItemThreads = 256;
 constexpr size_t kItemSmemLimit = 200 * 1024;
-// Byte offsets of the item kernel's shared-memory regions (same for all CTAs of a launch):
-// mbarrier, own records (AoS as copied, then SoA), contact indices, the link-end streams
-// partner word / CT0..CT5 / state / initial length, then the force terms.
-struct StageLayout {
-    size_t own, soa, nbr, spw, sct, sst, sl0, terms, total;
-};
-inline __host__ __device__ size_t stage_align(size_t v) { return (v + 127) & ~size_t(127); }
-inline __host__ __device__ StageLayout stage_layout(size_t rec, size_t lp, int maxContacts,
-                                                    int maxEnds) {
-    StageLayout L;
-    const size_t ends = (size_t)maxEnds * 32;
-    L.own = 128;
-    L.soa = stage_align(L.own + 32 * rec);
-    L.nbr = stage_align(L.soa + 96 * 8 + 320 * lp + 64 * 4);
-    L.spw = stage_align(L.nbr + (size_t)maxContacts * 32 * 4);
-    L.sct = stage_align(L.spw + ends * 4);
-    L.sst = stage_align(L.sct + 6 * ends * lp);
-    L.sl0 = stage_align(L.sst + ends);
-    L.terms = stage_align(L.sl0 + ends * lp);
-    L.total = stage_align(L.terms + (size_t)(maxContacts * 6 + maxEnds * 12) * 32 * lp);
-    return L;
+// shared memory of the item kernel: the force terms of a block of 32 particles (six per
+// contact, twelve per link end) and their sums
+inline size_t item_smem(size_t lp, int maxContacts, int maxEnds) {
+    return (size_t)(maxContacts * 6 + maxEnds * 12 + 6) * 32 * lp;
 }
 
 // One set of link-end ("side") arrays in the warp-blocked ELL layout.
@@ -157,7 +140,7 @@ void launch_side_fill(const int *orig, int n, const int *slotOf, const int *plSt
 // particle for rows too wide for its shared-memory buffers).
 template <class LP>
 void launch_step(const Consts<LP> &c, const StepArgs<LP> &a, int maxContacts, int maxEnds, int kernel,
-                 cudaStream_t s);
+                 int smCount, cudaStream_t s);
 // The force pass (a.gather holds the records in the gather layout), applying the previous
 // step's link update on the way when a.breakPending; the integrate pass on the gather layout
 // (rec: the records too, or null; reduce: the diff maxima into diffMax); and the two layouts'

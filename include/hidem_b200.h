@@ -245,8 +245,7 @@ hidem_status hidem_set_halo_exchange(hidem_ctx *ctx, const int32_t *send_index, 
 hidem_status hidem_pack_halo_forces(hidem_ctx *ctx, void *device_out);
 /* hidem_compute_forces followed by hidem_pack_halo_forces into `device_out`, with the send
  * records written by the force pass itself as it finishes each listed particle (the pack
- * fused into its epilogue; after the item and asynchronous-copy force kernels the pack
- * kernel runs instead). The same forces and records as the two calls. */
+ * fused into its epilogue). The same forces and records as the two calls. */
 hidem_status hidem_compute_forces_packed(hidem_ctx *ctx, void *device_out);
 /* Overwrites the forces of the receive list with n_recv x 6 lp values read from
  * `device_in` (device memory), on the context's stream; the caller has made the stream
@@ -507,19 +506,19 @@ hidem_status hidem_momentum(hidem_ctx *ctx, double linear[3], double angular[3])
 
 /* ---- step kernel choice ----------------------------------------------- */
 
-/* No counterpart in the reference. The fused step has several kernels that give
- * bit-identical results and differ only in speed: one thread per (particle, contact) and
- * (particle, link end) item with the block's streams staged in shared memory (ITEMS), one
- * thread per particle with software-pipelined partner loads (THREAD), and the same with
- * registers capped for more CTAs per SM (THREAD_CAPPED: five in the mixed build, three in
- * FP64), and one thread per particle whose next two items' partner data travel by
- * asynchronous copies into shared memory (THREAD_ASYNC). TWO_PASS runs each timestep as
- * the THREAD_CAPPED force pass without the integrate tail, then the integrate pass over
- * the particles and the break pass over the links, as hidem_compute_forces /
- * hidem_integrate / hidem_link_update do. AUTO (the default) times each on the context's
- * own first steps (three rounds, the first discarded) and keeps the fastest; those steps
- * are ordinary timesteps. hidem_get_step_kernel returns the kernel in use (AUTO while
- * still timing). */
+/* No counterpart in the reference. A timestep has several kernels that give bit-identical
+ * results and differ only in speed: one warp lane per particle of a 32-particle block with the
+ * block's contacts and link ends spread over the CTA's warps (ITEMS), one thread per particle
+ * with software-pipelined partner loads (THREAD), the same with registers capped for more CTAs
+ * per SM (THREAD_CAPPED: five in the mixed build, three in FP64), and one thread per particle
+ * whose next two items' partner data travel by asynchronous copies into shared memory
+ * (THREAD_ASYNC); TWO_PASS runs each timestep as a force pass, which applies the previous
+ * step's link update on the way, and an integrate pass, the state kept between them in a
+ * layout of its own until the call's last step. AUTO (the default) is TWO_PASS above 65,536
+ * particles; a smaller context times ITEMS against it on its own first steps (five rounds, the
+ * first discarded) and keeps the faster; those steps are ordinary timesteps.
+ * hidem_get_step_kernel returns the kernel in use (AUTO before the first step and while still
+ * timing). */
 #define HIDEM_STEP_KERNEL_AUTO 0
 #define HIDEM_STEP_KERNEL_ITEMS 1
 #define HIDEM_STEP_KERNEL_THREAD 2
