@@ -128,6 +128,7 @@ struct hidem_ctx {
     int32_t *cellOf[2] = {nullptr, nullptr};
     int32_t *slotOf = nullptr;
     int32_t *perm = nullptr;
+    int32_t *newSlot = nullptr;  // of every slot of the layout before the last rebuild
     int32_t *bigCells = nullptr;  // crowded cells of a rebuild's sort (n / 32 + 2 entries, count last)
     int32_t *haloSendPos = nullptr;  // per slot: position in the halo send list, or -1
     void *force = nullptr;
@@ -145,6 +146,8 @@ struct hidem_ctx {
     uint32_t *counts = nullptr;
     int *blockWidth = nullptr;
     long long *nOff = nullptr, *sOff = nullptr, *offTotal = nullptr;
+    long long *sOffOld = nullptr;  // the link ends' offsets before the last rebuild
+    bool sidesBlocked = false;     // the link ends lie in the blocked layout of sOff
     int32_t *nbr = nullptr;
     long long nbrCap = 0;
     long long numPairs = 0, maxNeigh = 0, maxLinksPP = 0;
@@ -553,7 +556,7 @@ hidem_status rebuild(hidem_ctx *ctx) {
                                        ctx->errorFlag, 5, ctx->smCount, st);
     launch_permute<LP>(ctx->perm, n, recp<LP>(ctx, cur), recp<LP>(ctx, nxt), ctx->type[od],
                        ctx->type[nd], ctx->orig[od], ctx->orig[nd], ctx->cellOf[od],
-                       ctx->cellOf[nd], ctx->slotOf, st);
+                       ctx->cellOf[nd], ctx->slotOf, ctx->newSlot, st);
     ctx->launches += 3;
     if (ctx->L > 0) {
         launch_link_slots(ctx->linkA, ctx->linkB, ctx->slotOf, ctx->L, ctx->linkSlotA, ctx->linkSlotB, st);
@@ -563,6 +566,10 @@ hidem_status rebuild(hidem_ctx *ctx) {
         launch_send_pos(ctx->slotOf, ctx->haloSend, ctx->nHaloSend, n, ctx->haloSendPos, st);
         ctx->launches += 1;
     }
+    // until the link ends follow, they lie in a layout that `perm` does not start from: a rebuild
+    // after one that fails below goes through the links
+    const bool sidesBlocked = ctx->sidesBlocked;
+    ctx->sidesBlocked = false;
     ctx->cur = nxt;
     ctx->ord = nd;
     const int c = nd;   // slot-order arrays
@@ -571,25 +578,29 @@ hidem_status rebuild(hidem_ctx *ctx) {
     // 4. contact list (NeighAccel::generateNeighbours: count pass, widths, fill pass)
     const long long nb32 = nblocks32(n);
     CK(cudaMemsetAsync(ctx->blockWidth, 0, sizeof(int) * (size_t)(nb32 + 1), st));
-    launch_nbr_count<LP>(recp<LP>(ctx, rc), n, ctx->cellOf[c], g, ctx->cellStart, ctx->cellCount,
+    // candidates are read from the gather layout, in the buffer of the old records
+    launch_to_gather<LP>(recp<LP>(ctx, rc), n, static_cast<int4 *>(ctx->rec[cur]), st);
+    ctx->launches += 1;
+    const int4 *places = static_cast<const int4 *>(ctx->rec[cur]);
+    launch_nbr_count<LP>(places, n, ctx->cellOf[c], g, ctx->cellStart, ctx->cellCount,
                          ctx->interactDist, ctx->counts, ctx->blockWidth, ctx->errorFlag, st);
     ctx->launches += 1;
     ctx->launches += launch_scan<int, long long>(ctx->blockWidth, nb32 + 1, 32ll, ctx->nOff,
                                                  ctx->scanSums64, ctx->offTotal, st);
     long long nTotal = 0;
     CK(cudaMemcpyAsync(&nTotal, ctx->offTotal, sizeof nTotal, cudaMemcpyDeviceToHost, st));
-    CK(cudaStreamSynchronize(st));
-    TRY(check_device_error(ctx));
+    TRY(check_device_error(ctx));  // waits for both
     if (nTotal > ctx->nbrCap) {
         long long cap = nTotal + nTotal / 8 + 1024;
         TRY(dalloc(ctx, &ctx->nbr, cap));
         ctx->nbrCap = cap;
     }
-    launch_nbr_fill<LP>(recp<LP>(ctx, rc), n, ctx->cellOf[c], g, ctx->cellStart, ctx->cellCount,
+    launch_nbr_fill<LP>(places, n, ctx->cellOf[c], g, ctx->cellStart, ctx->cellCount,
                         ctx->interactDist, ctx->nOff, ctx->nbr, st);
     ctx->launches += 1;
 
     // 5. link ends in the new slot order (LinkAccelSide::generateLinks + sortSideData)
+    std::swap(ctx->sOff, ctx->sOffOld);
     CK(cudaMemsetAsync(ctx->blockWidth, 0, sizeof(int) * (size_t)(nb32 + 1), st));
     launch_side_count(ctx->orig[c], n, ctx->plStart, ctx->counts, ctx->blockWidth, ctx->errorFlag, st);
     ctx->launches += 1;
@@ -600,14 +611,17 @@ hidem_status rebuild(hidem_ctx *ctx) {
     ctx->launches += 1;
     long long tot[4] = {0, 0, 0, 0};
     CK(cudaMemcpyAsync(tot, ctx->offTotal, sizeof tot, cudaMemcpyDeviceToHost, st));
-    CK(cudaStreamSynchronize(st));
     TRY(check_device_error(ctx));
     const long long sTotal = tot[0];
     if (sTotal >= (1ll << 31))
         return fail(ctx, HIDEM_ERR_CAPACITY, "%lld link-end slots (limit 2^31)", sTotal);
     // side[0] / sideSlot[0] hold the current layout; the new one is built in [1], then swapped
     TRY(side_alloc(ctx, ctx->side[1], std::max<long long>(sTotal, 2 * ctx->L)));
-    if (ctx->L > 0) {
+    if (ctx->L > 0 && sidesBlocked) {
+        launch_side_move<LP>(ctx->perm, n, ctx->newSlot, ctx->counts, ctx->sOffOld, side_view<LP>(ctx->side[0]),
+                             ctx->sOff, side_view<LP>(ctx->side[1]), ctx->sideSlot[1], st);
+        ctx->launches += 1;
+    } else if (ctx->L > 0) {
         launch_side_fill<LP>(ctx->orig[c], n, ctx->slotOf, ctx->plStart, ctx->plLink, ctx->plEnd,
                              ctx->linkA, ctx->linkB, static_cast<const LP *>(ctx->L0link),
                              ctx->sideSlot[0], side_view<LP>(ctx->side[0]), ctx->sOff,
@@ -617,6 +631,7 @@ hidem_status rebuild(hidem_ctx *ctx) {
     std::swap(ctx->sideSlot[0], ctx->sideSlot[1]);
     std::swap(ctx->side[0], ctx->side[1]);
 
+    ctx->sidesBlocked = true;
     ctx->numPairs = tot[1];
     ctx->maxNeigh = tot[2];
     ctx->maxLinksPP = tot[3];
@@ -922,8 +937,8 @@ hidem_status run_steps(hidem_ctx *ctx, int nsteps) {
         }
         if (gs_decide(ctx, currDist)) {
             records_now();
-            gathered = false;
             TRY(do_rebuild(ctx));
+            gathered = true;  // the rebuild walked it
         }
         const bool reduce = ctx->P.gridRegenInterval == -1 && (t + 1) % 10 == 0;
         diffReady = reduce;
@@ -1636,6 +1651,8 @@ void hidem_destroy(hidem_ctx *ctx) {
     }
     dfree(ctx->slotOf);
     dfree(ctx->perm);
+    dfree(ctx->newSlot);
+    dfree(ctx->sOffOld);
     dfree(ctx->bigCells);
     dfree(ctx->haloSendPos);
     dfree(ctx->force);
@@ -1732,6 +1749,7 @@ hidem_status hidem_set_particles(hidem_ctx *ctx, const hidem_particle_soa *p, in
     }
     TRY(dalloc(ctx, &ctx->slotOf, n));
     TRY(dalloc(ctx, &ctx->perm, n));
+    TRY(dalloc(ctx, &ctx->newSlot, n));
     TRY(dalloc(ctx, &ctx->bigCells, n / kSmallCell + 2));
     TRY(dalloc_bytes(ctx, &ctx->force, 6 * lp * (size_t)n));
     TRY(dalloc(ctx, &ctx->counts, n));
@@ -1739,6 +1757,7 @@ hidem_status hidem_set_particles(hidem_ctx *ctx, const hidem_particle_soa *p, in
     TRY(dalloc(ctx, &ctx->blockWidth, nb32 + 1));
     TRY(dalloc(ctx, &ctx->nOff, nb32 + 1));
     TRY(dalloc(ctx, &ctx->sOff, nb32 + 1));
+    TRY(dalloc(ctx, &ctx->sOffOld, nb32 + 1));
     ctx->cur = 0;
     ctx->ord = 0;
     TRY(ctx->mixed ? upload_particles<float>(ctx, p, n) : upload_particles<double>(ctx, p, n));
@@ -1890,6 +1909,7 @@ hidem_status hidem_set_links(hidem_ctx *ctx, const hidem_link_soa *l, int64_t L)
     side_free(ctx->side[1], st);
     TRY(side_alloc(ctx, ctx->side[0], 2 * L));
     ctx->curSide = 0;
+    ctx->sidesBlocked = false;
     TRY(dalloc(ctx, &ctx->events, std::max<long long>(L, 1)));
     ctx->eventCap = std::max<long long>(L, 1);
     ctx->eventsRead = 0;

@@ -372,249 +372,17 @@ __global__ void k_permute(const int *__restrict__ perm, int n, const PRec<LP> *_
                           PRec<LP> *__restrict__ recNew, const uint8_t *__restrict__ typeOld,
                           uint8_t *__restrict__ typeNew, const int *__restrict__ origOld,
                           int *__restrict__ origNew, const int *__restrict__ cellOld,
-                          int *__restrict__ cellNew, int *__restrict__ slotOf) {
+                          int *__restrict__ cellNew, int *__restrict__ slotOf, int *__restrict__ newSlot) {
     int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
     int o = perm[k];
+    newSlot[o] = k;
     store_rec(recNew + k, load_rec(recOld + o));
     typeNew[k] = typeOld[o];
     int g = origOld[o];
     origNew[k] = g;
     cellNew[k] = cellOld[o];
     slotOf[g] = k;
-}
-
-// ------------------------------------------------------------------ contacts
-
-// Walk of NeighbourGrid::iteratePossibleNeighbours (PLiB/NeighbourGrid.h:87-105) with
-// the filter of NeighAccel::iterateBlocks (PLiB/Accel/NeighAccel.h:98-137). FILL=false
-// counts, FILL=true writes the row.
-template <class LP, bool FILL>
-__device__ __forceinline__ int walk_cells(const PRec<LP> *__restrict__ rec, int i, int colour,
-                                          const GridInfo &g, const int *__restrict__ cellStart,
-                                          const int *__restrict__ cellCount, double interactDist,
-                                          int32_t *__restrict__ row, long long rowBase) {
-    const double xc = rec[i].x, yc = rec[i].y, zc = rec[i].z;
-    const LP ri = rec[i].r;
-    int count = 0;
-    for (int k = 0; k < 27; ++k) {
-        int target = (int)((long long)colour + g.off[k]);
-        if (target < 0 || (long long)target >= g.total) continue;
-        int cnt = cellCount[target];
-        if (cnt == 0) continue;
-        int start = cellStart[target];
-        for (int j = start; j < start + cnt; ++j) {
-            if (j == i) continue;
-            const PRec<LP> *q = rec + j;
-            LP xDist = (LP)(xc - q->x);
-            LP xDist2 = xDist * xDist;
-            LP yDist = (LP)(yc - q->y);
-            LP yDist2 = yDist * yDist;
-            LP zDist = (LP)(zc - q->z);
-            LP zDist2 = zDist * zDist;
-            LP particleDistance2 = xDist2 + yDist2 + zDist2;
-            LP radSum = ri + q->r;
-            // candidates farther than the interaction distance by a relative 1e-5 (far above
-            // the rounding of the square root and the subtraction below) fail the test
-            // whatever the rounding: skip the IEEE square root for them
-            const double reach = interactDist + (double)radSum;
-            if ((double)particleDistance2 > reach * reach * (1.0 + 1e-5) && reach > 0.0) continue;
-            LP particleDistance = lsqrt(particleDistance2);
-            LP dist = particleDistance - radSum;
-            if ((double)dist < interactDist) {
-                if (FILL) row[rowBase + (long long)count * kWarp] = j;
-                ++count;
-            }
-        }
-    }
-    return count;
-}
-
-template <class LP>
-__global__ void k_nbr_count(const PRec<LP> *__restrict__ rec, int n, const int *__restrict__ cellOf,
-                            GridInfo g, const int *__restrict__ cellStart,
-                            const int *__restrict__ cellCount, double interactDist,
-                            uint32_t *__restrict__ counts, int *__restrict__ blockWidth,
-                            int *errorFlag) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    int c = 0;
-    // a failed check earlier in the rebuild (a particle outside the grid, a cell too crowded
-    // to sort) ends the rebuild at the next host check: skip the walk, whose cost grows with
-    // the square of a crowded cell's population
-    const bool failed = *reinterpret_cast<volatile int *>(errorFlag) != 0;
-    if (i < n) {
-        if (!failed)
-            c = walk_cells<LP, false>(rec, i, cellOf[i], g, cellStart, cellCount, interactDist, nullptr, 0);
-        if (c > 0xffff) {
-            set_error(errorFlag, 2);
-            c = 0xffff;
-        }
-        counts[i] = (uint32_t)c;
-    }
-    int m = c;
-    for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
-    if ((threadIdx.x & 31) == 0 && (i >> 5) * kWarp < n) blockWidth[i >> 5] = m;
-}
-
-template <class LP>
-__global__ void k_nbr_fill(const PRec<LP> *__restrict__ rec, int n, const int *__restrict__ cellOf,
-                           GridInfo g, const int *__restrict__ cellStart,
-                           const int *__restrict__ cellCount, double interactDist,
-                           const long long *__restrict__ nOff, int32_t *__restrict__ nbr) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    walk_cells<LP, true>(rec, i, cellOf[i], g, cellStart, cellCount, interactDist, nbr,
-                         nOff[i >> 5] + (i & 31));
-}
-
-// Contact-list statistics of a rebuild from the per-slot counts (low 16 bits: contacts,
-// high 16 bits: link ends): out[0] total contacts, out[1] the largest contact count,
-// out[2] the largest link-end count (integer sums and maxima: order-independent).
-__global__ void k_count_stats(const uint32_t *__restrict__ counts, int n, long long *__restrict__ out) {
-    long long pairs = 0, mn = 0, ml = 0;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const uint32_t c = counts[i];
-        const long long a = c & 0xffffu, e = c >> 16;
-        pairs += a;
-        mn = a > mn ? a : mn;
-        ml = e > ml ? e : ml;
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-        pairs += __shfl_xor_sync(0xffffffffu, pairs, o);
-        const long long a = __shfl_xor_sync(0xffffffffu, mn, o), e = __shfl_xor_sync(0xffffffffu, ml, o);
-        mn = a > mn ? a : mn;
-        ml = e > ml ? e : ml;
-    }
-    if ((threadIdx.x & 31) == 0) {
-        atomicAdd(reinterpret_cast<unsigned long long *>(out), (unsigned long long)pairs);
-        atomicMax(out + 1, mn);
-        atomicMax(out + 2, ml);
-    }
-}
-
-// ------------------------------------------------------------------ link ends
-
-__global__ void k_side_count(const int *__restrict__ orig, int n, const int *__restrict__ plStart,
-                             uint32_t *__restrict__ counts, int *__restrict__ blockWidth,
-                             int *errorFlag) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    int c = 0;
-    if (i < n) {
-        int o = orig[i];
-        c = plStart[o + 1] - plStart[o];
-        if (c > 0xffff) {
-            set_error(errorFlag, 3);
-            c = 0xffff;
-        }
-        counts[i] = (counts[i] & 0xffffu) | ((uint32_t)c << 16);
-    }
-    int m = c;
-    for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
-    if ((threadIdx.x & 31) == 0 && (i >> 5) * kWarp < n) blockWidth[i >> 5] = m;
-}
-
-template <class LP>
-__global__ void k_side_fill(const int *__restrict__ orig, int n, const int *__restrict__ slotOf,
-                            const int *__restrict__ plStart, const int *__restrict__ plLink,
-                            const uint8_t *__restrict__ plEnd, const int *__restrict__ linkA,
-                            const int *__restrict__ linkB, const LP *__restrict__ L0link,
-                            const int *__restrict__ sideSlotOld, SideView<LP> oldS,
-                            const long long *__restrict__ sOff, SideView<LP> newS,
-                            int *__restrict__ sideSlotNew) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    int o = orig[i];
-    int ps = plStart[o], pe = plStart[o + 1];
-    long long base = sOff[i >> 5] + (i & 31);
-    for (int k = 0; k < pe - ps; ++k) {
-        int l = plLink[ps + k];
-        int e = plEnd[ps + k];
-        int other = e ? linkA[l] : linkB[l];
-        long long dst = base + (long long)k * kWarp;
-        int src = sideSlotOld[2 * l + e];
-        newS.partner[dst] = (uint32_t)slotOf[other] | (e ? kSideIsB : 0u);
-        newS.state[dst] = oldS.state[src];
-#pragma unroll
-        for (int c = 0; c < 6; ++c) newS.ct[c][dst] = oldS.ct[c][src];
-        newS.L0[dst] = L0link[l];
-        newS.link[dst] = l;
-        sideSlotNew[2 * l + e] = (int)dst;
-    }
-}
-
-// ------------------------------------------------------------------ timestep
-
-// The first CHUNKS 16-byte chunks of a record (the fields a functor reads); the rest of
-// the returned record is left unset and must not be read.
-template <class LP, int CHUNKS>
-__device__ __forceinline__ PRec<LP> load_rec_head(const PRec<LP> *p) {
-    PRec<LP> r;
-    const int4 *src = reinterpret_cast<const int4 *>(p);
-    int4 *dst = reinterpret_cast<int4 *>(&r);
-#pragma unroll
-    for (int k = 0; k < CHUNKS; ++k) dst[k] = __ldg(src + k);
-    return r;
-}
-// chunks holding x, y, z, d[6], r
-template <class LP>
-constexpr int kContactChunks = (int)((3 * sizeof(double) + 7 * sizeof(LP) + 15) / 16);
-
-// Start the L2 fetch of everything this warp will stream: its block's contact indices and its
-// link ends' partner words, CT0..CT5, states (and initial lengths), each one contiguous run of
-// the warp-blocked layout. One bulk prefetch per array, one lane each (nothing to wait for),
-// instead of a prefetch per array and item. Runs are multiples of 32 entries from 32-entry
-// offsets: 16-byte aligned for the byte arrays too.
-__device__ __forceinline__ void bulk_prefetch_l2(const void *p, unsigned bytes) {
-    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
-}
-template <class LP>
-__device__ __forceinline__ void prefetch_block(const StepArgs<LP> &a, int w, bool lengths) {
-    const int lane = threadIdx.x & 31;
-    const long long s0 = __ldg(a.sOff + w), n0 = __ldg(a.nOff + w);
-    const unsigned ends = (unsigned)(__ldg(a.sOff + w + 1) - s0), contacts = (unsigned)(__ldg(a.nOff + w + 1) - n0);
-    const void *p = nullptr;
-    unsigned bytes = 0;
-#pragma unroll
-    for (int q = 0; q < 6; ++q)
-        if (lane == q) p = a.ct[q] + s0, bytes = ends * (unsigned)sizeof(LP);
-    if (lane == 6) p = a.sPartner + s0, bytes = ends * 4u;
-    if (lane == 7) p = a.sState + s0, bytes = ends;
-    if (lane == 8) p = a.nbr + n0, bytes = contacts * 4u;
-    if (lane == 9 && lengths) p = a.sL0 + s0, bytes = ends * (unsigned)sizeof(LP);
-    if (bytes) bulk_prefetch_l2(p, bytes);
-}
-
-// Whether a whole link between two particles a squared distance D apart (as the break functor
-// forms it) stays whole for certain: its load is below maxLoad by more than 1e-5 (1 + |maxLoad|
-// + |bendBreak| bend), far above the functor's and this test's rounding (a few 2^-23 of the same
-// sum), so the functor's root and division are left to the links near the threshold. A test
-// that is not certain (NaN, a non-positive bound) is false.
-template <class LP>
-__device__ __forceinline__ bool stays_whole(const StepArgs<LP> &a, LP D, const LP *thA, const LP *thB, LP L0) {
-    const LP ax = labs_(thA[0] - thB[0]), ay = labs_(thA[1] - thB[1]), az = labs_(thA[2] - thB[2]);
-    const LP myz = (ay < az) ? az : ay;
-    const LP bend = (ax < myz) ? myz : ax;
-    const LP t = L0 * (a.wholeLoad - a.wholeBend * bend);
-    return t > LP(0) && D < t * t;
-}
-
-// The link state of one end after the previous step's link update (a.breakPending), both ends
-// of a link deciding alike from the same records; end A appends the break event.
-template <class LP, class P>
-__device__ __forceinline__ uint8_t pending_break(const StepArgs<LP> &a, unsigned si, uint32_t pw, const P &me,
-                                                 const P &other, uint8_t st, LP L0, LP x, LP y, LP z) {
-    if (st == 0 || stays_whole<LP>(a, x * x + y * y + z * z, me.th, other.th, L0)) return st;
-    const uint8_t nst = (pw & kSideIsB) ? break_link<LP>(a.bendBreak, a.maxLoad, other, me, st, L0)
-                                        : break_link<LP>(a.bendBreak, a.maxLoad, me, other, st, L0);
-    if (nst != st) {
-        a.sState[si] = nst;
-        a.linkState[__ldg(a.sLink + si)] = nst;  // both sides write the same value
-        if (nst == 0 && !(pw & kSideIsB)) {
-            unsigned long long slot = atomicAdd(a.eventCount, 1ull);
-            if ((long long)slot < a.eventCap) a.events[slot] = make_int2(__ldg(a.sLink + si), (int)a.breakStep);
-        }
-    }
-    return nst;
 }
 
 // ---- the gather layout (internal.h) ----
@@ -713,6 +481,300 @@ __device__ __forceinline__ PRec<LP> gather_rec(const int4 *base, int slot) {
     for (int q = 0; q < 3; ++q) r.th[q] = b.th[q];
     if constexpr (sizeof(PRec<LP>) == 128) r.pad[0] = r.pad[1] = r.pad[2] = 0.0;
     return r;
+}
+
+// ------------------------------------------------------------------ contacts
+
+// Walk of NeighbourGrid::iteratePossibleNeighbours (PLiB/NeighbourGrid.h:87-105) with
+// the filter of NeighAccel::iterateBlocks (PLiB/Accel/NeighAccel.h:98-137). FILL=false
+// counts, FILL=true writes the row. The 27 cells are nine runs of three consecutive colours, and
+// particles are stored by colour: each run is one range of slots, walked in the reference's
+// order. Candidates come from the gather layout (positions and radii of consecutive slots in
+// consecutive chunks).
+template <class LP>
+__device__ __forceinline__ void load_place(const int4 *base, int slot, double &x, double &y, double &z, LP &r) {
+    const int4 *p = base + gather_index<LP>(slot);
+    const double2 c0 = __ldg(reinterpret_cast<const double2 *>(p));
+    x = c0.x;
+    y = c0.y;
+    z = __ldg(reinterpret_cast<const double *>(p + 32));
+    if constexpr (sizeof(LP) == 4)
+        r = __ldg(reinterpret_cast<const float *>(p + 96));
+    else
+        r = __ldg(reinterpret_cast<const double *>(p + 128) + 1);
+}
+template <class LP, bool FILL>
+__device__ __forceinline__ int walk_cells(const int4 *__restrict__ gather, int i, int colour,
+                                          const GridInfo &g, const int *__restrict__ cellStart,
+                                          const int *__restrict__ cellCount, double interactDist,
+                                          int32_t *__restrict__ row, long long rowBase) {
+    double xc, yc, zc;
+    LP ri;
+    load_place<LP>(gather, i, xc, yc, zc, ri);
+    int count = 0;
+    // the ends of the nine ranges first, so that their loads overlap
+    int from[9], to[9];
+#pragma unroll
+    for (int k = 0; k < 9; ++k) {
+        const long long c0 = (long long)colour + g.off[3 * k], c1 = c0 + 2;
+        from[k] = to[k] = 0;
+        if (c1 >= 0 && c0 < g.total) {
+            from[k] = __ldg(cellStart + (c0 < 0 ? 0 : c0));
+            const long long e = c1 >= g.total ? g.total - 1 : c1;
+            to[k] = __ldg(cellStart + e) + __ldg(cellCount + e);
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < 9; ++k) {
+        for (int j = from[k]; j < to[k]; ++j) {
+            if (j == i) continue;
+            double xq, yq, zq;
+            LP rq;
+            load_place<LP>(gather, j, xq, yq, zq, rq);
+            LP xDist = (LP)(xc - xq);
+            LP xDist2 = xDist * xDist;
+            LP yDist = (LP)(yc - yq);
+            LP yDist2 = yDist * yDist;
+            LP zDist = (LP)(zc - zq);
+            LP zDist2 = zDist * zDist;
+            LP particleDistance2 = xDist2 + yDist2 + zDist2;
+            LP radSum = ri + rq;
+            // candidates farther than the interaction distance by a relative 1e-5 (far above
+            // the rounding of this bound, of the square root and of the subtraction below) fail
+            // the test whatever the rounding: skip the IEEE square root for them
+            const LP reach = (LP)interactDist + radSum;
+            if (particleDistance2 > reach * reach * LP(1.00002) && reach > LP(0)) continue;
+            LP particleDistance = lsqrt(particleDistance2);
+            LP dist = particleDistance - radSum;
+            if ((double)dist < interactDist) {
+                if (FILL) row[rowBase + (long long)count * kWarp] = j;
+                ++count;
+            }
+        }
+    }
+    return count;
+}
+
+template <class LP>
+__global__ void __launch_bounds__(128) k_nbr_count(const int4 *__restrict__ rec, int n, const int *__restrict__ cellOf,
+                            GridInfo g, const int *__restrict__ cellStart,
+                            const int *__restrict__ cellCount, double interactDist,
+                            uint32_t *__restrict__ counts, int *__restrict__ blockWidth,
+                            int *errorFlag) {
+    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    int c = 0;
+    // a failed check earlier in the rebuild (a particle outside the grid, a cell too crowded
+    // to sort) ends the rebuild at the next host check: skip the walk, whose cost grows with
+    // the square of a crowded cell's population
+    const bool failed = *reinterpret_cast<volatile int *>(errorFlag) != 0;
+    if (i < n) {
+        if (!failed)
+            c = walk_cells<LP, false>(rec, i, cellOf[i], g, cellStart, cellCount, interactDist, nullptr, 0);
+        if (c > 0xffff) {
+            set_error(errorFlag, 2);
+            c = 0xffff;
+        }
+        counts[i] = (uint32_t)c;
+    }
+    int m = c;
+    for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if ((threadIdx.x & 31) == 0 && (i >> 5) * kWarp < n) blockWidth[i >> 5] = m;
+}
+
+template <class LP>
+__global__ void __launch_bounds__(128) k_nbr_fill(const int4 *__restrict__ rec, int n, const int *__restrict__ cellOf,
+                           GridInfo g, const int *__restrict__ cellStart,
+                           const int *__restrict__ cellCount, double interactDist,
+                           const long long *__restrict__ nOff, int32_t *__restrict__ nbr) {
+    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    walk_cells<LP, true>(rec, i, cellOf[i], g, cellStart, cellCount, interactDist, nbr,
+                         nOff[i >> 5] + (i & 31));
+}
+
+// Contact-list statistics of a rebuild from the per-slot counts (low 16 bits: contacts,
+// high 16 bits: link ends): out[0] total contacts, out[1] the largest contact count,
+// out[2] the largest link-end count (integer sums and maxima: order-independent).
+__global__ void k_count_stats(const uint32_t *__restrict__ counts, int n, long long *__restrict__ out) {
+    long long pairs = 0, mn = 0, ml = 0;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const uint32_t c = counts[i];
+        const long long a = c & 0xffffu, e = c >> 16;
+        pairs += a;
+        mn = a > mn ? a : mn;
+        ml = e > ml ? e : ml;
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+        pairs += __shfl_xor_sync(0xffffffffu, pairs, o);
+        const long long a = __shfl_xor_sync(0xffffffffu, mn, o), e = __shfl_xor_sync(0xffffffffu, ml, o);
+        mn = a > mn ? a : mn;
+        ml = e > ml ? e : ml;
+    }
+    if ((threadIdx.x & 31) == 0) {
+        atomicAdd(reinterpret_cast<unsigned long long *>(out), (unsigned long long)pairs);
+        atomicMax(out + 1, mn);
+        atomicMax(out + 2, ml);
+    }
+}
+
+// ------------------------------------------------------------------ link ends
+
+__global__ void k_side_count(const int *__restrict__ orig, int n, const int *__restrict__ plStart,
+                             uint32_t *__restrict__ counts, int *__restrict__ blockWidth,
+                             int *errorFlag) {
+    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    int c = 0;
+    if (i < n) {
+        int o = orig[i];
+        c = plStart[o + 1] - plStart[o];
+        if (c > 0xffff) {
+            set_error(errorFlag, 3);
+            c = 0xffff;
+        }
+        counts[i] = (counts[i] & 0xffffu) | ((uint32_t)c << 16);
+    }
+    int m = c;
+    for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if ((threadIdx.x & 31) == 0 && (i >> 5) * kWarp < n) blockWidth[i >> 5] = m;
+}
+
+template <class LP>
+__global__ void k_side_fill(const int *__restrict__ orig, int n, const int *__restrict__ slotOf,
+                            const int *__restrict__ plStart, const int *__restrict__ plLink,
+                            const uint8_t *__restrict__ plEnd, const int *__restrict__ linkA,
+                            const int *__restrict__ linkB, const LP *__restrict__ L0link,
+                            const int *__restrict__ sideSlotOld, SideView<LP> oldS,
+                            const long long *__restrict__ sOff, SideView<LP> newS,
+                            int *__restrict__ sideSlotNew) {
+    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    int o = orig[i];
+    int ps = plStart[o], pe = plStart[o + 1];
+    long long base = sOff[i >> 5] + (i & 31);
+    for (int k = 0; k < pe - ps; ++k) {
+        int l = plLink[ps + k];
+        int e = plEnd[ps + k];
+        int other = e ? linkA[l] : linkB[l];
+        long long dst = base + (long long)k * kWarp;
+        int src = sideSlotOld[2 * l + e];
+        newS.partner[dst] = (uint32_t)slotOf[other] | (e ? kSideIsB : 0u);
+        newS.state[dst] = oldS.state[src];
+#pragma unroll
+        for (int c = 0; c < 6; ++c) newS.ct[c][dst] = oldS.ct[c][src];
+        newS.L0[dst] = L0link[l];
+        newS.link[dst] = l;
+        sideSlotNew[2 * l + e] = (int)dst;
+    }
+}
+
+// The link ends moved from one slot layout to the next: end k of a slot comes from end k of the
+// slot its particle had (both in ascending link index), so every array is read in runs of a
+// block's entries, and only the partner's new slot (of a nearby particle) and the link's record
+// of where its end lies are looked up. Through the links (k_side_fill, which the first layout
+// after set_links still takes) each end costs four scattered 32-byte sectors more: 344 us
+// against 167 us on the 0.8M slab (mixed).
+template <class LP>
+__global__ void __launch_bounds__(256) k_side_move(const int *__restrict__ perm, int n, const int *__restrict__ newSlot,
+                            const uint32_t *__restrict__ counts, const long long *__restrict__ sOffOld,
+                            SideView<LP> oldS, const long long *__restrict__ sOff, SideView<LP> newS,
+                            int *__restrict__ sideSlotNew) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const int o = __ldg(perm + i);
+    const int ns = (int)(__ldg(counts + i) >> 16);
+    unsigned src = (unsigned)(__ldg(sOffOld + (o >> 5)) + (o & 31));
+    unsigned dst = (unsigned)(__ldg(sOff + (i >> 5)) + (i & 31));
+    for (int k = 0; k < ns; ++k, src += kWarp, dst += kWarp) {
+        const uint32_t pw = oldS.partner[src];
+        const int l = oldS.link[src];
+        LP ct[6];
+#pragma unroll
+        for (int c = 0; c < 6; ++c) ct[c] = oldS.ct[c][src];
+        const LP L0 = oldS.L0[src];
+        const uint8_t st = oldS.state[src];
+        newS.partner[dst] = (uint32_t)__ldg(newSlot + (pw & kSlotMask)) | (pw & kSideIsB);
+        newS.state[dst] = st;
+#pragma unroll
+        for (int c = 0; c < 6; ++c) newS.ct[c][dst] = ct[c];
+        newS.L0[dst] = L0;
+        newS.link[dst] = l;
+        sideSlotNew[2 * l + ((pw & kSideIsB) ? 1 : 0)] = (int)dst;
+    }
+}
+
+// ------------------------------------------------------------------ timestep
+
+// The first CHUNKS 16-byte chunks of a record (the fields a functor reads); the rest of
+// the returned record is left unset and must not be read.
+template <class LP, int CHUNKS>
+__device__ __forceinline__ PRec<LP> load_rec_head(const PRec<LP> *p) {
+    PRec<LP> r;
+    const int4 *src = reinterpret_cast<const int4 *>(p);
+    int4 *dst = reinterpret_cast<int4 *>(&r);
+#pragma unroll
+    for (int k = 0; k < CHUNKS; ++k) dst[k] = __ldg(src + k);
+    return r;
+}
+// chunks holding x, y, z, d[6], r
+template <class LP>
+constexpr int kContactChunks = (int)((3 * sizeof(double) + 7 * sizeof(LP) + 15) / 16);
+
+// Start the L2 fetch of everything this warp will stream: its block's contact indices and its
+// link ends' partner words, CT0..CT5, states (and initial lengths), each one contiguous run of
+// the warp-blocked layout. One bulk prefetch per array, one lane each (nothing to wait for),
+// instead of a prefetch per array and item. Runs are multiples of 32 entries from 32-entry
+// offsets: 16-byte aligned for the byte arrays too.
+__device__ __forceinline__ void bulk_prefetch_l2(const void *p, unsigned bytes) {
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
+}
+template <class LP>
+__device__ __forceinline__ void prefetch_block(const StepArgs<LP> &a, int w, bool lengths) {
+    const int lane = threadIdx.x & 31;
+    const long long s0 = __ldg(a.sOff + w), n0 = __ldg(a.nOff + w);
+    const unsigned ends = (unsigned)(__ldg(a.sOff + w + 1) - s0), contacts = (unsigned)(__ldg(a.nOff + w + 1) - n0);
+    const void *p = nullptr;
+    unsigned bytes = 0;
+#pragma unroll
+    for (int q = 0; q < 6; ++q)
+        if (lane == q) p = a.ct[q] + s0, bytes = ends * (unsigned)sizeof(LP);
+    if (lane == 6) p = a.sPartner + s0, bytes = ends * 4u;
+    if (lane == 7) p = a.sState + s0, bytes = ends;
+    if (lane == 8) p = a.nbr + n0, bytes = contacts * 4u;
+    if (lane == 9 && lengths) p = a.sL0 + s0, bytes = ends * (unsigned)sizeof(LP);
+    if (bytes) bulk_prefetch_l2(p, bytes);
+}
+
+// Whether a whole link between two particles a squared distance D apart (as the break functor
+// forms it) stays whole for certain: its load is below maxLoad by more than 1e-5 (1 + |maxLoad|
+// + |bendBreak| bend), far above the functor's and this test's rounding (a few 2^-23 of the same
+// sum), so the functor's root and division are left to the links near the threshold. A test
+// that is not certain (NaN, a non-positive bound) is false.
+template <class LP>
+__device__ __forceinline__ bool stays_whole(const StepArgs<LP> &a, LP D, const LP *thA, const LP *thB, LP L0) {
+    const LP ax = labs_(thA[0] - thB[0]), ay = labs_(thA[1] - thB[1]), az = labs_(thA[2] - thB[2]);
+    const LP myz = (ay < az) ? az : ay;
+    const LP bend = (ax < myz) ? myz : ax;
+    const LP t = L0 * (a.wholeLoad - a.wholeBend * bend);
+    return t > LP(0) && D < t * t;
+}
+
+// The link state of one end after the previous step's link update (a.breakPending), both ends
+// of a link deciding alike from the same records; end A appends the break event.
+template <class LP, class P>
+__device__ __forceinline__ uint8_t pending_break(const StepArgs<LP> &a, unsigned si, uint32_t pw, const P &me,
+                                                 const P &other, uint8_t st, LP L0, LP x, LP y, LP z) {
+    if (st == 0 || stays_whole<LP>(a, x * x + y * y + z * z, me.th, other.th, L0)) return st;
+    const uint8_t nst = (pw & kSideIsB) ? break_link<LP>(a.bendBreak, a.maxLoad, other, me, st, L0)
+                                        : break_link<LP>(a.bendBreak, a.maxLoad, me, other, st, L0);
+    if (nst != st) {
+        a.sState[si] = nst;
+        a.linkState[__ldg(a.sLink + si)] = nst;  // both sides write the same value
+        if (nst == 0 && !(pw & kSideIsB)) {
+            unsigned long long slot = atomicAdd(a.eventCount, 1ull);
+            if ((long long)slot < a.eventCap) a.events[slot] = make_int2(__ldg(a.sLink + si), (int)a.breakStep);
+        }
+    }
+    return nst;
 }
 
 // The force pass: one particle per thread, contacts, then link ends, forces to a.force
@@ -1595,13 +1657,13 @@ int launch_sort_cells(const int *cellStart, const int *cellCount, long long tota
 template <class LP>
 void launch_permute(const int *perm, int n, const PRec<LP> *recOld, PRec<LP> *recNew,
                     const uint8_t *typeOld, uint8_t *typeNew, const int *origOld, int *origNew,
-                    const int *cellOld, int *cellNew, int *slotOf, cudaStream_t s) {
+                    const int *cellOld, int *cellNew, int *slotOf, int *newSlot, cudaStream_t s) {
     k_permute<LP><<<nblk(n, 256), 256, 0, s>>>(perm, n, recOld, recNew, typeOld, typeNew, origOld,
-                                               origNew, cellOld, cellNew, slotOf);
+                                               origNew, cellOld, cellNew, slotOf, newSlot);
 }
 
 template <class LP>
-void launch_nbr_count(const PRec<LP> *rec, int n, const int *cellOf, const GridInfo &g,
+void launch_nbr_count(const int4 *rec, int n, const int *cellOf, const GridInfo &g,
                       const int *cellStart, const int *cellCount, double interactDist,
                       uint32_t *counts, int *blockWidth, int *errorFlag, cudaStream_t s) {
     k_nbr_count<LP><<<nblk(n, 128), 128, 0, s>>>(rec, n, cellOf, g, cellStart, cellCount,
@@ -1609,7 +1671,7 @@ void launch_nbr_count(const PRec<LP> *rec, int n, const int *cellOf, const GridI
 }
 
 template <class LP>
-void launch_nbr_fill(const PRec<LP> *rec, int n, const int *cellOf, const GridInfo &g,
+void launch_nbr_fill(const int4 *rec, int n, const int *cellOf, const GridInfo &g,
                      const int *cellStart, const int *cellCount, double interactDist,
                      const long long *nOff, int32_t *nbr, cudaStream_t s) {
     k_nbr_fill<LP><<<nblk(n, 128), 128, 0, s>>>(rec, n, cellOf, g, cellStart, cellCount,
@@ -1677,6 +1739,13 @@ void launch_step(const Consts<LP> &c, const StepArgs<LP> &a0, int maxContacts, i
         k_step<LP, kCapBlocks<LP>><<<nb, kStepThreads, 0, s>>>(c, a);
     else
         k_step<LP, kThreadBlocks<LP>><<<nb, kStepThreads, 0, s>>>(c, a);
+}
+
+template <class LP>
+void launch_side_move(const int *perm, int n, const int *newSlot, const uint32_t *counts, const long long *sOffOld,
+                      const SideView<LP> &oldS, const long long *sOff, const SideView<LP> &newS, int *sideSlotNew,
+                      cudaStream_t s) {
+    k_side_move<LP><<<nblk(n, 256), 256, 0, s>>>(perm, n, newSlot, counts, sOffOld, oldS, sOff, newS, sideSlotNew);
 }
 
 template <class LP, bool AHEAD, int MINB>
@@ -1918,11 +1987,11 @@ void launch_max_diff(const PRec<LP> *rec, int n, unsigned long long *out, int nb
                                    cudaStream_t);                                                  \
     template void launch_permute<LP>(const int *, int, const PRec<LP> *, PRec<LP> *,               \
                                      const uint8_t *, uint8_t *, const int *, int *, const int *,  \
-                                     int *, int *, cudaStream_t);                                  \
-    template void launch_nbr_count<LP>(const PRec<LP> *, int, const int *, const GridInfo &,       \
+                                     int *, int *, int *, cudaStream_t);                                  \
+    template void launch_nbr_count<LP>(const int4 *, int, const int *, const GridInfo &,       \
                                        const int *, const int *, double, uint32_t *, int *, int *, \
                                        cudaStream_t);                                              \
-    template void launch_nbr_fill<LP>(const PRec<LP> *, int, const int *, const GridInfo &,        \
+    template void launch_nbr_fill<LP>(const int4 *, int, const int *, const GridInfo &,        \
                                       const int *, const int *, double, const long long *,         \
                                       int32_t *, cudaStream_t);                                    \
     template void launch_side_fill<LP>(const int *, int, const int *, const int *, const int *,    \
@@ -1931,6 +2000,9 @@ void launch_max_diff(const PRec<LP> *rec, int n, unsigned long long *out, int nb
                                        const SideView<LP> &, int *, cudaStream_t);                 \
     template void launch_step<LP>(const Consts<LP> &, const StepArgs<LP> &, int, int, int, int,     \
                                   cudaStream_t);                                                   \
+    template void launch_side_move<LP>(const int *, int, const int *, const uint32_t *, const long long *, \
+                                       const SideView<LP> &, const long long *, const SideView<LP> &, int *, \
+                                       cudaStream_t);                                              \
     template void launch_force<LP>(const Consts<LP> &, const StepArgs<LP> &, int, cudaStream_t);           \
     template void launch_to_gather<LP>(const PRec<LP> *, int, int4 *, cudaStream_t);               \
     template void launch_from_gather<LP>(const int4 *, int, PRec<LP> *, cudaStream_t);             \

@@ -114,13 +114,14 @@ int launch_sort_cells(const int *cellStart, const int *cellCount, long long tota
 template <class LP>
 void launch_permute(const int *perm, int n, const PRec<LP> *recOld, PRec<LP> *recNew,
                     const uint8_t *typeOld, uint8_t *typeNew, const int *origOld, int *origNew,
-                    const int *cellOld, int *cellNew, int *slotOf, cudaStream_t s);
+                    const int *cellOld, int *cellNew, int *slotOf, int *newSlot, cudaStream_t s);
+// (gather: the records in the gather layout)
 template <class LP>
-void launch_nbr_count(const PRec<LP> *rec, int n, const int *cellOf, const GridInfo &g,
+void launch_nbr_count(const int4 *gather, int n, const int *cellOf, const GridInfo &g,
                       const int *cellStart, const int *cellCount, double interactDist,
                       uint32_t *counts, int *blockWidth, int *errorFlag, cudaStream_t s);
 template <class LP>
-void launch_nbr_fill(const PRec<LP> *rec, int n, const int *cellOf, const GridInfo &g,
+void launch_nbr_fill(const int4 *gather, int n, const int *cellOf, const GridInfo &g,
                      const int *cellStart, const int *cellCount, double interactDist,
                      const long long *nOff, int32_t *nbr, cudaStream_t s);
 // out[0..2] = total contacts, largest contact count, largest link-end count of the
@@ -133,6 +134,12 @@ void launch_side_fill(const int *orig, int n, const int *slotOf, const int *plSt
                       const int *plLink, const uint8_t *plEnd, const int *linkA, const int *linkB,
                       const LP *L0link, const int *sideSlotOld, const SideView<LP> &oldS,
                       const long long *sOff, const SideView<LP> &newS, int *sideSlotNew,
+                      cudaStream_t s);
+// the link ends moved from the layout sOffOld to sOff: particle of slot i was at slot perm[i],
+// newSlot is the inverse
+template <class LP>
+void launch_side_move(const int *perm, int n, const int *newSlot, const uint32_t *counts, const long long *sOffOld,
+                      const SideView<LP> &oldS, const long long *sOff, const SideView<LP> &newS, int *sideSlotNew,
                       cudaStream_t s);
 // One fused timestep (previous link update, forces, integrate, record swap) for rows of at
 // most maxContacts contacts and maxEnds link ends, by the kernel `kernel`

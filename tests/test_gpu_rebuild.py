@@ -1,0 +1,52 @@
+"""Rebuilds that move the link ends from one slot layout to the next: after particles have
+changed cells, at sizes around the blocks of 32, and after a rebuild that failed midway."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+from hidem_b200 import abi, workloads
+from hidem_b200.hidemlib import HiDEMLib
+from oracle import oracle
+from test_gpu_parity import L_OUT, P_OUT, PRECS, assert_same, gpu_run
+
+pytestmark = pytest.mark.gpu
+
+
+# an unsupported, spinning-up block whose particles change cells (and slots) between rebuilds
+@pytest.mark.parametrize("precision", PRECS)
+@pytest.mark.parametrize("cells", [(1, 1, 1), (2, 2, 2), (3, 3, 1), (5, 4, 3)])
+def test_moving_particles(gpu, precision, cells):
+    P, p, l = workloads.ice_block(cells=cells, precision=precision, seed=6, fixed_bottom=False, g=-2e6,
+                                  gridRegenInterval=3)
+    ref = oracle.port().run(P, p, l, 25)
+    for kernel in (abi.STEP_KERNEL_TWO_PASS, abi.STEP_KERNEL_ITEMS):
+        assert_same(gpu_run(P, p, l, 25, kernel=kernel), ref[0], ref[1], ref[3])
+
+
+@pytest.mark.parametrize("precision", PRECS)
+def test_rebuild_after_a_failed_one(gpu, precision):
+    P, p, l = workloads.ice_block(cells=(12, 12, 12), precision=precision, seed=5, g=-1e5)
+    out = []
+    for fail in (True, False):
+        lib = HiDEMLib(P)
+        lib.set_particles(p)
+        lib.set_links(l)
+        lib.step(8)
+        if fail:
+            wide = abi.HidemParams.from_buffer_copy(P)
+            wide.searchDistanceScale = 20.0  # every particle in one cell: refused after the sort
+            lib.set_params(wide)
+            with pytest.raises(abi.HidemError) as e:
+                lib.regenerate()
+            assert e.value.status == abi.HIDEM_ERR_CAPACITY
+            lib.set_params(P)
+        lib.regenerate()
+        lib.step(8)
+        out.append((lib.get_particles(), lib.get_links(), lib.get_neighbours()[0]))
+        lib.close()
+    for k in P_OUT:
+        assert np.array_equal(out[0][0][k], out[1][0][k]), k
+    for k in L_OUT:
+        assert np.array_equal(out[0][1][k], out[1][1][k]), k
+    assert np.array_equal(out[0][2], out[1][2])
