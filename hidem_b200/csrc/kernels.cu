@@ -1430,7 +1430,9 @@ __global__ void __launch_bounds__(kStepThreads, kForceBlocks<LP>)
 }
 
 // The integrate step on the gather layout, in place; the records too where rec is not null.
-// Streaming: 64 + 24 B read and 64 B (128 B with the records) written per particle (mixed).
+// Streaming: 64 + 24 B read and 64 B (128 B with the records) written per particle (mixed); what
+// it takes is warps enough to keep the loads in flight, so the registers are capped (a few bytes
+// spill): 5.7M slab 136 us mixed, 257 us FP64, 153 and 439 us from and to the records uncapped.
 template <class LP>
 __device__ __forceinline__ void integrate_gather(const Consts<LP> &c, int4 *g, PRec<LP> *rec, const uint8_t *type,
                                                  const LP *force, int n, int i, bool reduce,
@@ -1461,7 +1463,7 @@ __device__ __forceinline__ void integrate_gather(const Consts<LP> &c, int4 *g, P
 }
 
 template <class LP>
-__global__ void __launch_bounds__(kStepThreads)
+__global__ void __launch_bounds__(kStepThreads, sizeof(LP) == 8 ? 7 : 8)
     k_integrate_gather(const Consts<LP> c, int4 *g, PRec<LP> *rec, const uint8_t *__restrict__ type,
                        const LP *__restrict__ force, int n, bool reduce, unsigned long long *diffMax) {
     dependent_start();
@@ -1482,6 +1484,34 @@ __global__ void __launch_bounds__(kStepThreads)
                          e.reduceEvery10 && (step + 1) % 10 == 0, e.a.diffMax);
 }
 
+// Position and rotations alone (what the break functor reads).
+template <class LP>
+struct Pose {
+    double x, y, z;
+    LP th[3];
+};
+__device__ __forceinline__ void load_pose(Pose<float> &o, const int4 *base, int slot) {
+    const int4 *p = base + gather_index<float>(slot);
+    const double2 c0 = __ldg(reinterpret_cast<const double2 *>(p));
+    const float4 c3 = __ldg(reinterpret_cast<const float4 *>(p + 96));
+    o.x = c0.x;
+    o.y = c0.y;
+    o.z = __ldg(reinterpret_cast<const double *>(p + 32));
+    o.th[0] = c3.y;
+    o.th[1] = c3.z;
+    o.th[2] = c3.w;
+}
+__device__ __forceinline__ void load_pose(Pose<double> &o, const int4 *base, int slot) {
+    const double2 *p = reinterpret_cast<const double2 *>(base + gather_index<double>(slot));
+    const double2 c0 = __ldg(p), c5 = __ldg(p + 160);
+    o.x = c0.x;
+    o.y = c0.y;
+    o.z = __ldg(reinterpret_cast<const double *>(p + 32));
+    o.th[0] = c5.x;
+    o.th[1] = c5.y;
+    o.th[2] = __ldg(reinterpret_cast<const double *>(p + 192));
+}
+
 // The break pass of the batch: one thread per link over a grid of its own (the links of
 // entry e take CTAs [linkFirst[e], linkFirst[e + 1]), linkEntry maps a CTA to its entry),
 // so that each thread's two gathers are in flight beside every other thread's, as in the
@@ -1500,9 +1530,9 @@ __global__ void __launch_bounds__(kStepThreads)
         const uint8_t st = e.a.linkState[l];
         if (st != 0) {
             const int4 *g = reinterpret_cast<const int4 *>(e.rec[e.cur0 ^ 1]);
-            Body<LP> pa, pb;
-            load_body<true, true>(pa, g, __ldg(e.slotA + l));
-            load_body<true, true>(pb, g, __ldg(e.slotB + l));
+            Pose<LP> pa, pb;
+            load_pose(pa, g, __ldg(e.slotA + l));
+            load_pose(pb, g, __ldg(e.slotB + l));
             const LP L0 = __ldg(e.L0link + l);
             const LP x = (LP)(pa.x - pb.x), y = (LP)(pa.y - pb.y), z = (LP)(pa.z - pb.z);
             if (stays_whole<LP>(e.a, x * x + y * y + z * z, pa.th, pb.th, L0)) return;
@@ -2138,23 +2168,41 @@ __global__ void k_link_fill(const int *__restrict__ A, const int *__restrict__ B
     plEnd[b] = 1;
 }
 
-// a particle's ends in ascending link index (LinkAccelSide::generateLinks, LinkAccelSide.h:118-131)
-__global__ void k_link_sort_ends(const int *__restrict__ start, int n, int *__restrict__ plLink,
-                                 uint8_t *__restrict__ plEnd) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const int s = start[i], e = start[i + 1];
-    for (int a = s + 1; a < e; ++a) {
-        const int v = plLink[a];
-        const uint8_t ve = plEnd[a];
-        int b = a - 1;
-        while (b >= s && plLink[b] > v) {
-            plLink[b + 1] = plLink[b];
-            plEnd[b + 1] = plEnd[b];
-            --b;
-        }
-        plLink[b + 1] = v;
-        plEnd[b + 1] = ve;
+// A particle's ends in ascending link index (LinkAccelSide::generateLinks, LinkAccelSide.h:118-131).
+// Sixteen lanes per particle: each holds one end, whose place is the number of smaller link
+// indices among the others (indices of one particle's links are distinct); particles of more
+// than sixteen ends are sorted by insertion by one lane. 0.48 ms on the 5.7M slab; one thread per
+// particle sorting in memory took 1.47 ms.
+constexpr int kSortLanes = 16;
+__global__ void __launch_bounds__(256) k_link_sort_ends(const int *__restrict__ start, int n, int *__restrict__ plLink,
+                                                        uint8_t *__restrict__ plEnd) {
+    const int lane = threadIdx.x & (kSortLanes - 1);
+    const long long i = ((long long)blockIdx.x * blockDim.x + threadIdx.x) / kSortLanes;
+    const int s = i < n ? start[i] : 0, cnt = i < n ? start[i + 1] - s : 0;
+    if (cnt > kSortLanes) {
+        if (lane == 0)
+            for (int a = s + 1; a < s + cnt; ++a) {
+                const int v = plLink[a];
+                const uint8_t ve = plEnd[a];
+                int b = a - 1;
+                while (b >= s && plLink[b] > v) {
+                    plLink[b + 1] = plLink[b];
+                    plEnd[b + 1] = plEnd[b];
+                    --b;
+                }
+                plLink[b + 1] = v;
+                plEnd[b + 1] = ve;
+            }
+    }
+    const bool mine = cnt <= kSortLanes && lane < cnt;
+    const int v = mine ? plLink[s + lane] : 0x7fffffff;
+    const uint8_t e = mine ? plEnd[s + lane] : uint8_t(0);
+    int rank = 0;
+#pragma unroll
+    for (int k = 0; k < kSortLanes; ++k) rank += __shfl_sync(0xffffffffu, v, k, kSortLanes) < v ? 1 : 0;
+    if (mine) {
+        plLink[s + rank] = v;
+        plEnd[s + rank] = e;
     }
 }
 
@@ -2337,7 +2385,7 @@ void launch_link_lists(const int *A, const int *B, long long L, int n, int *deg,
     // start[0..n] = exclusive scan of deg[0..n] with deg[n] = 0
     launch_scan<int, int>(deg, (long long)n + 1, 1, start, sums, nullptr, st);
     if (L > 0) k_link_fill<<<nblk(L, 256), 256, 0, st>>>(A, B, L, start, cursor, plLink, plEnd);
-    k_link_sort_ends<<<nblk(n, 256), 256, 0, st>>>(start, n, plLink, plEnd);
+    k_link_sort_ends<<<nblk((long long)n * kSortLanes, 256), 256, 0, st>>>(start, n, plLink, plEnd);
 }
 void launch_side_init(const uint8_t *linkState, long long L, int *sideSlot, uint8_t *sideState,
                       cudaStream_t st) {
