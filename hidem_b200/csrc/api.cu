@@ -275,11 +275,20 @@ void dfree(T *&p) {
     p = nullptr;
 }
 
-// where the shared-root beam geometry holds (Consts::beamFastLo)
+// what follows from the functors' parameters: the products and pairs of Consts, and where the
+// shared-root beam geometry holds (beamFastLo)
 template <class LP>
-void set_beam_range(Consts<LP> &c) {
-    const double ew4 = (double)(LP)(c.E * c.W4);
-    c.beamFastLo = (ew4 >= std::ldexp(1.0, -40) && ew4 <= std::ldexp(1.0, 60))
+void set_functor_products(Consts<LP> &c) {
+    c.EW2 = c.E * c.W2;
+    c.EW4 = c.E * c.W4;
+    c.GW4 = c.G * c.W4;
+    const LP n[4] = {c.invDt, c.invDt, -c.damping, -c.dampingRotation};
+    const LP l[4] = {c.linkInvDt, c.linkInvDt, -c.linkDamping, -c.linkDampingRotation};
+    for (int k = 0; k < 4; ++k) {
+        c.neighPair[k] = n[k];
+        c.linkPair[k] = l[k];
+    }
+    c.beamFastLo = ((double)c.EW4 >= std::ldexp(1.0, -40) && (double)c.EW4 <= std::ldexp(1.0, 60))
                        ? (LP)std::ldexp(1.0, -40)
                        : std::numeric_limits<LP>::infinity();
 }
@@ -304,12 +313,12 @@ void derive(const hidem_params &P, Consts<LP> &c, double &searchDistance, double
     c.W2 = beamWidth * beamWidth;
     c.W4 = beamWidth * beamWidth * beamWidth * beamWidth;
     c.G = (LP)((double)E / 2.0);
-    set_beam_range(c);
     c.bendBreak = (LP)P.bendBreak;
     c.maxLoad = (LP)P.maxLoad;
     c.linkInvDt = c.invDt;
     c.linkDamping = c.damping;
     c.linkDampingRotation = c.dampingRotation;
+    set_functor_products(c);
     c.mainInvDt = c.invDt;
     c.dt = dt;
     c.invDt2 = (LP)(1.0 / (2.0 * (double)dt));
@@ -2579,7 +2588,7 @@ hidem_status hidem_set_functor_params(hidem_ctx *ctx, const hidem_functor_params
         c.W2 = (LP)f->link_W2;
         c.W4 = (LP)f->link_W4;
         c.G = (LP)f->link_G;
-        set_beam_range(c);
+        set_functor_products(c);
         c.bendBreak = (LP)f->break_bendBreak;
         c.maxLoad = (LP)f->break_maxLoad;
     };

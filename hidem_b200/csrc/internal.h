@@ -103,6 +103,10 @@ struct Consts {
     // least xy part of a squared link length for which the shared-root evaluation of the
     // beam's geometry holds (physics.cuh): 2^-40, infinite when E W4 is outside [2^-40, 2^60]
     LP beamFastLo;
+    // products and pairs the functors start from, formed once: E W2, E W4, G W4; (1, 1) invDt and
+    // -(damping, dampingRotation) of the contact and the beam functor
+    LP EW2, EW4, GW4;
+    alignas(16) LP neighPair[4], linkPair[4];
     // HiDEMDefLinkBreakFunc
     LP bendBreak, maxLoad;
     // integrate (mainInvDt: the sample main's invDt, used by the velocity limit)
