@@ -866,8 +866,8 @@ int fused_kernel(int k) { return k == HIDEM_STEP_KERNEL_TWO_PASS ? HIDEM_STEP_KE
 int step_kernel_now(hidem_ctx *ctx, cudaEvent_t *e0, cudaEvent_t *e1) {
     *e0 = *e1 = nullptr;
     if (ctx->stepKernel != HIDEM_STEP_KERNEL_AUTO) return ctx->stepKernel;
-    if (ctx->tunedKernel != HIDEM_STEP_KERNEL_AUTO) return ctx->tunedKernel;
     if (ctx->n > kTuneMax) return ctx->tunedKernel = HIDEM_STEP_KERNEL_TWO_PASS;
+    if (ctx->tunedKernel != HIDEM_STEP_KERNEL_AUTO) return ctx->tunedKernel;
     if (ctx->tuneStep < kNumCandidates * kTuneRounds) {
         const int k = ctx->tuneStep++;
         for (int q = 0; q < 2; ++q)
@@ -946,6 +946,9 @@ hidem_status run_steps(hidem_ctx *ctx, int nsteps) {
         }
         if (gs_decide(ctx, currDist)) {
             records_now();
+            // a rebuild may fail: the link update still owed is the previous step's
+            if (pending) TRY(link_update_now<LP>(ctx, pendingStep));
+            pending = false;
             TRY(do_rebuild(ctx));
             gathered = true;  // the rebuild walked it
         }

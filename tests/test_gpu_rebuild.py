@@ -50,3 +50,33 @@ def test_rebuild_after_a_failed_one(gpu, precision):
     for k in L_OUT:
         assert np.array_equal(out[0][1][k], out[1][1][k]), k
     assert np.array_equal(out[0][2], out[1][2])
+
+
+# a run that ends in a refused rebuild leaves the state of the steps before it, their link
+# updates included
+@pytest.mark.parametrize("precision", PRECS)
+@pytest.mark.parametrize("kernel", [abi.STEP_KERNEL_TWO_PASS, abi.STEP_KERNEL_ITEMS])
+def test_run_that_ends_in_a_refused_rebuild(gpu, precision, kernel):
+    P, p, l = workloads.ice_block(cells=(4, 4, 4), precision=precision, seed=7, g=-2e6, gridRegenInterval=8)
+    p["zDiff"][-1] = 60.0  # leaves the block: the grid of step 8 has far more cells
+    out = []
+    for steps in (16, 8):
+        lib = HiDEMLib(P)
+        lib.set_step_kernel(kernel)
+        lib.set_checks(abi.CHECK_GRID_GROWTH)
+        lib.set_particles(p)
+        lib.set_links(l)
+        if steps == 16:
+            with pytest.raises(abi.HidemError) as e:
+                lib.step(16)
+            assert e.value.status == abi.HIDEM_ERR_DEVICE
+        else:
+            lib.step(8)
+        li, st = lib.get_break_events()
+        out.append((lib.get_particles(), lib.get_links(), sorted(zip(li.tolist(), st.tolist()))))
+        lib.close()
+    for k in P_OUT:
+        assert np.array_equal(out[0][0][k], out[1][0][k], equal_nan=True), k
+    for k in L_OUT:
+        assert np.array_equal(out[0][1][k], out[1][1][k], equal_nan=True), k
+    assert out[0][2] == out[1][2] and len(out[0][2]) > 0
