@@ -1266,7 +1266,7 @@ struct hidem_surrogate {
     std::vector<bf16 *> dZ, dZT, inT;
     std::vector<float *> part, partB;
     float *partOut = nullptr;                    // chunk partials of the output layer's gradient
-    std::vector<cudaStream_t> side;              // per hidden layer, then the output layer's
+    std::vector<cudaStream_t> side;              // per hidden layer, then loss, output layer and biases
     std::vector<cudaEvent_t> evDz, evDone;
     cudaEvent_t evForward = nullptr;
     WeightViews weights{};
@@ -1499,9 +1499,9 @@ hidem_status order_after(hidem_surrogate *s, cudaStream_t from, cudaStream_t to,
 
 // Loss and all gradients into G for the rows of X0 (targets[idx[b]] or targets[b]).
 // The chain of data gradients (dZ of the last layer down to the first) is the critical path
-// and runs on the surrogate's stream; each layer's weight and bias gradients, and the loss with
-// the output layer's, need only that layer's dZ and run beside it on a stream of their own,
-// in buffers of their own. A settling batch (8,192 rows) is some forty kernels of 3-20 us that
+// and runs on the surrogate's stream; each layer's weight gradient needs only that layer's dZ and
+// runs beside it on a stream and in buffers of its own, the bias gradients and the loss with the
+// output layer's gradient on one more. A settling batch (8,192 rows) is some forty kernels of 3-20 us that
 // fill a fraction of the chip each: one after another they took 0.36 of the step's 0.48 ms.
 // The sums and their order are those of the serial chain.
 hidem_status backward(hidem_surrogate *s, int rows, const float *targets, const int *idx) {
@@ -1515,7 +1515,6 @@ hidem_status backward(hidem_surrogate *s, int rows, const float *targets, const 
     k_out_grad<<<dim3((W + 1 + 31) / 32, chunks), dim3(32, 8), 0, so>>>(s->dY, s->H[L - 1], rows, W, s->partOut);
     k_sum_out<<<sum_splits_grid((long long)kOut * (W + 1)), dim3(32, 8), 0, so>>>(s->partOut, chunks, W, s->G + s->offWo,
                                                                                s->G + s->offBo);
-    SCK(cudaEventRecord(s->evDone[L], so));
     k_out_bwd<<<dim3((unsigned)rows, (unsigned)((W + 255) / 256)), 256, 0, st>>>(s->Y, targets, idx, s->P + s->offWo,
                                                                                s->Z[L - 1], rows, W, s->dZ[L - 1]);
     SCK(cudaGetLastError());
@@ -1529,6 +1528,10 @@ hidem_status backward(hidem_surrogate *s, int rows, const float *targets, const 
         SCK(cudaStreamWaitEvent(sl, s->evForward, 0));
         k_transpose<<<dim3((K + kTrTile - 1) / kTrTile, (rows + kTrTile - 1) / kTrTile), 256, 0, sl>>>(in, rows, K, s->inT[l]);
         STRY(order_after(s, st, sl, s->evDz[l]));
+        // db_l = column sums of dZ, beside the weight gradient
+        SCK(cudaStreamWaitEvent(so, s->evDz[l], 0));
+        k_colsum_bf16<<<dim3((W + 63) / 64, chunks), dim3(32, 8), 0, so>>>(dZ, rows, W, s->partB[l]);
+        k_sum_splits<<<sum_splits_grid(W), dim3(32, 8), 0, so>>>(s->partB[l], chunks, W, s->G + s->offB[l]);
         k_transpose<<<dim3((W + kTrTile - 1) / kTrTile, (rows + kTrTile - 1) / kTrTile), 256, 0, sl>>>(dZ, rows, W, s->dZT[l]);
         if (l > 0) {
             // dZ_{l-1} = (dZ_l * W_l) . SiLU'(Z_{l-1}); B operand W_l^T is [K_l][W]
@@ -1551,11 +1554,9 @@ hidem_status backward(hidem_surrogate *s, int rows, const float *targets, const 
             n0 += bn;
         }
         k_sum_splits<<<sum_splits_grid((long long)W * K), dim3(32, 8), 0, sl>>>(s->part[l], splits, (long long)W * K, s->G + s->offW[l]);
-        // db_l = column sums of dZ
-        k_colsum_bf16<<<dim3((W + 63) / 64, chunks), dim3(32, 8), 0, sl>>>(dZ, rows, W, s->partB[l]);
-        k_sum_splits<<<sum_splits_grid(W), dim3(32, 8), 0, sl>>>(s->partB[l], chunks, W, s->G + s->offB[l]);
         SCK(cudaEventRecord(s->evDone[l], sl));
     }
+    SCK(cudaEventRecord(s->evDone[L], so));
     for (int l = 0; l <= L; ++l) SCK(cudaStreamWaitEvent(st, s->evDone[l], 0));
     SCK(cudaGetLastError());
     return HIDEM_OK;
