@@ -195,7 +195,7 @@ def measured_peak():
 def step_label(kernel: int, extra: str = "") -> str:
     """What one step launches, for roofline.kernel."""
     if kernel == KERNELS["two-pass"]:
-        return f"step passes (k_step force pass, k_integrate{extra}, k_link_break), two-pass kernel"
+        return f"step passes (k_force with the link update, k_integrate_gather{extra}), two-pass kernel"
     return f"fused step{extra}, " + KERNEL_NAMES.get(kernel, "?") + " kernel"
 
 
