@@ -451,19 +451,12 @@ hidem_status side_alloc(hidem_ctx *ctx, SideSet &s, long long cap) {
     return HIDEM_OK;
 }
 
-// frees on a stream (buffers come from the stream-ordered pool: a plain cudaFree waits for the
-// whole device first)
-template <class T>
-void dfree_on(T *&p, cudaStream_t st) {
-    if (p) cudaFreeAsync((void *)p, st);
-    p = nullptr;
-}
-void side_free(SideSet &s, cudaStream_t st) {
-    dfree_on(s.partner, st);
-    for (int k = 0; k < 6; ++k) dfree_on(s.ct[k], st);
-    dfree_on(s.state, st);
-    dfree_on(s.L0, st);
-    dfree_on(s.link, st);
+void side_free(SideSet &s) {
+    dfree(s.partner);
+    for (int k = 0; k < 6; ++k) dfree(s.ct[k]);
+    dfree(s.state);
+    dfree(s.L0);
+    dfree(s.link);
     s.cap = 0;
 }
 
@@ -1659,7 +1652,7 @@ void hidem_destroy(hidem_ctx *ctx) {
         dfree(ctx->orig[b]);
         dfree(ctx->cellOf[b]);
         dfree(ctx->sideSlot[b]);
-        side_free(ctx->side[b], ctx->stream);
+        side_free(ctx->side[b]);
     }
     dfree(ctx->slotOf);
     dfree(ctx->perm);
@@ -1857,8 +1850,8 @@ hidem_status hidem_set_links(hidem_ctx *ctx, const hidem_link_soa *l, int64_t L)
         unsigned long long h[2];
         CK(cudaMemcpyAsync(h, mins, sizeof h, cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
-        dfree_on(mins, st);
-        dfree_on(dkeys, st);
+        dfree(mins);
+        if (dkeys) dfree(dkeys);
         if (h[0] != ~0ull) bad = (long long)h[0];
         if (h[1] != ~0ull) self = (long long)h[1];
     } else {
@@ -1917,8 +1910,8 @@ hidem_status hidem_set_links(hidem_ctx *ctx, const hidem_link_soa *l, int64_t L)
     TRY(dalloc(ctx, &ctx->plLink, 2 * L));
     TRY(dalloc(ctx, &ctx->plEnd, 2 * L));
     for (int b = 0; b < 2; ++b) TRY(dalloc(ctx, &ctx->sideSlot[b], 2 * L));
-    side_free(ctx->side[0], st);
-    side_free(ctx->side[1], st);
+    side_free(ctx->side[0]);
+    side_free(ctx->side[1]);
     TRY(side_alloc(ctx, ctx->side[0], 2 * L));
     ctx->curSide = 0;
     ctx->sidesBlocked = false;
@@ -1963,10 +1956,12 @@ hidem_status hidem_set_links(hidem_ctx *ctx, const hidem_link_soa *l, int64_t L)
         if (l->globalKeys) CK(cudaMemcpyAsync(ctx->dLinkKeys, l->globalKeys, 8 * (size_t)L, cudaMemcpyDefault, st));
         else launch_iota64(ctx->dLinkKeys, L, st);
     }
-    dfree_on(deg, st);
-    dfree_on(cursor, st);
     CK(cudaStreamSynchronize(st));
     CK(cudaGetLastError());
+    // after the wait: memory freed before one is given back to the system by it where the pool
+    // holds more than it keeps, and the next context of an ensemble takes it anew (20 ms each)
+    dfree(deg);
+    dfree(cursor);
     ctx->L = L;
     ctx->haveLinks = true;
     ctx->built = false;
@@ -2272,9 +2267,9 @@ static hidem_status get_particles_t(hidem_ctx *ctx, hidem_particle_soa *out) {
 }
 
 // Side data and link state in caller order, straight into the caller's device memory or, array
-// after array, through one staging buffer.
+// after array, through one staging buffer (the caller frees it once the stream has drained).
 template <class LP>
-static hidem_status get_sides_t(hidem_ctx *ctx, hidem_link_soa *out) {
+static hidem_status get_sides_t(hidem_ctx *ctx, hidem_link_soa *out, void **staging) {
     const long long L = ctx->L;
     cudaStream_t st = ctx->stream;
     SideSet &s = ctx->side[ctx->curSide];
@@ -2306,8 +2301,8 @@ static hidem_status get_sides_t(hidem_ctx *ctx, hidem_link_soa *out) {
         ctx->launches += 1;
     }
     if (!staged) return HIDEM_OK;
-    void *stage = nullptr;
-    TRY(dalloc_bytes(ctx, &stage, sizeof(LP) * (size_t)(2 * L)));
+    TRY(dalloc_bytes(ctx, staging, sizeof(LP) * (size_t)(2 * L)));
+    void *stage = *staging;
     for (int k = 0; k < 7; ++k) {
         SideGather<LP> g = all;
         void *dst = nullptr;
@@ -2327,7 +2322,6 @@ static hidem_status get_sides_t(hidem_ctx *ctx, hidem_link_soa *out) {
         ctx->launches += 1;
         CK(cudaMemcpyAsync(dst, stage, bytes, cudaMemcpyDefault, st));
     }
-    CK(cudaFreeAsync(stage, st));
     return HIDEM_OK;
 }
 }  // extern "C++"
@@ -2351,7 +2345,8 @@ hidem_status hidem_get_links(hidem_ctx *ctx, hidem_link_soa *out) {
     const long long L = ctx->L;
     if (L == 0) return HIDEM_OK;
     cudaStream_t st = ctx->stream;
-    TRY(ctx->mixed ? get_sides_t<float>(ctx, out) : get_sides_t<double>(ctx, out));
+    void *staging = nullptr;
+    TRY(ctx->mixed ? get_sides_t<float>(ctx, out, &staging) : get_sides_t<double>(ctx, out, &staging));
     const size_t lp = ctx->lp;
     if (out->initialLen) CK(cudaMemcpyAsync(out->initialLen, ctx->L0link, lp * (size_t)L, cudaMemcpyDefault, st));
     if (out->owners) CK(cudaMemcpyAsync(out->owners, ctx->dLinkOwners, 4 * (size_t)L, cudaMemcpyDefault, st));
@@ -2360,6 +2355,7 @@ hidem_status hidem_get_links(hidem_ctx *ctx, hidem_link_soa *out) {
     if (out->globalKeyEndB) CK(cudaMemcpyAsync(out->globalKeyEndB, ctx->dLinkKeyB, 8 * (size_t)L, cudaMemcpyDefault, st));
     if (out->particleLinkNum) CK(cudaMemcpyAsync(out->particleLinkNum, ctx->dLinkNum, 4 * (size_t)L, cudaMemcpyDefault, st));
     CK(cudaStreamSynchronize(st));
+    dfree(staging);
     return HIDEM_OK;
 }
 
