@@ -918,6 +918,7 @@ hidem_status run_steps(hidem_ctx *ctx, int nsteps) {
     bool diffReady = false;
     bool gathered = false;     // the gather layout holds the state
     bool recStale = false;     // the records do not
+    bool chained = false;      // the stream's last kernel is a timestep's or a layout conversion
     auto records_now = [&]() {
         if (!recStale) return;
         launch_from_gather<LP>(gather_buf<LP>(ctx), (int)ctx->n, recp<LP>(ctx, ctx->cur), ctx->stream);
@@ -944,6 +945,7 @@ hidem_status run_steps(hidem_ctx *ctx, int nsteps) {
             pending = false;
             TRY(do_rebuild(ctx));
             gathered = true;  // the rebuild walked it
+            chained = false;
         }
         const bool reduce = ctx->P.gridRegenInterval == -1 && (t + 1) % 10 == 0;
         diffReady = reduce;
@@ -953,6 +955,7 @@ hidem_status run_steps(hidem_ctx *ctx, int nsteps) {
             launch_to_gather<LP>(recp<LP>(ctx, ctx->cur), (int)ctx->n, gather_buf<LP>(ctx), ctx->stream);
             ctx->launches += 1;
             gathered = true;
+            chained = true;
         }
         if (!twoPass) {
             records_now();
@@ -968,17 +971,18 @@ hidem_status run_steps(hidem_ctx *ctx, int nsteps) {
         if (t0) CK(cudaEventRecord(t0, ctx->stream));
         if (twoPass) {
             const bool last = s == nsteps - 1;
-            launch_force<LP>(consts<LP>(ctx), a, ctx->smCount, ctx->stream);
+            launch_force<LP>(consts<LP>(ctx), a, ctx->smCount, chained, ctx->stream);
             launch_integrate_gather<LP>(consts<LP>(ctx), a.gather, last ? recp<LP>(ctx, ctx->cur) : nullptr, a.type,
                                         a.force, a.n, reduce, ctx->diffMax, ctx->stream);
             recStale = !last;
             ctx->launches += 2;
         } else {
             launch_step<LP>(consts<LP>(ctx), a, (int)ctx->maxNeigh, (int)ctx->maxLinksPP, kern, ctx->smCount,
-                            ctx->stream);
+                            chained, ctx->stream);
             ctx->launches += 1;
             ctx->cur = 1 - ctx->cur;  // the slot order (type / orig / cellOf) is unchanged
         }
+        chained = true;
         if (t1) CK(cudaEventRecord(t1, ctx->stream));
         if (e1) CK(cudaEventRecord(e1, ctx->stream));
         pending = break_active<LP>(ctx, t);
@@ -1494,7 +1498,7 @@ hidem_status batch_run(hidem_batch *b, int nsteps) {
                     if (a.reduceDiff)
                         BCK(cudaMemsetAsync(c->diffMax, 0, 3 * sizeof(unsigned long long), b->stream));
                     launch_step<LP>(consts<LP>(c), a, (int)c->maxNeigh, (int)c->maxLinksPP,
-                                    fused_kernel(step_kernel_settled(c)), c->smCount, b->stream);
+                                    fused_kernel(step_kernel_settled(c)), c->smCount, j > 0 || idx > 0, b->stream);
                     c->launches += 1;
                     b->launches += 1;
                 }
@@ -2000,7 +2004,7 @@ static hidem_status compute_forces_t(hidem_ctx *ctx, void *sendBuf) {
         a.sendPos = ctx->haloSendPos;
         a.sendBuf = static_cast<LP *>(sendBuf);
     }
-    launch_force<LP>(consts<LP>(ctx), a, ctx->smCount, ctx->stream);
+    launch_force<LP>(consts<LP>(ctx), a, ctx->smCount, true, ctx->stream);
     ctx->launches += 2;
     CK(cudaGetLastError());
     if (sendBuf && !packed) TRY(halo_forces(ctx, sendBuf, true));

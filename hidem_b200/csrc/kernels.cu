@@ -31,6 +31,18 @@ __device__ __forceinline__ PRec<LP> load_rec(const PRec<LP> *p) {
     return r;
 }
 
+// The first CHUNKS 16-byte chunks of a record that the kernel before may have written (the rest
+// stays unset): plain loads, for kernels that are launched dependent (dependent_start).
+template <class LP, int CHUNKS = (int)(sizeof(PRec<LP>) / 16)>
+__device__ __forceinline__ PRec<LP> load_rec_written(const PRec<LP> *p) {
+    PRec<LP> r;
+    const int4 *src = reinterpret_cast<const int4 *>(p);
+    int4 *dst = reinterpret_cast<int4 *>(&r);
+#pragma unroll
+    for (int k = 0; k < CHUNKS; ++k) dst[k] = src[k];
+    return r;
+}
+
 template <class LP>
 __device__ __forceinline__ void store_rec(PRec<LP> *p, const PRec<LP> &r) {
     int4 *dst = reinterpret_cast<int4 *>(p);
@@ -56,12 +68,20 @@ __device__ __forceinline__ void set_error(int *flag, int code) {
 // ends when the predecessor has completed) before the first access, then lets its own successor
 // be placed. Worth a launch's latency per kernel: 9.1 -> 8.2 us a step on
 // 256 particles, 26.1 -> 23.3 us on 32,000 (two kernels a step).
+// Such a kernel is resident while its predecessor still writes, so what the predecessor may
+// write is not read-only for its lifetime: records, gather layout and forces are read with plain
+// loads, which stay behind the wait (no __ldg, no const __restrict__; load_rec_written,
+// load_body). The lists and constants are read through the read-only path, so the kernels that
+// read them (k_force, k_step_items) are launched dependent only where the kernel before them is
+// one of a timestep's own, none of which writes a list (`chained`); one that follows a rebuild, an
+// upload or whatever came before the call is launched plainly.
 __device__ __forceinline__ void dependent_start() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 template <class... P, class... A>
-static void launch_dependent(void (*kernel)(P...), int grid, int block, size_t smem, cudaStream_t s, A &&...args) {
+static void launch_dependent(bool dependent, void (*kernel)(P...), int grid, int block, size_t smem, cudaStream_t s,
+                             A &&...args) {
     cudaLaunchAttribute attr{};
     attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr.val.programmaticStreamSerializationAllowed = 1;
@@ -71,7 +91,7 @@ static void launch_dependent(void (*kernel)(P...), int grid, int block, size_t s
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
     cfg.attrs = &attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = dependent ? 1 : 0;
     cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
 }
 
@@ -418,13 +438,14 @@ struct Body {
     Six<LP> d;
     LP r, th[3];
 };
-// (WITH_R: the radius too; WITH_TH: the rotations too; fields not asked for stay unset)
+// (WITH_R: the radius too; WITH_TH: the rotations too; fields not asked for stay unset. Plain
+// loads: the kernel before may have written the layout, dependent_start)
 template <bool WITH_R, bool WITH_TH>
 __device__ __forceinline__ void load_body(Body<float> &o, const int4 *base, int slot) {
     const int4 *p = base + gather_index<float>(slot);
-    const double2 c0 = __ldg(reinterpret_cast<const double2 *>(p));
-    const ulonglong2 c1 = __ldg(reinterpret_cast<const ulonglong2 *>(p + 32));
-    const ulonglong2 c2 = __ldg(reinterpret_cast<const ulonglong2 *>(p + 64));
+    const double2 c0 = *reinterpret_cast<const double2 *>(p);
+    const ulonglong2 c1 = *reinterpret_cast<const ulonglong2 *>(p + 32);
+    const ulonglong2 c2 = *reinterpret_cast<const ulonglong2 *>(p + 64);
     o.x = c0.x;
     o.y = c0.y;
     o.z = __longlong_as_double((long long)c1.x);
@@ -432,19 +453,19 @@ __device__ __forceinline__ void load_body(Body<float> &o, const int4 *base, int 
     o.d.p[1].v = c2.x;
     o.d.p[2].v = c2.y;
     if (WITH_TH) {
-        const float4 c3 = __ldg(reinterpret_cast<const float4 *>(p + 96));
+        const float4 c3 = *reinterpret_cast<const float4 *>(p + 96);
         o.r = c3.x;
         o.th[0] = c3.y;
         o.th[1] = c3.z;
         o.th[2] = c3.w;
     } else if (WITH_R) {
-        o.r = __ldg(reinterpret_cast<const float *>(p + 96));
+        o.r = *reinterpret_cast<const float *>(p + 96);
     }
 }
 template <bool WITH_R, bool WITH_TH>
 __device__ __forceinline__ void load_body(Body<double> &o, const int4 *base, int slot) {
     const double2 *p = reinterpret_cast<const double2 *>(base + gather_index<double>(slot));
-    const double2 c0 = __ldg(p), c1 = __ldg(p + 32), c2 = __ldg(p + 64), c3 = __ldg(p + 96);
+    const double2 c0 = p[0], c1 = p[32], c2 = p[64], c3 = p[96];
     o.x = c0.x;
     o.y = c0.y;
     o.z = c1.x;
@@ -454,17 +475,17 @@ __device__ __forceinline__ void load_body(Body<double> &o, const int4 *base, int
     o.d.f[3] = c3.x;
     o.d.f[4] = c3.y;
     if (WITH_R) {
-        const double2 c4 = __ldg(p + 128);
+        const double2 c4 = p[128];
         o.d.f[5] = c4.x;
         o.r = c4.y;
     } else {
-        o.d.f[5] = __ldg(reinterpret_cast<const double *>(p + 128));
+        o.d.f[5] = *reinterpret_cast<const double *>(p + 128);
     }
     if (WITH_TH) {
-        const double2 c5 = __ldg(p + 160);
+        const double2 c5 = p[160];
         o.th[0] = c5.x;
         o.th[1] = c5.y;
-        o.th[2] = __ldg(reinterpret_cast<const double *>(p + 192));
+        o.th[2] = *reinterpret_cast<const double *>(p + 192);
     }
 }
 template <class LP>
@@ -1040,10 +1061,10 @@ __global__ void __launch_bounds__(kStepThreads, MINB)
 
 // records -> gather layout, and back
 template <class LP>
-__global__ void __launch_bounds__(256) k_to_gather(const PRec<LP> *__restrict__ rec, int n, int4 *__restrict__ g) {
+__global__ void __launch_bounds__(256) k_to_gather(const PRec<LP> *rec, int n, int4 *g) {
     dependent_start();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) store_gather(g, i, load_rec(rec + i));
+    if (i < n) store_gather(g, i, load_rec_written(rec + i));
 }
 template <class LP>
 __global__ void __launch_bounds__(256) k_from_gather(const int4 *__restrict__ g, int n, PRec<LP> *__restrict__ rec) {
@@ -1255,7 +1276,7 @@ __device__ __forceinline__ void step_items_block(const Consts<LP> &c, const Step
         ns = (int)(cnt >> 16);
         const unsigned sbase = (unsigned)__ldg(a.sOff + w) + lane;
         const int32_t *nb = a.nbr + __ldg(a.nOff + w) + lane;
-        me = load_rec(a.in + i);
+        me = load_rec_written(a.in + i);
         const Six<LP> mine = Six<LP>::of(me.d);
         for (int k = wid; k < ns; k += WARPS) {
             const unsigned si = sbase + k * kWarp;
@@ -1264,7 +1285,7 @@ __device__ __forceinline__ void step_items_block(const Consts<LP> &c, const Step
             LP CT[6];
 #pragma unroll
             for (int u = 0; u < 6; ++u) CT[u] = a.ct[u][si];
-            const PRec<LP> o = load_rec(a.in + (pw & kSlotMask));
+            const PRec<LP> o = load_rec_written(a.in + (pw & kSlotMask));
             const LP x = (LP)(me.x - o.x), y = (LP)(me.y - o.y), z = (LP)(me.z - o.z);
             if (brk) st = pending_break<LP>(a, si, pw, me, o, st, __ldg(a.sL0 + si), x, y, z);
             Six<LP> dpv, ctv;
@@ -1280,7 +1301,7 @@ __device__ __forceinline__ void step_items_block(const Consts<LP> &c, const Step
             }
         }
         for (int k = WARPS - 1 - wid; k < nn; k += WARPS) {
-            const PRec<LP> o = load_rec_head<LP, kContactChunks<LP>>(a.in + __ldg(nb + k * kWarp));
+            const PRec<LP> o = load_rec_written<LP, kContactChunks<LP>>(a.in + __ldg(nb + k * kWarp));
             Six<LP> tv = Six<LP>::zero();
             contact_terms(c, R, (LP)(me.x - o.x), (LP)(me.y - o.y), (LP)(me.z - o.z), mine, me.r,
                           Six<LP>::of(o.d), o.r, tv);
@@ -1465,7 +1486,7 @@ __device__ __forceinline__ void integrate_gather(const Consts<LP> &c, int4 *g, P
 template <class LP>
 __global__ void __launch_bounds__(kStepThreads, sizeof(LP) == 8 ? 7 : 8)
     k_integrate_gather(const Consts<LP> c, int4 *g, PRec<LP> *rec, const uint8_t *__restrict__ type,
-                       const LP *__restrict__ force, int n, bool reduce, unsigned long long *diffMax) {
+                       const LP *force, int n, bool reduce, unsigned long long *diffMax) {
     dependent_start();
     integrate_gather<LP>(c, g, rec, type, force, n, blockIdx.x * blockDim.x + threadIdx.x, reduce, diffMax);
 }
@@ -1731,7 +1752,8 @@ void launch_side_fill(const int *orig, int n, const int *slotOf, const int *plSt
 }
 
 template <class LP, int WARPS>
-static void launch_items(const Consts<LP> &c, const StepArgs<LP> &a, int blocks, size_t bytes, cudaStream_t s) {
+static void launch_items(const Consts<LP> &c, const StepArgs<LP> &a, int blocks, size_t bytes, bool chained,
+                         cudaStream_t s) {
     // the shared-memory limit is a per-device attribute: set it once on each device
     // (setting it twice, as racing threads may, is harmless)
     static std::atomic<unsigned long long> configured;
@@ -1742,12 +1764,12 @@ static void launch_items(const Consts<LP> &c, const StepArgs<LP> &a, int blocks,
         cudaFuncSetAttribute(k_step_items<LP, WARPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kItemSmemLimit);
         configured.fetch_or(bit);
     }
-    launch_dependent(k_step_items<LP, WARPS>, blocks, WARPS * 32, bytes, s, c, a);
+    launch_dependent(chained, k_step_items<LP, WARPS>, blocks, WARPS * 32, bytes, s, c, a);
 }
 
 template <class LP>
 void launch_step(const Consts<LP> &c, const StepArgs<LP> &a0, int maxContacts, int maxEnds, int kernel, int smCount,
-                 cudaStream_t s) {
+                 bool chained, cudaStream_t s) {
     StepArgs<LP> a = a0;
     a.maxContacts = maxContacts;
     a.maxEnds = maxEnds;
@@ -1756,9 +1778,9 @@ void launch_step(const Consts<LP> &c, const StepArgs<LP> &a0, int maxContacts, i
         // the fewer blocks, the more warps each (one block an SM: 16, so that no warp has more
         // than one link end and one contact of a lattice particle's twelve)
         const int nb = nblk(a.n, 32);
-        if (nb <= smCount) launch_items<LP, 16>(c, a, nb, bytes, s);
-        else if (nb <= 3 * smCount) launch_items<LP, 8>(c, a, nb, bytes, s);
-        else launch_items<LP, 4>(c, a, nb, bytes, s);
+        if (nb <= smCount) launch_items<LP, 16>(c, a, nb, bytes, chained, s);
+        else if (nb <= 3 * smCount) launch_items<LP, 8>(c, a, nb, bytes, chained, s);
+        else launch_items<LP, 4>(c, a, nb, bytes, chained, s);
         return;
     }
     // one thread per particle (also for rows too wide for the item kernel's buffers)
@@ -1779,27 +1801,27 @@ void launch_side_move(const int *perm, int n, const int *newSlot, const uint32_t
 }
 
 template <class LP, bool AHEAD, int MINB>
-static void launch_force_as(const Consts<LP> &c, const StepArgs<LP> &a, cudaStream_t s) {
+static void launch_force_as(const Consts<LP> &c, const StepArgs<LP> &a, bool chained, cudaStream_t s) {
     const int nb = nblk(a.n, kStepThreads);
     if (a.breakPending)
-        launch_dependent(k_force<LP, true, AHEAD, MINB>, nb, kStepThreads, 0, s, c, a);
+        launch_dependent(chained, k_force<LP, true, AHEAD, MINB>, nb, kStepThreads, 0, s, c, a);
     else
-        launch_dependent(k_force<LP, false, AHEAD, MINB>, nb, kStepThreads, 0, s, c, a);
+        launch_dependent(chained, k_force<LP, false, AHEAD, MINB>, nb, kStepThreads, 0, s, c, a);
 }
 
 // A particle set that fits the chip in one wave at kFewBlocks CTAs an SM gains nothing from
 // more warps an SM: it takes the variant that keeps the next item in flight.
 template <class LP>
-void launch_force(const Consts<LP> &c, const StepArgs<LP> &a, int smCount, cudaStream_t s) {
+void launch_force(const Consts<LP> &c, const StepArgs<LP> &a, int smCount, bool chained, cudaStream_t s) {
     if (nblk(a.n, kStepThreads) <= kFewBlocks<LP> * smCount)
-        launch_force_as<LP, true, kFewBlocks<LP>>(c, a, s);
+        launch_force_as<LP, true, kFewBlocks<LP>>(c, a, chained, s);
     else
-        launch_force_as<LP, kForceAhead<LP>, kForceBlocks<LP>>(c, a, s);
+        launch_force_as<LP, kForceAhead<LP>, kForceBlocks<LP>>(c, a, chained, s);
 }
 
 template <class LP>
 void launch_to_gather(const PRec<LP> *rec, int n, int4 *g, cudaStream_t s) {
-    launch_dependent(k_to_gather<LP>, nblk(n, 256), 256, 0, s, rec, n, g);
+    launch_dependent(true, k_to_gather<LP>, nblk(n, 256), 256, 0, s, rec, n, g);
 }
 template <class LP>
 void launch_from_gather(const int4 *g, int n, PRec<LP> *rec, cudaStream_t s) {
@@ -1808,8 +1830,8 @@ void launch_from_gather(const int4 *g, int n, PRec<LP> *rec, cudaStream_t s) {
 template <class LP>
 void launch_integrate_gather(const Consts<LP> &c, int4 *g, PRec<LP> *rec, const uint8_t *type, const LP *force,
                              int n, bool reduce, unsigned long long *diffMax, cudaStream_t s) {
-    launch_dependent(k_integrate_gather<LP>, nblk(n, kStepThreads), kStepThreads, 0, s, c, g, rec, type, force, n, reduce,
-                     diffMax);
+    launch_dependent(true, k_integrate_gather<LP>, nblk(n, kStepThreads), kStepThreads, 0, s, c, g, rec, type, force, n,
+                     reduce, diffMax);
 }
 
 template <class LP>
@@ -2028,12 +2050,12 @@ void launch_max_diff(const PRec<LP> *rec, int n, unsigned long long *out, int nb
                                        const uint8_t *, const int *, const int *, const LP *,      \
                                        const int *, const SideView<LP> &, const long long *,       \
                                        const SideView<LP> &, int *, cudaStream_t);                 \
-    template void launch_step<LP>(const Consts<LP> &, const StepArgs<LP> &, int, int, int, int,     \
+    template void launch_step<LP>(const Consts<LP> &, const StepArgs<LP> &, int, int, int, int, bool, \
                                   cudaStream_t);                                                   \
     template void launch_side_move<LP>(const int *, int, const int *, const uint32_t *, const long long *, \
                                        const SideView<LP> &, const long long *, const SideView<LP> &, int *, \
                                        cudaStream_t);                                              \
-    template void launch_force<LP>(const Consts<LP> &, const StepArgs<LP> &, int, cudaStream_t);           \
+    template void launch_force<LP>(const Consts<LP> &, const StepArgs<LP> &, int, bool, cudaStream_t);     \
     template void launch_to_gather<LP>(const PRec<LP> *, int, int4 *, cudaStream_t);               \
     template void launch_from_gather<LP>(const int4 *, int, PRec<LP> *, cudaStream_t);             \
     template void launch_integrate_gather<LP>(const Consts<LP> &, int4 *, PRec<LP> *, const uint8_t *, \

@@ -144,16 +144,18 @@ void launch_side_move(const int *perm, int n, const int *newSlot, const uint32_t
 // One fused timestep (previous link update, forces, integrate, record swap) for rows of at
 // most maxContacts contacts and maxEnds link ends, by the kernel `kernel`
 // (HIDEM_STEP_KERNEL_*, not AUTO or TWO_PASS; the item kernel falls back to one thread per
-// particle for rows too wide for its shared-memory buffers).
+// particle for rows too wide for its shared-memory buffers). chained: the stream's kernel before
+// this one is one of the timestep kernels or layout conversions below, none of which writes a
+// list that this one reads (launch_dependent, kernels.cu).
 template <class LP>
 void launch_step(const Consts<LP> &c, const StepArgs<LP> &a, int maxContacts, int maxEnds, int kernel,
-                 int smCount, cudaStream_t s);
+                 int smCount, bool chained, cudaStream_t s);
 // The force pass (a.gather holds the records in the gather layout), applying the previous
-// step's link update on the way when a.breakPending; the integrate pass on the gather layout
+// step's link update on the way when a.breakPending (chained: as above); the integrate pass on the gather layout
 // (rec: the records too, or null; reduce: the diff maxima into diffMax); and the two layouts'
 // conversions (a gather buffer holds whole blocks of 32 slots).
 template <class LP>
-void launch_force(const Consts<LP> &c, const StepArgs<LP> &a, int smCount, cudaStream_t s);
+void launch_force(const Consts<LP> &c, const StepArgs<LP> &a, int smCount, bool chained, cudaStream_t s);
 template <class LP>
 void launch_integrate_gather(const Consts<LP> &c, int4 *g, PRec<LP> *rec, const uint8_t *type, const LP *force,
                              int n, bool reduce, unsigned long long *diffMax, cudaStream_t s);
