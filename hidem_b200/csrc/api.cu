@@ -189,7 +189,7 @@ struct hidem_ctx {
     long long launches = 0;
     int smCount = 148;
 
-    // step kernel: fixed by the caller, or timed on the first fused steps (AUTO)
+    // step kernel: fixed by the caller, or timed on a small set's first steps (AUTO)
     int stepKernel = HIDEM_STEP_KERNEL_AUTO;
     int tunedKernel = HIDEM_STEP_KERNEL_AUTO;
     int tuneStep = 0;
@@ -842,10 +842,14 @@ hidem_status profile_pair(hidem_ctx *ctx, cudaEvent_t *e0, cudaEvent_t *e1) {
 
 // The step kernel of AUTO. A context of more than kTuneMax particles takes the two-pass step:
 // 5.7M particles 1.44 ms a step against 2.17 ms for the best one-kernel step (mixed), 0.8M
-// 0.24 ms against 0.34 ms. Smaller ones time the item kernel against it: the first kTuneRounds * 2 steps of
-// the context alternate with an event pair around each; the faster, summed over all but the
-// first round, is kept (8,892 particles in FP64: 14.5 us a step against 22.0 us; 32,000 mixed:
-// 24.3 against 23.3 us).
+// 0.24 ms against 0.34 ms; just above the border, 67,600 particles, 29.3 against 35.5 us mixed and
+// 47.2 against 65.8 FP64, without links 15.3 against 18.7 and 21.2 against 30.9, with neither
+// links nor contacts 8.6 against 8.2 and 10.5 against 12.4. Smaller ones time the item kernel
+// against it: the first kTuneRounds * 2 steps with a set of that many particles alternate with an
+// event pair around each; the faster, summed over all but the first round, is kept (8,892
+// particles in FP64: 14.5 us a step against 22.0 us; 32,000 mixed: 24.3 against 23.3 us; 62,500
+// with neither links nor contacts 8.0 against 8.4). The choice lasts until a set of another size
+// arrives (hidem_set_particles).
 constexpr long long kTuneMax = 65536;
 constexpr int kTuneCandidates[] = {HIDEM_STEP_KERNEL_ITEMS, HIDEM_STEP_KERNEL_TWO_PASS};
 constexpr int kNumCandidates = (int)(sizeof(kTuneCandidates) / sizeof(int));
@@ -859,7 +863,7 @@ int fused_kernel(int k) { return k == HIDEM_STEP_KERNEL_TWO_PASS ? HIDEM_STEP_KE
 int step_kernel_now(hidem_ctx *ctx, cudaEvent_t *e0, cudaEvent_t *e1) {
     *e0 = *e1 = nullptr;
     if (ctx->stepKernel != HIDEM_STEP_KERNEL_AUTO) return ctx->stepKernel;
-    if (ctx->n > kTuneMax) return ctx->tunedKernel = HIDEM_STEP_KERNEL_TWO_PASS;
+    if (ctx->n > kTuneMax) return HIDEM_STEP_KERNEL_TWO_PASS;
     if (ctx->tunedKernel != HIDEM_STEP_KERNEL_AUTO) return ctx->tunedKernel;
     if (ctx->tuneStep < kNumCandidates * kTuneRounds) {
         const int k = ctx->tuneStep++;
@@ -873,11 +877,16 @@ int step_kernel_now(hidem_ctx *ctx, cudaEvent_t *e0, cudaEvent_t *e1) {
     return HIDEM_STEP_KERNEL_TWO_PASS;  // rounds done, choice made at the next sync
 }
 
+// the kernel in use, AUTO while a small set's is still to be timed
+int step_kernel_known(const hidem_ctx *ctx) {
+    if (ctx->stepKernel != HIDEM_STEP_KERNEL_AUTO) return ctx->stepKernel;
+    return ctx->n > kTuneMax ? HIDEM_STEP_KERNEL_TWO_PASS : ctx->tunedKernel;
+}
+
 // the kernel of a launch outside the tuning rounds
 int step_kernel_settled(const hidem_ctx *ctx) {
-    if (ctx->stepKernel != HIDEM_STEP_KERNEL_AUTO) return ctx->stepKernel;
-    if (ctx->tunedKernel != HIDEM_STEP_KERNEL_AUTO) return ctx->tunedKernel;
-    return HIDEM_STEP_KERNEL_TWO_PASS;
+    const int k = step_kernel_known(ctx);
+    return k != HIDEM_STEP_KERNEL_AUTO ? k : HIDEM_STEP_KERNEL_TWO_PASS;
 }
 
 // called after the stream has been synchronised
@@ -1136,16 +1145,21 @@ struct BatchBind {
     }
 };
 
-// the kernel a batch run uses: the first context's fixed or tuned choice (the
-// asynchronous-copy kernel has no batched form: its register-capped sibling stands in),
-// else the register-capped one-thread-per-particle kernel
+// The kernel a batch run uses: the first context's fixed choice (the asynchronous-copy kernel has
+// no batched form: its register-capped sibling stands in), or its tuned one where the whole batch
+// is no larger than a set AUTO times (a choice timed on a small set says nothing about a large
+// launch), else the two-pass step (measured on the 256-block ensemble: 2.96 ms per step against
+// 3.53 ms for the capped fused kernel).
 int batch_kernel(const hidem_batch *b) {
     const hidem_ctx *c = b->ctxs[0];
-    // the two-pass step unless the first context names another kernel (measured on the
-    // 256-block ensemble: 2.96 ms per step against 3.53 ms for the capped fused kernel)
     int k = HIDEM_STEP_KERNEL_TWO_PASS;
-    if (c->stepKernel != HIDEM_STEP_KERNEL_AUTO) k = c->stepKernel;
-    else if (c->tunedKernel != HIDEM_STEP_KERNEL_AUTO) k = c->tunedKernel;
+    if (c->stepKernel != HIDEM_STEP_KERNEL_AUTO) {
+        k = c->stepKernel;
+    } else {
+        long long total = 0;
+        for (const hidem_ctx *m : b->ctxs) total += m->n;
+        if (total <= kTuneMax) k = step_kernel_settled(c);
+    }
     return k == HIDEM_STEP_KERNEL_THREAD_ASYNC ? HIDEM_STEP_KERNEL_THREAD_CAPPED : k;
 }
 
@@ -1786,6 +1800,11 @@ hidem_status hidem_set_particles(hidem_ctx *ctx, const hidem_particle_soa *p, in
     else for (int64_t i = 0; i < n; ++i) ctx->keys[i] = i;
     CK(cudaStreamSynchronize(ctx->stream));
     CK(cudaGetLastError());
+    if (n != ctx->n) {
+        // AUTO's choice was timed on the previous set
+        ctx->tuneStep = 0;
+        ctx->tunedKernel = HIDEM_STEP_KERNEL_AUTO;
+    }
     ctx->n = n;
     ctx->haveParticles = true;
     ctx->built = false;
@@ -3008,7 +3027,7 @@ hidem_status hidem_set_step_kernel(hidem_ctx *ctx, int32_t kernel) {
 
 int32_t hidem_get_step_kernel(const hidem_ctx *ctx) {
     if (!ctx) return -1;
-    return ctx->stepKernel != HIDEM_STEP_KERNEL_AUTO ? ctx->stepKernel : ctx->tunedKernel;
+    return step_kernel_known(ctx);
 }
 
 hidem_status hidem_batch_create(hidem_ctx *const *ctxs, int32_t nctx, int32_t flags,

@@ -516,9 +516,9 @@ hidem_status hidem_momentum(hidem_ctx *ctx, double linear[3], double angular[3])
  * step's link update on the way, and an integrate pass, the state kept between them in a
  * layout of its own until the call's last step. AUTO (the default) is TWO_PASS above 65,536
  * particles; a smaller context times ITEMS against it on its own first steps (five rounds, the
- * first discarded) and keeps the faster; those steps are ordinary timesteps.
- * hidem_get_step_kernel returns the kernel in use (AUTO before the first step and while still
- * timing). */
+ * first discarded) and keeps the faster until a set of another size is given; those steps are
+ * ordinary timesteps. hidem_get_step_kernel returns the kernel in use (AUTO while a small context
+ * is still to time its own). */
 #define HIDEM_STEP_KERNEL_AUTO 0
 #define HIDEM_STEP_KERNEL_ITEMS 1
 #define HIDEM_STEP_KERNEL_THREAD 2
@@ -540,8 +540,8 @@ int32_t hidem_get_step_kernel(const hidem_ctx *ctx);
  * HIDEM_BATCH_GRAPHS is set. Each context's results are bit-identical to hidem_step on
  * that context alone: the batch runs the same gridService policy and the same step and
  * link update per context. The step kernel is the first context's
- * (hidem_set_step_kernel; AUTO or untimed means TWO_PASS, THREAD_ASYNC runs as
- * THREAD_CAPPED).
+ * (hidem_set_step_kernel; THREAD_ASYNC runs as THREAD_CAPPED). AUTO means TWO_PASS, or what the
+ * first context has timed where the batch has no more than 65,536 particles in all.
  * HIDEM_BATCH_PER_CONTEXT runs the single-context launch sequence context after context
  * instead (the same results, for comparison); rows too wide for the ITEMS kernel's shared
  * memory take that path too. During a batch call the contexts' work runs on the batch's
