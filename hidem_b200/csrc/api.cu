@@ -1414,6 +1414,17 @@ hidem_status batch_run(hidem_batch *b, int nsteps) {
     BCK(cudaMemsetAsync(b->diff, 0, 3 * sizeof(unsigned long long) * nc, b->stream));
     std::vector<char> pending(nc, 0), diffReady(nc, 0);
     std::vector<long long> pendStep(nc, 0);
+    // the link updates these contexts owe from a fused step
+    std::vector<int> all(nc);
+    for (int idx = 0; idx < nc; ++idx) all[idx] = idx;
+    auto settle = [&](const std::vector<int> &list) -> hidem_status {
+        for (int idx : list)
+            if (pending[idx]) {
+                BTRY(link_update_now<LP>(b->ctxs[idx], pendStep[idx]));
+                pending[idx] = 0;
+            }
+        return HIDEM_OK;
+    };
     bool dirty = true;
     int s = 0;
     while (s < nsteps) {
@@ -1443,7 +1454,17 @@ hidem_status batch_run(hidem_batch *b, int nsteps) {
                 const double cd = gs_wants_diff(c) ? curr_dist<LP>(mx) : 0.0;
                 if (gs_decide(c, cd)) regen.push_back(idx);
             }
-            if (!regen.empty()) TRY(batch_rebuild(b, regen, bind.streams));
+            // a rebuild may fail: the link updates still owed are the previous step's
+            if (!regen.empty()) {
+                TRY(settle(regen));
+                const hidem_status st = batch_rebuild(b, regen, bind.streams);
+                if (st != HIDEM_OK) {
+                    const std::string why = b->err;
+                    TRY(settle(all));
+                    b->err = why;
+                    return st;
+                }
+            }
             dirty = true;
         }
         long long run = nsteps - s;
@@ -1475,14 +1496,7 @@ hidem_status batch_run(hidem_batch *b, int nsteps) {
             BCK(cudaEventRecord(e0, b->stream));
         }
         const bool twoPass = oneLaunch && kernel == HIDEM_STEP_KERNEL_TWO_PASS;
-        if (twoPass) {
-            // a link update still owed by a fused run, before the two-pass steps
-            for (int idx = 0; idx < nc; ++idx)
-                if (pending[idx]) {
-                    BTRY(link_update_now<LP>(b->ctxs[idx], pendStep[idx]));
-                    pending[idx] = 0;
-                }
-        }
+        if (twoPass) TRY(settle(all));  // what a fused run still owes, before the two-pass steps
         if (oneLaunch) {
             // every run's launches take their steps as 0 .. run - 1 after the entries' first
             // step (parameters fixed in a captured run): each run starts from the host's step
@@ -1535,8 +1549,7 @@ hidem_status batch_run(hidem_batch *b, int nsteps) {
         }
         s += (int)run;
     }
-    for (int idx = 0; idx < nc; ++idx)
-        if (pending[idx]) BTRY(link_update_now<LP>(b->ctxs[idx], pendStep[idx]));
+    TRY(settle(all));
     BCK(cudaGetLastError());
     for (int idx = 0; idx < nc; ++idx) BTRY(check_device_error(b->ctxs[idx]));
     return HIDEM_OK;

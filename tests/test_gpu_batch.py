@@ -233,3 +233,41 @@ def test_batch_runs_without_grid_service_between_them(gpu, kernel):
         assert_same(snapshot(lib), ref)
         lib.close()
     assert sum(len(r[2]) for r in alone) > 0  # links broke inside the runs
+
+
+# a rebuild the batch is refused leaves every context the state of the steps before it, their
+# link updates included, as hidem_step alone does
+@pytest.mark.parametrize("precision", PRECS)
+@pytest.mark.parametrize("kernel", [abi.STEP_KERNEL_TWO_PASS, abi.STEP_KERNEL_ITEMS, abi.STEP_KERNEL_THREAD_CAPPED])
+def test_batch_that_ends_in_a_refused_rebuild(gpu, precision, kernel):
+    out = []
+    for batched in (True, False):
+        libs = []
+        for interval in (8, 50):  # the second context has no rebuild due at step 8
+            P, p, l = workloads.ice_block(cells=(4, 4, 4), precision=precision, seed=7, g=-2e6,
+                                          gridRegenInterval=interval)
+            if interval == 8:
+                p["zDiff"][-1] = 60.0  # leaves the block: the grid of step 8 has far more cells
+            lib = open_lib(P, p, l, 0)
+            lib.set_checks(abi.CHECK_GRID_GROWTH)
+            lib.set_step_kernel(kernel)
+            libs.append(lib)
+        if batched:
+            batch = HiDEMBatch(libs)
+            with pytest.raises(abi.HidemError) as e:
+                batch.step(16)
+            assert e.value.status == abi.HIDEM_ERR_DEVICE and "10x" in str(e.value)
+            batch.close()
+        else:
+            for lib in libs:
+                lib.step(8)
+        out.append([snapshot(lib) for lib in libs])
+        for lib in libs:
+            lib.close()
+    for a, b in zip(*out):
+        for k in P_OUT:
+            assert np.array_equal(a[0][k], b[0][k], equal_nan=True), k
+        for k in L_OUT:
+            assert np.array_equal(a[1][k], b[1][k], equal_nan=True), k
+        assert np.array_equal(a[2], b[2]) and a[4] == b[4] == 8
+        assert np.any(a[2][:, 1] == 7)  # links broke in the last step before the rebuild
