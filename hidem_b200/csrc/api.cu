@@ -568,10 +568,12 @@ hidem_status rebuild(hidem_ctx *ctx) {
         launch_send_pos(ctx->slotOf, ctx->haloSend, ctx->nHaloSend, n, ctx->haloSendPos, st);
         ctx->launches += 1;
     }
-    // until the link ends follow, they lie in a layout that `perm` does not start from: a rebuild
-    // after one that fails below goes through the links
+    // until the contact list and the link ends follow, neither is of the slot order: a rebuild that
+    // fails below leaves no structure behind, and the one after it goes through the links (they lie
+    // in a layout that `perm` does not start from)
     const bool sidesBlocked = ctx->sidesBlocked;
     ctx->sidesBlocked = false;
+    ctx->built = false;
     ctx->cur = nxt;
     ctx->ord = nd;
     const int c = nd;   // slot-order arrays

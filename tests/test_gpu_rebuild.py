@@ -6,7 +6,7 @@ import numpy as np
 import pytest
 
 from hidem_b200 import abi, workloads
-from hidem_b200.hidemlib import HiDEMLib
+from hidem_b200.hidemlib import HiDEMBatch, HiDEMLib
 from oracle import oracle
 from test_gpu_parity import L_OUT, P_OUT, PRECS, assert_same, gpu_run
 
@@ -80,3 +80,42 @@ def test_run_that_ends_in_a_refused_rebuild(gpu, precision, kernel):
     for k in L_OUT:
         assert np.array_equal(out[0][1][k], out[1][1][k], equal_nan=True), k
     assert out[0][2] == out[1][2] and len(out[0][2]) > 0
+
+
+# what follows a rebuild that failed midway starts with a rebuild of its own: the lists of the
+# layout before it are not read in the new slot order
+@pytest.mark.parametrize("precision", PRECS)
+@pytest.mark.parametrize("batched", [False, True])
+def test_steps_after_a_failed_rebuild(gpu, precision, batched):
+    P, p, l = workloads.ice_block(cells=(12, 12, 12), precision=precision, seed=5, g=-1e5)
+    out = []
+    for fail in (True, False):
+        lib = HiDEMLib(P)
+        lib.set_particles(p)
+        lib.set_links(l)
+        lib.step(8)
+        if fail:
+            wide = abi.HidemParams.from_buffer_copy(P)
+            wide.searchDistanceScale = 20.0
+            lib.set_params(wide)
+            with pytest.raises(abi.HidemError):
+                lib.regenerate()
+            with pytest.raises(abi.HidemError):  # refused again, not answered from the old lists
+                lib.computePartForce()
+            with pytest.raises(abi.HidemError):
+                lib.get_neighbours()
+            lib.set_params(P)
+        else:
+            lib.regenerate()
+        if batched:
+            with HiDEMBatch([lib]) as batch:
+                batch.step(9)
+        else:
+            lib.step(9)
+        out.append((lib.get_particles(), lib.get_links(), lib.get_neighbours()[0]))
+        lib.close()
+    for k in P_OUT:
+        assert np.array_equal(out[0][0][k], out[1][0][k]), k
+    for k in L_OUT:
+        assert np.array_equal(out[0][1][k], out[1][1][k]), k
+    assert np.array_equal(out[0][2], out[1][2])
