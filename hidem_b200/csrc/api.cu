@@ -442,6 +442,7 @@ hidem_status side_alloc(hidem_ctx *ctx, SideSet &s, long long cap) {
     if (s.cap >= cap && s.partner) return HIDEM_OK;
     if (cap <= 0) cap = 1;
     cap += cap / 4;
+    s.cap = 0;  // until every array has grown
     TRY(dalloc(ctx, &s.partner, cap));
     for (int k = 0; k < 6; ++k) TRY(dalloc_bytes(ctx, &s.ct[k], ctx->lp * (size_t)cap));
     TRY(dalloc(ctx, &s.state, cap));
@@ -465,6 +466,7 @@ long long nblocks32(long long n) { return (n + 31) / 32; }
 hidem_status ensure_scan(hidem_ctx *ctx, long long n) {
     long long need = (n + 1023) / 1024 + 1;
     if (ctx->scanCap >= need) return HIDEM_OK;
+    ctx->scanCap = 0;
     TRY(dalloc(ctx, &ctx->scanSums32, need));
     TRY(dalloc(ctx, &ctx->scanSums64, need));
     ctx->scanCap = need;
@@ -537,6 +539,7 @@ hidem_status rebuild(hidem_ctx *ctx) {
                 g.off[k++] = (long long)xD + (long long)yD * g.X + (long long)zD * g.X * g.Y;
     if (ctx->cellCap < g.total) {
         long long cap = g.total + g.total / 4 + 1024;
+        ctx->cellCap = 0;
         TRY(dalloc(ctx, &ctx->cellCount, cap));
         TRY(dalloc(ctx, &ctx->cellStart, cap));
         TRY(dalloc(ctx, &ctx->cursor, cap));
@@ -596,6 +599,7 @@ hidem_status rebuild(hidem_ctx *ctx) {
     TRY(check_device_error(ctx));  // waits for both
     if (nTotal > ctx->nbrCap) {
         long long cap = nTotal + nTotal / 8 + 1024;
+        ctx->nbrCap = 0;
         TRY(dalloc(ctx, &ctx->nbr, cap));
         ctx->nbrCap = cap;
     }
@@ -1778,6 +1782,8 @@ hidem_status hidem_set_particles(hidem_ctx *ctx, const hidem_particle_soa *p, in
     CK(cudaSetDevice(ctx->device));
     const size_t lp = ctx->lp;
     const size_t recBytes = ctx->mixed ? sizeof(PRec<float>) : sizeof(PRec<double>);
+    // from here the buffers are the new set's: a call that fails leaves no set behind
+    ctx->haveParticles = ctx->haveLinks = ctx->built = false;
     for (int b = 0; b < 2; ++b) {
         // whole blocks of 32: either buffer may hold the gather layout
         TRY(dalloc_bytes(ctx, &ctx->rec[b], recBytes * (size_t)(nblocks32(n) * 32)));
@@ -1822,14 +1828,12 @@ hidem_status hidem_set_particles(hidem_ctx *ctx, const hidem_particle_soa *p, in
     }
     ctx->n = n;
     ctx->haveParticles = true;
-    ctx->built = false;
     ctx->maxParticleRadius = -1.0;  // found on the device when a collision mesh needs it
     TRY(prune_mesh(ctx));
     ctx->startStep = ctx->step;
     // halo lists refer to particle indices of the previous particle set
     ctx->nHaloSend = ctx->nHaloRecv = 0;
     // a link set refers to particle indices of the previous particle set
-    ctx->haveLinks = false;
     ctx->L = 0;
     return HIDEM_OK;
 }
@@ -1861,6 +1865,8 @@ hidem_status hidem_set_links(hidem_ctx *ctx, const hidem_link_soa *l, int64_t L)
         ascending = up.load();
     }
     cudaStream_t st = ctx->stream;
+    // from here the buffers are the new set's: a call that fails leaves no link set behind
+    ctx->haveLinks = ctx->built = false;
     TRY(dalloc(ctx, &ctx->linkA, L));
     TRY(dalloc(ctx, &ctx->linkB, L));
     TRY(dalloc(ctx, &ctx->dLinkKeyA, L));
@@ -2002,7 +2008,6 @@ hidem_status hidem_set_links(hidem_ctx *ctx, const hidem_link_soa *l, int64_t L)
     dfree(cursor);
     ctx->L = L;
     ctx->haveLinks = true;
-    ctx->built = false;
     return HIDEM_OK;
 }
 

@@ -160,7 +160,10 @@ int hidem_abi_version(void);
  * hidem_get_particles / hidem_get_links may be host memory (pageable or pinned) or device
  * memory of the context's GPU (the copies stay on the device); device arrays handed in must
  * be complete when the call is made (the caller has synchronised the work that wrote
- * them), and the readbacks' arrays are complete when the call returns. */
+ * them), and the readbacks' arrays are complete when the call returns. A call refused for its
+ * arguments alone (missing arrays, counts out of range) changes nothing; one that fails later
+ * (a link end that names no particle, no memory) leaves the context without that set, and calls
+ * that need it answer HIDEM_ERR_STATE until it is given again. */
 hidem_status hidem_set_particles(hidem_ctx *ctx, const hidem_particle_soa *p, int64_t n);
 /* Replaces LinkDataHandler::appendInitLinks + LinkData::makeLocalPartEnds
  * (PLiB/LinkDataHandler.h:212-241, PLiB/LinkData.h:91-115): copies L links,

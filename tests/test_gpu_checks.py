@@ -136,3 +136,31 @@ def test_overcrowded_cell_is_refused(gpu):
     lib.set_links(abi.empty_links(0, abi.PREC_MIXED))
     assert _status(lib.regenerate) == abi.HIDEM_ERR_CAPACITY
     lib.close()
+
+
+def test_refused_link_set_leaves_none_behind(gpu):
+    """The buffers are the refused set's by then, so the one before it cannot be stepped on; the
+    context takes the next set as a new one."""
+    P, p, l = workloads.ice_block(cells=(4, 4, 4), precision=abi.PREC_MIXED, seed=5)
+    few = {k: v[:2 * 7] if k.startswith("CT") else v[:7] for k, v in l.items()}
+    out = []
+    for refused in (True, False):
+        lib = HiDEMLib(P)
+        lib.set_particles(p)
+        lib.set_links(l)
+        lib.step(3)
+        if refused:
+            for end, status in ((10 ** 6, abi.HIDEM_ERR_NOT_FOUND), (int(few["globalKeyEndA"][3]), abi.HIDEM_ERR_ARG)):
+                bad = {k: v.copy() for k, v in few.items()}
+                bad["globalKeyEndB"][3] = end
+                assert _status(lambda: lib.set_links(bad)) == status
+                for call in (lambda: lib.step(1), lib.regenerate, lib.computePartForce, lib.linkUpdate, lib.get_links):
+                    assert _status(call) == abi.HIDEM_ERR_STATE
+        lib.set_links(l)
+        lib.step(12)
+        out.append((lib.get_particles(), lib.get_links()))
+        lib.close()
+    for k in ("xCord", "zCord", "wDiff"):
+        assert np.array_equal(out[0][0][k], out[1][0][k]), k
+    for k in ("state", "CT0", "CT5"):
+        assert np.array_equal(out[0][1][k], out[1][1][k]), k
