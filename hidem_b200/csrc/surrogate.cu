@@ -1504,7 +1504,7 @@ hidem_status order_after(hidem_surrogate *s, cudaStream_t from, cudaStream_t to,
 // output layer's gradient on one more. A settling batch (8,192 rows) is some forty kernels of 3-20 us that
 // fill a fraction of the chip each: one after another they took 0.36 of the step's 0.48 ms.
 // The sums and their order are those of the serial chain.
-hidem_status backward(hidem_surrogate *s, int rows, const float *targets, const int *idx) {
+hidem_status backward_fork(hidem_surrogate *s, int rows, const float *targets, const int *idx) {
     const int W = s->W, L = s->L;
     const int nb = (rows + 255) / 256;
     const int chunks = (rows + kChunk - 1) / kChunk;
@@ -1554,12 +1554,26 @@ hidem_status backward(hidem_surrogate *s, int rows, const float *targets, const 
             n0 += bn;
         }
         k_sum_splits<<<sum_splits_grid((long long)W * K), dim3(32, 8), 0, sl>>>(s->part[l], splits, (long long)W * K, s->G + s->offW[l]);
-        SCK(cudaEventRecord(s->evDone[l], sl));
     }
-    SCK(cudaEventRecord(s->evDone[L], so));
-    for (int l = 0; l <= L; ++l) SCK(cudaStreamWaitEvent(st, s->evDone[l], 0));
     SCK(cudaGetLastError());
     return HIDEM_OK;
+}
+
+// Every way out joins the side streams again, a failed launch's too: the next call writes the
+// buffers they read from the surrogate's stream. A failed call also waits, so that its caller's
+// arrays are no longer read when it returns.
+hidem_status backward(hidem_surrogate *s, int rows, const float *targets, const int *idx) {
+    hidem_status r = backward_fork(s, rows, targets, idx);
+    for (int l = 0; l <= s->L; ++l) {
+        cudaError_t e = cudaEventRecord(s->evDone[l], s->side[l]);
+        if (e == cudaSuccess) e = cudaStreamWaitEvent(s->stream, s->evDone[l], 0);
+        if (e != cudaSuccess) {
+            cudaStreamSynchronize(s->side[l]);
+            if (r == HIDEM_OK) r = sfail(s, HIDEM_ERR_CUDA, "joining the backward pass failed: %s", cudaGetErrorString(e));
+        }
+    }
+    if (r != HIDEM_OK) cudaStreamSynchronize(s->stream);
+    return r;
 }
 
 hidem_status read_loss(hidem_surrogate *s, int rows, double *loss) {
