@@ -1576,6 +1576,18 @@ hidem_status backward(hidem_surrogate *s, int rows, const float *targets, const 
     return r;
 }
 
+// whether the kernels may read or write a caller's rows where they lie: this GPU's memory, aligned
+// for a float (a copy takes any address, and other memory too)
+bool reachable(const hidem_surrogate *s, const float *p) {
+    if (reinterpret_cast<uintptr_t>(p) % alignof(float)) return false;
+    cudaPointerAttributes a{};
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return (a.type == cudaMemoryTypeDevice && a.device == s->device) || a.type == cudaMemoryTypeManaged;
+}
+
 hidem_status read_loss(hidem_surrogate *s, int rows, double *loss) {
     const int nb = (rows + 255) / 256;
     SCK(cudaMemcpyAsync(s->lossHost, s->lossPart, sizeof(float) * nb, cudaMemcpyDeviceToHost, s->stream));
@@ -1878,6 +1890,7 @@ hidem_status hidem_surrogate_predict_device(hidem_surrogate *s, const float *inp
     if (!s) return HIDEM_ERR_ARG;
     if (!inputs || !out || n < 0) return sfail(s, HIDEM_ERR_ARG, "bad arguments");
     SCK(cudaSetDevice(s->device));
+    const bool readDirect = reachable(s, inputs), writeDirect = reachable(s, out);
     // chunks of whole rounds of block pairs over the SMs, as equal as that allows: a chunk of the
     // buffer's size and a small rest cost a round of their own each
     const int64_t round = 256ll * std::max(1, s->smCount);
@@ -1886,17 +1899,19 @@ hidem_status hidem_surrogate_predict_device(hidem_surrogate *s, const float *inp
     for (int64_t r0 = 0; r0 < n; r0 += step) {
         const int rows = (int)std::min<int64_t>(step, n - r0);
         const int padded = (rows + 127) / 128 * 128;  // the ragged last block: zero rows
-        k_features<<<(padded + 7) / 8, dim3(32, 8), 0, s->stream>>>(inputs + r0 * s->nin, nullptr, 0, 0, 0, padded, rows,
-                                                                  s->nin, s->cfg.fourier_bands, s->K0, s->predX);
-        if (ping_pong(s)) {
-            STRY(mlp_forward_pp(s, s->predX, padded, rows, out + r0 * kOut, false));
-            continue;
+        const float *in = inputs + r0 * s->nin;
+        if (!readDirect) {
+            SCK(cudaMemcpyAsync(s->predIn, in, sizeof(float) * s->nin * rows, cudaMemcpyDefault, s->stream));
+            in = s->predIn;
         }
-        float *y = padded > rows ? s->predY : out + r0 * kOut;
-        STRY(mlp_forward(s, s->predX, padded, y, false));
-        if (padded > rows)
-            SCK(cudaMemcpyAsync(out + r0 * kOut, s->predY, sizeof(float) * kOut * rows, cudaMemcpyDeviceToDevice,
-                                s->stream));
+        k_features<<<(padded + 7) / 8, dim3(32, 8), 0, s->stream>>>(in, nullptr, 0, 0, 0, padded, rows, s->nin,
+                                                                  s->cfg.fourier_bands, s->K0, s->predX);
+        // the one-block pass writes whole blocks, the ping-pong pass only the rows there are
+        float *y = writeDirect && (ping_pong(s) || padded == rows) ? out + r0 * kOut : s->predY;
+        if (ping_pong(s)) STRY(mlp_forward_pp(s, s->predX, padded, rows, y, false));
+        else STRY(mlp_forward(s, s->predX, padded, y, false));
+        if (y == s->predY)
+            SCK(cudaMemcpyAsync(out + r0 * kOut, s->predY, sizeof(float) * kOut * rows, cudaMemcpyDefault, s->stream));
     }
     return check_err(s);
 }

@@ -227,3 +227,40 @@ def test_gpu_pingpong_forward_other_depths_and_widths(gpu, layers, nin, bands):
     assert np.max(np.abs(y_pp - y_block)) <= 1e-5 * (np.abs(y_block).max() + 1e-6)
     _, _, y_ref = so.forward_backward(p, layers, u, t, bands)
     assert np.max(np.abs(y_pp - y_ref)) <= 2e-2 * (np.max(np.abs(y_ref)) + 1e-3)
+
+
+# 128 * 2 rows (whole blocks), a ragged count, one row; each pass (the one-block pass for both
+# widths); rows the kernels cannot address themselves: misaligned by two bytes, pinned and pageable
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows", [1, 256, 300])
+@pytest.mark.parametrize("width,block", [(256, False), (256, True), (128, True)])
+def test_gpu_predict_takes_rows_wherever_they_lie(gpu, rows, width, block):
+    import torch
+    from hidem_b200 import abi
+    from hidem_b200 import surrogate as sg
+    cfg = sg.default_config(width=width, hidden_layers=2, fourier_bands=4, batch=256, seed=7, inputs=40)
+    u, _ = _rows(np.random.default_rng(rows), rows, 40)
+    with sg.Surrogate(cfg) as s:
+        if block:
+            s.set_forward(abi.SURROGATE_FORWARD_BLOCK)
+        y = s.predict(u)
+
+        def place(a, how):
+            t = torch.from_numpy(a)
+            if how == "device":
+                t = t.cuda()
+            elif how == "pinned":
+                t = t.pin_memory()
+            elif how == "misaligned":
+                raw = torch.zeros(a.nbytes + 2, dtype=torch.uint8, device="cuda")
+                raw[2:] = t.cuda().reshape(-1).view(torch.uint8)
+                return raw, raw.data_ptr() + 2
+            return t, t.data_ptr()
+        for read in ("device", "misaligned", "pinned", "pageable"):
+            for write in ("device", "misaligned", "pinned", "pageable"):
+                din, pin = place(u, read)
+                dout, pout = place(np.full((rows, 3), np.nan, np.float32), write)
+                torch.cuda.synchronize()
+                s.predict_device(pin, rows, pout)
+                got = dout.cpu() if write != "misaligned" else dout[2:].cpu().view(torch.float32).reshape(rows, 3)
+                assert np.array_equal(got.numpy(), y), (read, write)
