@@ -769,14 +769,15 @@ __device__ __forceinline__ void prefetch_block(const StepArgs<LP> &a, int w, boo
 // forms it) stays whole for certain: its load is below maxLoad by more than 1e-5 (1 + |maxLoad|
 // + |bendBreak| bend), far above the functor's and this test's rounding (a few 2^-23 of the same
 // sum), so the functor's root and division are left to the links near the threshold. A test
-// that is not certain (NaN, a non-positive bound) is false.
+// that is not certain is false: NaN, a non-positive bound, a negative initial length (which
+// turns the functor's inequality round), a bound so small that its square loses digits.
 template <class LP>
 __device__ __forceinline__ bool stays_whole(const StepArgs<LP> &a, LP D, const LP *thA, const LP *thB, LP L0) {
     const LP ax = labs_(thA[0] - thB[0]), ay = labs_(thA[1] - thB[1]), az = labs_(thA[2] - thB[2]);
     const LP myz = (ay < az) ? az : ay;
     const LP bend = (ax < myz) ? myz : ax;
     const LP t = L0 * (a.wholeLoad - a.wholeBend * bend);
-    return t > LP(0) && D < t * t;
+    return L0 > LP(0) && t > LP(1e-16) && D < t * t;
 }
 
 // The link state of one end after the previous step's link update (a.breakPending), both ends

@@ -8,7 +8,7 @@ import numpy as np
 import pytest
 
 from hidem_b200 import abi, workloads
-from hidem_b200.hidemlib import HiDEMLib
+from hidem_b200.hidemlib import HiDEMBatch, HiDEMLib
 from oracle import oracle
 from test_gpu_parity import L_OUT, P_OUT, PRECS, assert_same, gpu_run
 
@@ -78,3 +78,33 @@ def test_geometries_outside_the_shared_root_range(gpu, precision, sep, over):
             assert np.array_equal(out[k], ref[0][k], equal_nan=True), (k, kernel)
         for k in L_OUT:
             assert np.array_equal(links[k], ref[1][k], equal_nan=True), (k, kernel)
+
+
+# Initial lengths the quick test for an unbroken link must leave to the functor: negative with a
+# bend beyond the threshold (the functor breaks where (S - L0) / L0 turns its sign), zero, so small
+# that the squares lose digits, infinite; and ordinary ones on both sides of the threshold.
+@pytest.mark.parametrize("precision", PRECS)
+@pytest.mark.parametrize("bend", [0.0, 0.4, 5.0])
+@pytest.mark.parametrize("length", [-1.0, -0.2, -5.0, 0.0, 1e-20, 1e-30, np.inf, 0.9995, 0.8, 2.0])
+def test_break_decision_for_any_initial_length(gpu, precision, bend, length):
+    P, p, l = _pair(precision, (0.6, 0.5, 0.62))
+    P.breakTime, P.bendBreak, P.maxLoad = -1.0, 1.0, 0.5
+    p["yTheta"][1] = bend
+    l["initialLen"][0] = length
+    ref = oracle.port().run(P, p, l, 3)
+    for kernel in (abi.STEP_KERNEL_TWO_PASS, abi.STEP_KERNEL_ITEMS, abi.STEP_KERNEL_THREAD):
+        out_p, out_l, _, events, _ = gpu_run(P, p, l, 3, kernel=kernel)
+        assert np.array_equal(events.reshape(-1, 2), np.asarray(ref[3]).reshape(-1, 2)), kernel
+        for k in P_OUT:
+            assert np.array_equal(out_p[k], ref[0][k], equal_nan=True), (k, kernel)
+        for k in L_OUT:
+            assert np.array_equal(out_l[k], ref[1][k], equal_nan=True), (k, kernel)
+    # the batch's break pass
+    lib = HiDEMLib(P)
+    lib.set_particles(p)
+    lib.set_links(l)
+    with HiDEMBatch([lib]) as batch:
+        batch.step(3)
+    li, st = lib.get_break_events()
+    assert np.array_equal(np.stack([li, st], axis=1).reshape(-1, 2), np.asarray(ref[3]).reshape(-1, 2))
+    lib.close()
