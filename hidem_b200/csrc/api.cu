@@ -73,6 +73,19 @@ inline bool writable_here(int device, const void *p, size_t elem) {
     }
     return a.type == cudaMemoryTypeDevice && a.device == device;
 }
+// The arrays of one readback so far. One that overlaps an earlier one is not written by the kernel
+// but copied after it, so that the later field's values stand there whichever way each travels.
+struct Destinations {
+    std::vector<std::pair<uintptr_t, uintptr_t>> taken;
+    Destinations() { taken.reserve(14); }
+    bool overlaps(const void *p, size_t bytes) {
+        const uintptr_t a = reinterpret_cast<uintptr_t>(p), b = a + bytes;
+        bool hit = false;
+        for (const auto &t : taken) hit = hit || (a < t.second && t.first < b);
+        taken.emplace_back(a, b);
+        return hit;
+    }
+};
 // bytes between a caller's array (host or device memory) and host memory
 inline cudaError_t from_caller(void *hostDst, const void *src, size_t bytes) {
     if (on_device(src)) return cudaMemcpy(hostDst, src, bytes, cudaMemcpyDeviceToHost);
@@ -2281,8 +2294,12 @@ static hidem_status get_particles_t(hidem_ctx *ctx, hidem_particle_soa *out) {
     };
     std::vector<Copy> copies;
     size_t used = 0;
+    Destinations dests;
+    auto direct = [&](void *dst, size_t elem) {
+        return !dests.overlaps(dst, elem * (size_t)n) && writable_here(ctx->device, dst, elem);
+    };
     auto place = [&](void *dst, size_t elem) -> void * {
-        if (!dst || writable_here(ctx->device, dst, elem)) return dst;
+        if (!dst || direct(dst, elem)) return dst;
         void *p = stage + used;
         used += elem * (size_t)n;
         copies.push_back({dst, p, elem * (size_t)n});
@@ -2296,7 +2313,7 @@ static hidem_status get_particles_t(hidem_ctx *ctx, hidem_particle_soa *out) {
     for (int k = 0; k < 6; ++k) s.d[k] = static_cast<LP *>(place(d[k], sizeof(LP)));
     s.r = static_cast<LP *>(place(out->radius, sizeof(LP)));
     for (int k = 0; k < 3; ++k) s.th[k] = static_cast<LP *>(place(th[k], sizeof(LP)));
-    if (out->type && !writable_here(ctx->device, out->type, 1)) {
+    if (out->type && !direct(out->type, 1)) {
         // the record buffer is full when every field is staged: the rebuild's permutation scratch
         s.type = reinterpret_cast<uint8_t *>(ctx->perm);
         copies.push_back({out->type, s.type, (size_t)n});
@@ -2322,9 +2339,10 @@ static hidem_status get_sides_t(hidem_ctx *ctx, hidem_link_soa *out, void **stag
     all.state = s.state;
     direct = all;
     bool any = false, staged = false;
+    Destinations dests;
     for (int k = 0; k < 6; ++k) {
         if (!out->CT[k]) continue;
-        if (writable_here(ctx->device, out->CT[k], sizeof(LP))) {
+        if (!dests.overlaps(out->CT[k], sizeof(LP) * (size_t)(2 * L)) && writable_here(ctx->device, out->CT[k], sizeof(LP))) {
             direct.out[k] = static_cast<LP *>(out->CT[k]);
             any = true;
         } else {
@@ -2332,7 +2350,7 @@ static hidem_status get_sides_t(hidem_ctx *ctx, hidem_link_soa *out, void **stag
         }
     }
     if (out->state) {
-        if (writable_here(ctx->device, out->state, 1)) {
+        if (!dests.overlaps(out->state, (size_t)L) && writable_here(ctx->device, out->state, 1)) {
             direct.stateOut = out->state;
             any = true;
         } else {

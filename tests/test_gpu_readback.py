@@ -60,3 +60,40 @@ def test_destinations(gpu, precision, cells):
     got_ct = raw[2:2 + lib.L * 2 * lp.itemsize].cpu().numpy().tobytes()
     assert got_x == host_p["xCord"].tobytes() and got_ct == host_l["CT3"].tobytes()
     lib.close()
+
+
+# arrays that overlap (a buffer for fields that are not looked at, views into one allocation): the
+# later field's values stand where two meet, whether the first lies there whole, in part or in
+# another type
+@pytest.mark.parametrize("precision", [abi.PREC_MIXED, abi.PREC_FP64])
+@pytest.mark.parametrize("cells", [(5, 3, 3), (23, 11, 9)])
+def test_overlapping_destinations(gpu, precision, cells):
+    import torch
+    P, p, l = workloads.ice_block(cells=cells, precision=precision, seed=4)
+    lib = HiDEMLib(P)
+    lib.set_particles(p)
+    lib.set_links(l)
+    lib.step(12)
+    host_p, host_l = lib.get_particles(), lib.get_links()
+    n, L, lp = lib.n, lib.L, np.dtype(abi.lp_dtype(precision)).itemsize
+    # fields in the order of the reads, each with the byte its array starts at
+    fields = [("xCord", 0), ("yCord", 8 * (n // 3)), ("uDiff", 8 * (n // 2)), ("xTheta", 8 * (n // 2) + lp * (n // 4)),
+              ("type", 16 * (n // 5))]
+    ends = [("CT0", 0), ("CT1", lp * (L // 3)), ("CT4", lp * L), ("state", lp * (L // 2))]
+    psoa, lsoa = abi.HidemParticleSoA(), abi.HidemLinkSoA()
+    for soa, read, order, host in ((psoa, lib._lib.hidem_get_particles, fields, host_p),
+                                   (lsoa, lib._lib.hidem_get_links, ends, host_l)):
+        room = max(at + host[k].nbytes for k, at in order)
+        dev = torch.zeros(room, dtype=torch.uint8, device="cuda")
+        want = np.zeros(room, np.uint8)
+        torch.cuda.synchronize()
+        for k, at in order:
+            want[at:at + host[k].nbytes] = host[k].view(np.uint8)
+            if k.startswith("CT"):
+                soa.CT[int(k[2])] = dev.data_ptr() + at
+            else:
+                setattr(soa, k, dev.data_ptr() + at)
+        for _ in range(3):
+            lib._check(read(lib._ctx, C.byref(soa)))
+            assert np.array_equal(dev.cpu().numpy(), want)
+    lib.close()
