@@ -1796,7 +1796,9 @@ hidem_status hidem_surrogate_create(const hidem_surrogate_config *c, int device,
     }
     const double ao = 1.0 / std::sqrt((double)W);
     for (long long q = 0; q < (long long)kOut * W; ++q) p[s->offWo + q] = (float)((2 * next() - 1) * ao);
-    e = cudaMemcpy(s->P, p.data(), sizeof(float) * s->np, cudaMemcpyHostToDevice);
+    // on the surrogate's stream, ahead of the BF16 copies made from them: a copy on the default stream
+    // may return before its last piece has arrived, and this stream does not wait for that one
+    e = cudaMemcpyAsync(s->P, p.data(), sizeof(float) * s->np, cudaMemcpyHostToDevice, s->stream);
     if (e != cudaSuccess) return fail(e);
     if (refresh_bf16(s) != HIDEM_OK || cudaStreamSynchronize(s->stream) != cudaSuccess) {
         err = s->err;

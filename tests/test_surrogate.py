@@ -264,3 +264,28 @@ def test_gpu_predict_takes_rows_wherever_they_lie(gpu, rows, width, block):
                 s.predict_device(pin, rows, pout)
                 got = dout.cpu() if write != "misaligned" else dout[2:].cpu().view(torch.float32).reshape(rows, 3)
                 assert np.array_equal(got.numpy(), y), (read, write)
+
+
+# batches of fewer and of more blocks than SMs (one block a CTA, pairs of blocks), a split that the
+# rows do not divide evenly, an odd number of blocks
+@pytest.mark.gpu
+@pytest.mark.parametrize("width,layers,batch", [(256, 4, 1024), (256, 4, 128 * 149), (256, 2, 128 * 331), (128, 3, 128 * 7),
+                                                (256, 8, 128)])
+def test_gpu_training_runs_from_one_seed_are_equal(gpu, width, layers, batch):
+    """The gradients of a step come from several streams, the first weights from the host: nothing
+    may depend on how they interleave, nor on what the memory held before."""
+    from hidem_b200 import surrogate as sg
+    cfg = sg.default_config(width=width, hidden_layers=layers, fourier_bands=4, batch=batch, seed=11, inputs=40)
+    rng = np.random.default_rng(4)
+    u, t = _rows(rng, 5000, 40)
+    runs = []
+    for calls in ((12,), (12,), (5, 7)):
+        with sg.Surrogate(cfg) as s:
+            s.set_data(u, t)
+            losses = [s.train(k) for k in calls]
+            g, loss = s.gradients(u[:128], t[:128])
+            runs.append((s.get_params(), losses[-1], g, loss))
+    for params, loss, g, last in runs[1:]:
+        assert np.array_equal(params, runs[0][0]) and loss == runs[0][1]
+        assert np.array_equal(g, runs[0][2]) and last == runs[0][3]
+    assert np.isfinite(runs[0][0]).all()
