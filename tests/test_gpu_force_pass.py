@@ -57,7 +57,8 @@ def _pair(precision, sep, **over):
 
 
 # vertical (no xy part), nearly vertical (its square outside the shared-root range), near
-# coincidence, squared lengths whose root rounds to all ones, E W4 outside the admitted range
+# coincidence, next to a length whose root rounds to all ones (the lengths themselves:
+# test_lengths_the_shared_root_leaves_out), E W4 outside the admitted range
 @pytest.mark.parametrize("precision", PRECS)
 @pytest.mark.parametrize("sep,over", [((0.0, 0.0, 1.0), {}), ((1e-7, 0.0, 0.97), {}), ((1e-9, -1e-9, 0.9), {}),
                                       ((3e-7, 2e-7, 1e-7), {}), ((0.9999999, 0.0, 0.0), {}),
@@ -65,6 +66,10 @@ def _pair(precision, sep, **over):
                                       ((0.6, 0.5, 0.4), dict(E=1e21))])
 def test_geometries_outside_the_shared_root_range(gpu, precision, sep, over):
     P, p, l = _pair(precision, sep, **over)
+    check_one_step(P, p, l)
+
+
+def check_one_step(P, p, l):
     ref = oracle.port().run(P, p, l, 1)
     for kernel in (abi.STEP_KERNEL_TWO_PASS, abi.STEP_KERNEL_ITEMS, abi.STEP_KERNEL_THREAD):
         lib = HiDEMLib(P)
@@ -78,6 +83,35 @@ def test_geometries_outside_the_shared_root_range(gpu, precision, sep, over):
             assert np.array_equal(out[k], ref[0][k], equal_nan=True), (k, kernel)
         for k in L_OUT:
             assert np.array_equal(links[k], ref[1][k], equal_nan=True), (k, kernel)
+
+
+# The lengths at which the shared-root evaluation hands over to the IEEE operations, each shown to
+# be one here: a squared length whose root rounds to all ones (the two largest floats below an even
+# power of two), in contact and beyond it, as the whole length and as its part in the xy plane; and
+# a length whose square rounds to all ones (every squared length of 2 or 1/2: 1 / sqrt(2) * 2 is one
+# unit below sqrt(2)). No length's cube does: checked over every significand.
+@pytest.mark.parametrize("sep,where", [((1 - 2.0 ** -24, 0.0, 0.0), "root"), ((0.0, 0.0, 1 - 2.0 ** -24), "length only"),
+                                       ((0.0, 1 - 2.0 ** -24, 0.25), "plane only"), ((2 - 2.0 ** -23, 0.0, 0.0), "root"),
+                                       ((0.5 - 2.0 ** -25, 0.0, 0.0), "root"), ((1.0, 1.0, 0.0), "square"),
+                                       ((0.5, 0.0, 0.5), "square"), ((0.5, 0.25, 0.4330127018922193), "square")])
+def test_lengths_the_shared_root_leaves_out(gpu, sep, where):
+    f = np.float32
+    x, y, z = (f(v) for v in sep)
+    ones = lambda v: int(v.view(np.uint32)) & 0x7fffff == 0x7fffff  # noqa: E731
+    xy = x * x + y * y
+    D = xy + z * z
+    length = (f(1) / np.sqrt(D)) * D
+    root = ones(np.sqrt(D)), ones(np.sqrt(xy))
+    assert root == {"root": (True, True), "length only": (True, False), "plane only": (False, True),
+                    "square": (False, False)}[where]
+    assert ones(length * length) or where != "square"
+    check_one_step(*_pair(abi.PREC_MIXED, sep))
+
+
+def test_no_length_has_a_cube_of_all_ones():
+    m = np.arange(0x3f800000, 0x40000000, dtype=np.uint32).view(np.float32)  # the pattern repeats in every binade
+    cube = (m * m) * m
+    assert not np.any((cube.view(np.uint32) & 0x7fffff) == 0x7fffff)
 
 
 # Initial lengths the quick test for an unbroken link must leave to the functor: negative with a

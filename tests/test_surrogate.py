@@ -289,3 +289,27 @@ def test_gpu_training_runs_from_one_seed_are_equal(gpu, width, layers, batch):
         assert np.array_equal(params, runs[0][0]) and loss == runs[0][1]
         assert np.array_equal(g, runs[0][2]) and last == runs[0][3]
     assert np.isfinite(runs[0][0]).all()
+
+
+@pytest.mark.gpu
+def test_gpu_predict_device_on_both_sides_of_a_chunk_border(gpu):
+    """Row counts around the predict buffers' size and around the ends of equal chunks (whole rounds
+    of 256 rows an SM): the host call's outputs, and nothing written beyond the rows."""
+    import torch
+    from hidem_b200 import surrogate as sg
+    cfg = sg.default_config(width=256, hidden_layers=2, fourier_bands=2, batch=1024, seed=7, inputs=5)
+    buffer = 262144
+    turn = 256 * torch.cuda.get_device_properties(0).multi_processor_count
+    half = -(-(buffer // 2 + 1) // turn) * turn  # the chunk of the first count that takes two
+    counts = [turn - 1, turn, turn + 1, buffer - 1, buffer, buffer + 1, 2 * half - 129, 2 * half - 1, 2 * half, 2 * half + 1]
+    u, _ = _rows(np.random.default_rng(8), max(counts), 5)
+    du = torch.from_numpy(u).cuda()
+    with sg.Surrogate(cfg) as s:
+        y = s.predict(u)
+        for n in counts:
+            out = torch.full((n + 256, 3), 7.0, device="cuda")
+            torch.cuda.synchronize()
+            s.predict_device(du.data_ptr(), n, out.data_ptr())
+            got = out.cpu().numpy()
+            assert np.array_equal(got[:n], y[:n]), n
+            assert (got[n:] == 7.0).all(), n
