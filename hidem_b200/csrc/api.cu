@@ -92,8 +92,10 @@ inline cudaError_t from_caller(void *hostDst, const void *src, size_t bytes) {
     host_copy(hostDst, src, bytes);
     return cudaSuccess;
 }
-inline cudaError_t to_caller(void *dst, const void *hostSrc, size_t bytes) {
-    if (on_device(dst)) return cudaMemcpy(dst, hostSrc, bytes, cudaMemcpyHostToDevice);
+// (into device memory on `st`, whose next wait covers it: a copy on the default stream may return
+// before its last piece has arrived, and no other stream waits for that one)
+inline cudaError_t to_caller(void *dst, const void *hostSrc, size_t bytes, cudaStream_t st) {
+    if (on_device(dst)) return cudaMemcpyAsync(dst, hostSrc, bytes, cudaMemcpyHostToDevice, st);
     host_copy(dst, hostSrc, bytes);
     return cudaSuccess;
 }
@@ -2393,8 +2395,8 @@ hidem_status hidem_get_particles(hidem_ctx *ctx, hidem_particle_soa *out) {
     CK(cudaSetDevice(ctx->device));
     TRY(ctx->mixed ? get_particles_t<float>(ctx, out) : get_particles_t<double>(ctx, out));
     // the host-held fields while the copies run
-    if (out->owners) CK(to_caller(out->owners, ctx->owners.data(), 4 * (size_t)ctx->n));
-    if (out->globalKeys) CK(to_caller(out->globalKeys, ctx->keys.data(), 8 * (size_t)ctx->n));
+    if (out->owners) CK(to_caller(out->owners, ctx->owners.data(), 4 * (size_t)ctx->n, ctx->stream));
+    if (out->globalKeys) CK(to_caller(out->globalKeys, ctx->keys.data(), 8 * (size_t)ctx->n, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
     return HIDEM_OK;
 }
@@ -2860,7 +2862,7 @@ hidem_status build_mesh(hidem_ctx *ctx, const hidem_mesh *mesh, MeshView<LP> &m)
             keep[t] = (n2 > 1e-6f * e * e && std::isfinite(n2)) ? 0 : 1;
         }
         CK(cudaMalloc(&ctx->meshKeep, (size_t)T));
-        CK(cudaMemcpy(ctx->meshKeep, keep.data(), (size_t)T, cudaMemcpyHostToDevice));
+        CK(cudaMemcpyAsync(ctx->meshKeep, keep.data(), (size_t)T, cudaMemcpyHostToDevice, ctx->stream));
     }
     ctx->meshTris = T;
     const size_t vb = sizeof(LP) * 3 * (size_t)T, nb = sizeof(LP) * (size_t)T;
