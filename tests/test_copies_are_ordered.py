@@ -20,8 +20,5 @@ def test_copies_to_the_device_are_on_a_stream(source):
     assert not re.findall(r"\bcudaMemset(?:2D|3D)?\([^;]*;", text)
     # and every kernel launch names its stream
     for launch in re.findall(r"<<<(.*?)>>>", text, re.S):
-        depth, args = 0, 1
-        for ch in launch.replace("->", "."):
-            depth += {"(": 1, ")": -1, "<": 1, ">": -1}.get(ch, 0)
-            args += ch == "," and depth == 0
-        assert args == 4, launch
+        stream = launch.rsplit(",", 1)[-1].strip()
+        assert stream in ("s", "st", "so", "sl", "stream") or stream.endswith(("->stream", ".stream")), launch
