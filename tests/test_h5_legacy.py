@@ -4,16 +4,16 @@ benchmark inputs where its tree is present, and files of every supported storage
 by an independent encoder (tests/h5_legacy.py). Host code only: no GPU."""
 from __future__ import annotations
 
-import os
 from pathlib import Path
 
 import numpy as np
 import pytest
 
 import h5_legacy as h5
+from __graft_entry__ import REFERENCE_TREE
 from hidem_b200 import abi, workloads
 
-REF = Path(os.environ.get("HIDEM_REFERENCE_TREE", "/root/reference"))
+REF = Path(REFERENCE_TREE)
 BENCH = REF / "HiDEM" / "Benchmark"
 # particle counts of the benchmark inputs (the 5700k and 310k counts are the ones the
 # reference's scaling plot quotes, HiDEM/Docs/Images/GPU_scaling.png)

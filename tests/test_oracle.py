@@ -111,6 +111,7 @@ def test_oracle_bed_and_force_maps_match_reference(precision):
     assert not np.array_equal(a[0]["zCord"], c[0]["zCord"])
 
 
+@needs_ref
 @pytest.mark.parametrize("precision", [abi.PREC_MIXED, abi.PREC_FP64])
 def test_oracle_collision_mesh_matches_reference(precision):
     """Collision mesh of the MeshConstrainedDem sample: the restatement's MeshAccel grid
@@ -147,6 +148,7 @@ def test_oracle_collision_mesh_matches_reference(precision):
     assert not np.array_equal(a[0]["zCord"], c[0]["zCord"])
 
 
+@needs_ref
 @pytest.mark.parametrize("precision", [abi.PREC_MIXED, abi.PREC_FP64])
 def test_oracle_collision_mesh_cloud_matches_reference(precision):
     from conftest import mesh_cloud_case
@@ -165,6 +167,7 @@ def test_oracle_collision_mesh_cloud_matches_reference(precision):
         assert np.array_equal(a[0][k], b[0][k]), k
 
 
+@needs_ref
 @pytest.mark.parametrize("precision", [abi.PREC_MIXED, abi.PREC_FP64])
 def test_oracle_contact_list_matches_reference_on_irregular_input(precision):
     rng = np.random.default_rng(5)
