@@ -820,7 +820,6 @@ StepArgs<LP> step_args(hidem_ctx *ctx) {
     a.events = ctx->events;
     a.eventCount = ctx->eventCount;
     a.eventCap = ctx->eventCap;
-    a.errorFlag = ctx->errorFlag;
     return a;
 }
 

@@ -167,7 +167,6 @@ struct StepArgs {
     int2 *events;             // (link, step) of links that broke
     unsigned long long *eventCount;
     long long eventCap;
-    int *errorFlag;
     int maxContacts, maxEnds; // widest rows of this layout
     LP bendBreak, maxLoad;    // HiDEMDefLinkBreakFunc thresholds (per context in a batch)
     // stays_whole's bounds: 1 + maxLoad - 1e-5 (1 + |maxLoad|), bendBreak + 1e-5 |bendBreak|

@@ -608,12 +608,6 @@ __device__ __forceinline__ bool mb_wait_or_fail(uint64_t *b, uint32_t parity, co
     return false;
 }
 
-// One epilogue thread's share of a unit of k_mlp_pp: its row's 64 columns starting at
-// c0s, 32 at a time, from tensor memory (taddr: the row's lane, the block's accumulator):
-// bias + SiLU -> BF16. KEEP (training): pre-activations and activations to global memory.
-// LAST: the output layer's partial sums over these columns, in k order, into o; otherwise
-// the activations into the next layer's swizzled K-major A tile. The two flags are template
-// parameters so that neither path costs the other instructions.
 // 32 bytes in one store (32-byte aligned). A lane of the epilogue holds a row, so every store
 // touches 32 lines and their number is what the kept activations cost: half as many as with
 // 16-byte stores (a training forward pass of 8,192 rows 66 -> 43 us).
@@ -624,6 +618,12 @@ __device__ __forceinline__ void store32(void *p, uint32_t a, uint32_t b, uint32_
                  : "memory");
 }
 
+// One epilogue thread's share of a unit of k_mlp_pp: its row's 64 columns starting at
+// c0s, 16 at a time, from tensor memory (taddr: the row's lane, the block's accumulator):
+// bias + SiLU -> BF16. KEEP (training): pre-activations and activations to global memory.
+// LAST: the output layer's partial sums over these columns, in k order, into o; otherwise
+// the activations into the next layer's swizzled K-major A tile. The two flags are template
+// parameters so that neither path costs the other instructions.
 template <int BN, bool LAST, bool KEEP>
 __device__ __forceinline__ void pp_epilogue(uint32_t taddr, int c0s, int row, long long grow, bool live,
                                             const float *__restrict__ bias, float *zo, bf16 *ho,
@@ -1402,7 +1402,6 @@ hidem_status refresh_bf16(hidem_surrogate *s) {
     return HIDEM_OK;
 }
 
-// forward over `rows` rows whose features are in X0 (keepZ: store pre-activations)
 // The whole forward pass over `rows` rows of features X (a multiple of 128) in one fused
 // launch (k_mlp_fwd); keepZ: the training pass, which keeps every layer's pre-activations
 // and activations for the backward pass.
@@ -1440,7 +1439,8 @@ hidem_status mlp_forward_t(hidem_surrogate *s, const bf16 *X, int rows, float *Y
 }
 
 // The same pass as the persistent ping-pong kernel (k_mlp_pp, 256-wide networks): one CTA
-// per SM at most, each taking pairs of 128-row blocks.
+// per SM at most, each taking pairs of 128-row blocks, or one block alone where there are no more
+// blocks than SMs. Rows of Y from `live` on are not written.
 hidem_status mlp_forward_pp(hidem_surrogate *s, const bf16 *X, int rows, int live, float *Y, bool keepZ) {
     static std::atomic<unsigned long long> configured{0};
     int dev = 0;

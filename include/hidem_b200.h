@@ -257,8 +257,9 @@ hidem_status hidem_unpack_halo_forces(hidem_ctx *ctx, const void *device_in);
 /* n whole timesteps of the sample main loop (MainMeshBlock.cpp:274-323):
  * gridService, forces, integrate, gated link update, finalizeTs — each step as the
  * context's step kernel (hidem_set_step_kernel: one fused kernel, or the two-pass step's
- * force and integrate passes and break pass), launched back to back between the
- * gridService checks without host synchronisation. */
+ * force and integrate passes; either applies the previous step's link update, and the call's
+ * last one is a pass of its own), launched back to back between the gridService checks without
+ * host synchronisation. */
 hidem_status hidem_step(hidem_ctx *ctx, int32_t nsteps);
 /* The default functors as a caller's main constructs them (HiDEM/Common/
  * HiDEMDefaultFunctions.h): HiDEMDefNeighForceFunc(invDt, attractDistance,

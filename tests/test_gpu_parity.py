@@ -92,7 +92,7 @@ def test_step_kernel_autotuner_settles(gpu):
     lib.set_links(l)
     assert lib.step_kernel() == abi.STEP_KERNEL_AUTO
     lib.step(4)
-    assert lib.step_kernel() == abi.STEP_KERNEL_AUTO  # still timing (5 kernels x 3 rounds)
+    assert lib.step_kernel() == abi.STEP_KERNEL_AUTO  # still timing (2 kernels x 5 rounds)
     lib.step(11)
     assert lib.step_kernel() in (abi.STEP_KERNEL_ITEMS, abi.STEP_KERNEL_THREAD,
                                  abi.STEP_KERNEL_THREAD_CAPPED, abi.STEP_KERNEL_THREAD_ASYNC,
