@@ -1658,13 +1658,18 @@ hidem_status hidem_create(const hidem_params *params, int device, hidem_ctx **ou
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&ctx->smCount, cudaDevAttrMultiProcessorCount, device);
     if (e == cudaSuccess) {
-        // the contexts' buffers come from the device's default stream-ordered pool: keep up
-        // to 8 GiB of freed blocks for reuse (later contexts, regrown buffers) instead of
-        // returning them to the driver at every synchronisation
+        // The contexts' buffers come from the device's default stream-ordered pool: it keeps up to
+        // an eighth of the device's memory (8 GiB at least) for reuse by later contexts and regrown
+        // buffers, and returns what it holds beyond that to the driver at a synchronisation. The
+        // 5.7M slab takes 10.0 GiB (mixed) or 15.3 GiB (FP64): a pool that keeps 8 GiB has the rest
+        // mapped anew for every job, which takes 20 ms on a quiet host and up to 1.6 s on a busy
+        // one.
         cudaMemPool_t pool;
-        if (cudaDeviceGetDefaultMemPool(&pool, device) == cudaSuccess) {
-            uint64_t keep = 8ull << 30;
-            cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+        size_t freeBytes = 0, total = 0;
+        if (cudaDeviceGetDefaultMemPool(&pool, device) == cudaSuccess && cudaMemGetInfo(&freeBytes, &total) == cudaSuccess) {
+            uint64_t has = 0, keep = std::max<uint64_t>(8ull << 30, total / 8);
+            if (cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &has) == cudaSuccess && has < keep)
+                cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
         }
     }
     if (e != cudaSuccess) {

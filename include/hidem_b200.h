@@ -145,7 +145,9 @@ hidem_status hidem_params_from_toml(const char *path, int32_t argc, const char *
 /* ---- context --------------------------------------------------------- */
 
 /* Replaces HiDEMLib::setup (HiDEMLib/HiDEMLib.h:707-822) for the hot path:
- * selects `device`, creates the stream and the derived constants. */
+ * selects `device`, creates the stream and the derived constants. Device memory comes from the
+ * device's default stream-ordered pool; of what the contexts give back, the pool keeps up to an
+ * eighth of the device's memory for the next ones (cudaMemPoolTrimTo on that pool returns it). */
 hidem_status hidem_create(const hidem_params *params, int device, hidem_ctx **out);
 void hidem_destroy(hidem_ctx *ctx);
 const char *hidem_last_error(const hidem_ctx *ctx);
