@@ -1663,13 +1663,15 @@ hidem_status hidem_create(const hidem_params *params, int device, hidem_ctx **ou
         // buffers, and returns what it holds beyond that to the driver at a synchronisation. The
         // 5.7M slab takes 10.0 GiB (mixed) or 15.3 GiB (FP64): a pool that keeps 8 GiB has the rest
         // mapped anew for every job, which takes 20 ms on a quiet host and up to 1.6 s on a busy
-        // one.
+        // one. Set once: a threshold of 8 GiB or more, this one or the caller's, stays.
         cudaMemPool_t pool;
+        uint64_t has = 0;
         size_t freeBytes = 0, total = 0;
-        if (cudaDeviceGetDefaultMemPool(&pool, device) == cudaSuccess && cudaMemGetInfo(&freeBytes, &total) == cudaSuccess) {
-            uint64_t has = 0, keep = std::max<uint64_t>(8ull << 30, total / 8);
-            if (cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &has) == cudaSuccess && has < keep)
-                cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+        if (cudaDeviceGetDefaultMemPool(&pool, device) == cudaSuccess &&
+            cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &has) == cudaSuccess &&
+            has < (8ull << 30) && cudaMemGetInfo(&freeBytes, &total) == cudaSuccess) {
+            uint64_t keep = std::max<uint64_t>(8ull << 30, total / 8);
+            cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
         }
     }
     if (e != cudaSuccess) {
